@@ -111,6 +111,21 @@ struct SorFast {
     int tile_rank = 0;         // the one planned
 };
 
+// Plan and device buffers of the direct Coulomb solve (k_poisson.cu).
+struct PoissonDirect {
+    bool ok = false;           // the plane and its matrices fit on chip
+    int off = 0, wz = 0, ps = 0, py = 0;  // stored plane: second half's column, columns, pitch; y matrices' pitch
+    int rt = 0, nt = 0;        // kernel form: rows of a thread's tile, tiles per warp
+    int shared_tab = 0, keep_tab = 0, front = 0, cw_max = 0, nblocks = 0;
+    size_t smem = 0;
+    float *tables = nullptr;   // sine matrices of z and y, both directions, and the eigenvalues (owns the
+                               // allocation the pointers below lie in)
+    float *work = nullptr;     // the planes' spectrum
+    float *delta = nullptr;    // correction per node, zero on the faces
+    double *partials = nullptr;
+    unsigned *bar = nullptr;   // [0] arrivals, [1] generation
+};
+
 // Decomposed smoothing plan (k_smooth_fast.cu).
 constexpr int kSmoothMaxR = 16;  // largest |a|, |b| or z half-width handled
 // Capacity of the FFT smoothing's wrap list: particles that deposit within the
@@ -146,7 +161,9 @@ struct Fused {
     bool ready = false;
     double *phi64 = nullptr;      // Coulomb potential (double for every precision)
     double *phi64_prev = nullptr; // previous step's phi (extrapolated warm start)
-    double *phi64_prev2 = nullptr; // the step before's (quadratic extrapolation)
+    double *phi64_prev2 = nullptr; // the step before's (quadratic extrapolation); with the direct solve the
+                                   // extrapolated start of the next one
+    bool hist_direct = false;      // which of the two forms the history is in
     void *F4 = nullptr;           // interleaved forces, 4 x T per node
     double *obs_partials = nullptr;  // per-step observable partials
     int obs_blocks = 0;           // blocks of the particle step (one partial row each)
@@ -161,6 +178,7 @@ struct Fused {
     bool f4_current = false;      // F4 holds the forces of the current positions
     int m_hint = 8;               // iterations of the previous SOR solve (seeds the first cycle)
     SorFast sor;
+    PoissonDirect direct;
     SmoothFast smooth;
 };
 
@@ -248,6 +266,13 @@ hv_status fused_release(hv_ctx *c);
 hv_status fused_run(hv_ctx *c, int n_steps, hv_observables *obs);
 hv_status fused_autotune(hv_ctx *c, int trial, hv_autotune_report *rep);
 void fused_invalidate(hv_ctx *c);
+
+// Direct Coulomb solve of float contexts (k_poisson.cu)
+hv_status poisson_plan(hv_ctx *c);
+void poisson_release(hv_ctx *c);
+bool poisson_direct_runs(const hv_ctx *c);
+hv_status poisson_launch(hv_ctx *c, const float *rho, int *ctl, int *its_ring, int ring, bool step_solve);
+hv_status poisson_clear(hv_ctx *c);
 
 // Several float SOR solves run by one cooperative launch (k_sor_fast.cu).
 struct SorWave {

@@ -829,12 +829,20 @@ hv_status enqueue_phase_c(hv_ctx *c) {
     return HV_OK;
 }
 
+// The Coulomb solve: the direct correction where it runs, else the sweeps.
+template <typename T>
+hv_status launch_coulomb(hv_ctx *c, const T *rho, int *its_ring, bool step_solve) {
+    if constexpr (sizeof(T) == 4)
+        if (poisson_direct_runs(c)) return poisson_launch(c, rho, ctl_of(c), its_ring, kRing, step_solve);
+    return sor_fast_launch<T>(c, rho, ctl_of(c), its_ring, kRing, step_solve);
+}
+
 template <typename T>
 hv_status enqueue_step(hv_ctx *c) {
     HV_TRY(enqueue_phase_a<T>(c));
     {
         ProfScope ps(c, HV_K_SOR);
-        HV_TRY(sor_fast_launch<T>(c, st<T>(c).rho, ctl_of(c), c->fused.sor_its, kRing, true));
+        HV_TRY(launch_coulomb<T>(c, st<T>(c).rho, c->fused.sor_its, true));
     }
     return enqueue_phase_c<T>(c);
 }
@@ -901,7 +909,7 @@ hv_status initial_typed(hv_ctx *c) {
     HV_CUDA(cudaMemcpyAsync(ctl, h_ctl, sizeof(int) * 3, cudaMemcpyHostToDevice, c->stream));
     // from phi = 0: neither extrapolated nor recorded as an earlier solution
     HV_TRY(sor_fast_clear_error(c));
-    HV_TRY(sor_fast_launch<T>(c, s.rho, ctl, nullptr, kRing, false));
+    HV_TRY(launch_coulomb<T>(c, s.rho, nullptr, false));
     const T idx = T(1.0) / (T(2.0) * T(g.dmx) / g.nx), idy = T(1.0) / (T(2.0) * T(g.dmy) / g.ny),
             idz = T(1.0) / (T(2.0) * T(g.dmz) / g.nz);
     k_forces_f4<T><<<forces_grid(g, kForceRows), forces_block(g), 0, c->stream>>>(
@@ -951,6 +959,12 @@ hv_status run_begin(hv_ctx *c, int n_steps, int *exc_out) {
         int zero = 0;
         HV_CUDA(cudaMemcpyAsync(ctl + CTL_PREV, &zero, sizeof(int), cudaMemcpyHostToDevice, c->stream));
         f.f4_current = true;
+    }
+    // the sweeps and the direct solve keep phi's history in different forms
+    const bool direct = poisson_direct_runs(c);
+    if (direct != f.hist_direct) {
+        HV_CUDA(cudaMemsetAsync(ctl + CTL_PREV, 0, sizeof(int), c->stream));
+        f.hist_direct = direct;
     }
     // excitation step: first n with n dt >= t_exc (hyper_vlasov.cpp:86), in T
     int exc = -1;
@@ -1209,6 +1223,7 @@ hv_status fused_prepare(hv_ctx *c) {
         set_last_error("fused path: the SOR correction of this grid does not fit on chip");
         return HV_ERR_UNSUPPORTED;
     }
+    HV_TRY(poisson_plan(c));
     if (c->prec == HV_F32) HV_TRY(smooth_fast_plan(c));
     HV_CUDA(cudaStreamSynchronize(c->stream));
     f.ready = true;
@@ -1222,6 +1237,7 @@ hv_status fused_release(hv_ctx *c) {
     for (void *p : ptrs)
         if (p) cudaFree(p);
     sor_fast_release(c);
+    poisson_release(c);
     smooth_fast_release(c);
     f = Fused();
     return HV_OK;

@@ -1,0 +1,851 @@
+// Direct Coulomb solve of the fused path: every correction of the carried FP64
+// residual is solved exactly on the run's own grid.
+//
+// The cycle is the persistent SOR's (k_sor_fast.cu): phi in double, the double
+// residual r = b + lap_h phi, the stopping rule tested on it, and a float
+// correction delta with -lap_h delta = r folded in as phi += delta.  Only the
+// way delta is found differs.  The red-black sweeps need dozens of exchanges
+// between blocks per solve, each a round trip through L2; here delta comes
+// from sine transforms along y and z (dense float matrices, exact for every
+// extent) and a tridiagonal elimination along x, so that a solve is a fixed
+// four phases with a grid barrier after each:
+//   A  per x plane: r (double, from the extrapolated phi), the two forward
+//      transforms of the plane in shared memory
+//   B  per group of (ky, kz) columns: the tridiagonal systems along x
+//   C  per x plane: the two inverse transforms, delta
+//   D  per x plane: phi += delta, the history rotated, |r + lap delta|^2
+// and the rule is tested after A and after D.  A float correction leaves the
+// residual's rounding noise, ~1e-6 of it for the rough residual of an
+// extrapolated start and ~3e-4 for the smooth one of a first guess, so a step
+// takes one correction and a first solve two or three.
+//
+// A symmetric half-length form of the transforms halves their work: row j and
+// its mirror are replaced by their sum and difference, of which the odd and
+// the even wavenumbers see only one.  A plane is stored as its first half, a
+// gap that aligns the second half to 8 columns, and the second half; sums and
+// differences take the places of the two rows they come from.
+//
+// Why dense transforms: the sine transform of n - 2 interior nodes has length
+// 2 (n - 1), and n - 1 is odd or prime for the usual even n, so no short FFT
+// applies.  The four half-length passes are n^3 / 2 multiply-adds a plane each.
+//
+// Measured (208Pb, one step's solve, CUDA events; the sweeps it replaces in
+// brackets): 128^3 114 us (354), 64^3 41 us (227), 32^3 33 us (203), 75 x 61 x
+// 50 40 us (734: such extents had no coarse-grid correction and no tagged
+// exchange).  At 128^3, in thousands of cycles of one block: A walk 28 (latency
+// of its loads), transforms 35 (the shared loads of their operands, not the
+// multiply-adds), B 19 (its loads and the chain of eliminations), C 54, D 50
+// (latency), the four barriers with the wait for the slowest block about 25.
+#include <algorithm>
+#include <cmath>
+#include <cstring>
+#include <vector>
+
+#include "grid_sync.cuh"
+#include "hv_internal.h"
+
+namespace hv {
+namespace {
+
+constexpr int kThreads = 512;
+constexpr int kWarps = kThreads / 32;
+
+template <typename T>
+struct DirectArgs {
+    int nx, ny, nz, mx, my, mz;   // nodes, interior nodes
+    int hy, hz;                   // first halves: (m + 1) / 2 rows or columns
+    int off, wz, ps;              // second half's column, columns of a stored plane, its pitch in shared memory
+    int py;                       // pitch of the y matrices
+    int nblocks, cw, cpitch;      // columns of a phase-B group, their pitch
+    int zlen, ylen;               // floats of one z (y) matrix pair
+    int shared_tab, keep_tab;     // y matrices are the z ones; both directions stay in shared memory
+    int front;                    // floats of shared memory before the matrices
+    double dhx2i, dhy2i, dhz2i, ddiag, src_c, tol;
+    float scale;                  // hx^2: the elimination's equations are scaled by it
+    int max_iter, extrapolate;
+    long long max_spin;
+    const T *rho;
+    double *phi, *prev, *guess, *resid;  // guess: the next solve's start (interior nodes)
+    float *work, *delta;          // [mx][my][wz] spectrum, [nx][ny][nz] correction (zero on the faces)
+    const float *wz_f, *wz_i, *wy_f, *wy_i;  // matrix pairs: forward and inverse
+    const float *lamy, *lamz;     // eigenvalues times hx^2 in stored order (zero in the gaps)
+    double *partials;
+    unsigned *bar;
+    int *status;
+    double *metric;
+    int *ctl, *its_ring;
+    int ring;
+    const DirectArgs *batch;      // several solves in one launch: block -> instance, its first block
+    const int *binst, *bfirst;
+};
+
+__device__ __forceinline__ float rcp_fast(float v) {
+    float r;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(v));
+    return r;
+}
+
+__device__ __forceinline__ float lds(unsigned p) {
+    float v;
+    asm volatile("ld.shared.f32 %0, [%1];" : "=f"(v) : "r"(p) : "memory");
+    return v;
+}
+__device__ __forceinline__ void sts(unsigned p, float v) { asm volatile("st.shared.f32 [%0], %1;" ::"r"(p), "f"(v) : "memory"); }
+
+// The matrices' copy to shared memory runs under the work before their first
+// use (tab_wait and a block barrier).
+__device__ __forceinline__ void load_tab(float *dst, const float *src, int n) {
+    const unsigned d = (unsigned)__cvta_generic_to_shared(dst);
+    for (int e = 4 * threadIdx.x; e < n; e += 4 * kThreads)
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(d + 4 * e), "l"(src + e) : "memory");
+}
+__device__ __forceinline__ void tab_wait() { asm volatile("cp.async.wait_all;" ::: "memory"); }
+
+// Tile of a warp in a transform: parity (half), column groups of four and row
+// groups; lanes are 8 column groups x 4 row groups, so that a warp's loads of
+// the plane and of the matrix are each one 128-byte wavefront.
+struct Tile {
+    int par, cg, rg;
+    bool on;
+};
+template <int RT>
+__device__ __forceinline__ Tile tile_of(int wt, int CG, int RG) {
+    const int CB = (CG + 7) >> 3, RB = (RG + 3) >> 2, per = CB * RB, lane = threadIdx.x & 31;
+    Tile t;
+    t.par = wt / per;
+    const int rem = wt - t.par * per;
+    t.cg = (rem % CB) * 8 + (lane & 7);
+    t.rg = (rem / CB) * 4 + (lane >> 3);
+    t.on = t.par < 2 && t.cg < CG && t.rg < RG;
+    if (!t.on) t.par = t.cg = t.rg = 0;
+    return t;
+}
+
+// plane := plane x W along z, in place (the results wait in registers for the
+// whole block to have read its operands).  Thread tile: rows rg + RG i, four
+// columns; 12 shared loads of 16 bytes per 4 x 32 multiply-adds (RT = 8).
+template <typename T, int RT, int NT>
+__device__ __forceinline__ void transform_z(const DirectArgs<T> &a, float *P, const float *W) {
+    const int RG = (a.my + RT - 1) / RT, CG = a.off / 4, warp = threadIdx.x >> 5, ps = a.ps;
+    const int k1 = a.wz - a.off;
+    float acc[NT][RT][4];
+    Tile t[NT];
+#pragma unroll
+    for (int n = 0; n < NT; n++) {
+        t[n] = tile_of<RT>(warp + n * kWarps, CG, RG);
+        if (t[n].par && 4 * t[n].cg >= k1) t[n].on = false, t[n].cg = 0;
+#pragma unroll
+        for (int i = 0; i < RT; i++) acc[n][i][0] = acc[n][i][1] = acc[n][i][2] = acc[n][i][3] = 0.0f;
+        if (!__any_sync(0xffffffffu, t[n].on)) continue;
+        const float *w = W + t[n].par * a.off * a.off + 4 * t[n].cg;
+        const float *p = P + t[n].rg * ps + t[n].par * a.off;
+        const int K = t[n].par ? k1 : a.off;
+        for (int k = 0; k < K; k += 4) {
+            float4 v[RT];
+#pragma unroll
+            for (int i = 0; i < RT; i++) v[i] = *reinterpret_cast<const float4 *>(p + RG * i * ps + k);
+#pragma unroll
+            for (int q = 0; q < 4; q++) {
+                const float4 m = *reinterpret_cast<const float4 *>(w + (k + q) * a.off);
+#pragma unroll
+                for (int i = 0; i < RT; i++) {
+                    const float s = q == 0 ? v[i].x : q == 1 ? v[i].y : q == 2 ? v[i].z : v[i].w;
+                    acc[n][i][0] = fmaf(s, m.x, acc[n][i][0]);
+                    acc[n][i][1] = fmaf(s, m.y, acc[n][i][1]);
+                    acc[n][i][2] = fmaf(s, m.z, acc[n][i][2]);
+                    acc[n][i][3] = fmaf(s, m.w, acc[n][i][3]);
+                }
+            }
+        }
+    }
+    __syncthreads();
+#pragma unroll
+    for (int n = 0; n < NT; n++) {
+        if (!t[n].on) continue;
+#pragma unroll
+        for (int i = 0; i < RT; i++) {
+            const int r = t[n].rg + RG * i;
+            if (r < a.my)
+                *reinterpret_cast<float4 *>(P + r * ps + t[n].par * a.off + 4 * t[n].cg) =
+                    make_float4(acc[n][i][0], acc[n][i][1], acc[n][i][2], acc[n][i][3]);
+        }
+    }
+    __syncthreads();
+}
+
+// plane := W^T x plane along y: rows kk0 + i of a half from its nk rows.
+// `out` (pitch op) receives the plane; in place after a barrier when it is P.
+template <typename T, int RT, int NT>
+__device__ __forceinline__ void transform_y(const DirectArgs<T> &a, const float *P, const float *W, float *out,
+                                            int op, bool in_place) {
+    const int RG = (a.hy + RT - 1) / RT, CG = a.wz / 4, warp = threadIdx.x >> 5, ps = a.ps;
+    float acc[NT][RT][4];
+    Tile t[NT];
+#pragma unroll
+    for (int n = 0; n < NT; n++) {
+        t[n] = tile_of<RT>(warp + n * kWarps, CG, RG);
+#pragma unroll
+        for (int i = 0; i < RT; i++) acc[n][i][0] = acc[n][i][1] = acc[n][i][2] = acc[n][i][3] = 0.0f;
+        if (!__any_sync(0xffffffffu, t[n].on)) continue;
+        const int nk = t[n].par ? a.my - a.hy : a.hy;
+        const float *w = W + t[n].par * a.py * a.py + t[n].rg * RT;
+        const float *p = P + t[n].par * a.hy * ps + 4 * t[n].cg;
+#pragma unroll 4
+        for (int k = 0; k < nk; k++) {
+            const float4 v = *reinterpret_cast<const float4 *>(p + k * ps);
+            float m[RT];
+#pragma unroll
+            for (int i = 0; i < RT; i += 4)
+                *reinterpret_cast<float4 *>(m + i) = *reinterpret_cast<const float4 *>(w + k * a.py + i);
+#pragma unroll
+            for (int i = 0; i < RT; i++) {
+                acc[n][i][0] = fmaf(m[i], v.x, acc[n][i][0]);
+                acc[n][i][1] = fmaf(m[i], v.y, acc[n][i][1]);
+                acc[n][i][2] = fmaf(m[i], v.z, acc[n][i][2]);
+                acc[n][i][3] = fmaf(m[i], v.w, acc[n][i][3]);
+            }
+        }
+    }
+    if (in_place) __syncthreads();
+#pragma unroll
+    for (int n = 0; n < NT; n++) {
+        if (!t[n].on) continue;
+        const int nk = t[n].par ? a.my - a.hy : a.hy;
+#pragma unroll
+        for (int i = 0; i < RT; i++) {
+            const int kk = t[n].rg * RT + i;
+            if (kk < nk)
+                *reinterpret_cast<float4 *>(out + (size_t)(t[n].par * a.hy + kk) * op + 4 * t[n].cg) =
+                    make_float4(acc[n][i][0], acc[n][i][1], acc[n][i][2], acc[n][i][3]);
+        }
+    }
+    __syncthreads();
+}
+
+// Sums and differences of mirrored columns (rows), in the places of the pair.
+template <typename T>
+__device__ __forceinline__ void butterfly_z(const DirectArgs<T> &a, float *P) {
+    const int ha = a.mz - a.hz;
+    for (int r = threadIdx.x >> 5; r < a.my; r += kWarps)
+        for (int j = threadIdx.x & 31; j < ha; j += 32) {
+            float *u = P + r * a.ps + j, *v = P + r * a.ps + a.off + ha - 1 - j;
+            const float s = *u, d = *v;
+            *u = s + d;
+            *v = s - d;
+        }
+    __syncthreads();
+}
+template <typename T>
+__device__ __forceinline__ void butterfly_y(const DirectArgs<T> &a, float *P) {
+    const int ha = a.my - a.hy;
+    for (int j = threadIdx.x >> 5; j < ha; j += kWarps)
+        for (int c = 4 * (threadIdx.x & 31); c < a.wz; c += 128) {
+            float4 *u = reinterpret_cast<float4 *>(P + j * a.ps + c);
+            float4 *v = reinterpret_cast<float4 *>(P + (a.my - 1 - j) * a.ps + c);
+            const float4 s = *u, d = *v;
+            *u = make_float4(s.x + d.x, s.y + d.y, s.z + d.z, s.w + d.w);
+            *v = make_float4(s.x - d.x, s.y - d.y, s.z - d.z, s.w - d.w);
+        }
+    __syncthreads();
+}
+
+// Walks the interior rows of x plane i: each warp takes 32 consecutive z of a
+// run of y rows, kU rows at a time.  load(id, interior) is the field whose
+// 7-point stencil is formed: its y neighbours roll through registers, its z
+// neighbours come from the lanes (the edge lanes load theirs), its x
+// neighbours are loaded.  pre(id) reads what use() needs besides at a node.
+// All loads of the kU rows are issued before anything is used or stored: the
+// walk is bound by the latency of its loads.
+template <int kU, typename T, typename Load, typename Pre, typename Use>
+__device__ __forceinline__ void walk_plane(const DirectArgs<T> &a, int i, Load load, Pre pre, Use use) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int nchunk = (a.mz + 31) >> 5, nseg = max(1, kWarps / nchunk);
+    const int rows = (a.my + nseg - 1) / nseg;
+    const long long sx = (long long)a.ny * a.nz;
+    const bool xm_in = i > 1, xp_in = i < a.nx - 2;
+    for (int item = warp; item < nchunk * nseg; item += kWarps) {
+        const int ch = item % nchunk, sg = item / nchunk;
+        const int y0 = 1 + sg * rows, y1 = min(y0 + rows, a.ny - 1);
+        if (y0 >= y1) continue;
+        const int z0 = 1 + 32 * ch, zr = z0 + lane, z = min(zr, a.nz - 1);
+        const bool zin = zr <= a.nz - 2;
+        // the node past the lane's end of the run (z0 - 1 or z0 + 32)
+        const bool edge = lane == 0 || (lane == 31 && zr + 1 <= a.nz - 1);
+        const int ze = lane == 0 ? z0 - 1 : min(zr + 1, a.nz - 1);
+        const bool ze_in = ze >= 1 && ze <= a.nz - 2;
+        long long id = i * sx + (long long)y0 * a.nz + z, ide = i * sx + (long long)y0 * a.nz + ze;
+        auto ym = load(id - a.nz, zin && y0 > 1), c = load(id, zin);
+        using V = decltype(c);
+        for (int y = y0; y < y1; y += kU) {
+            V yn[kU], xm[kU], xp[kU], e[kU];
+            decltype(pre(id)) n[kU];
+#pragma unroll
+            for (int u = 0; u < kU; u++) {
+                // rows past the run's end repeat its last one
+                const int q = min(u, y1 - 1 - y), d = q * a.nz;
+                yn[u] = load(id + d + a.nz, zin && y + q + 1 <= a.ny - 2);
+                xm[u] = load(id + d - sx, xm_in && zin);
+                xp[u] = load(id + d + sx, xp_in && zin);
+                n[u] = pre(id + d);
+                e[u] = V(0);
+                if (edge) e[u] = load(ide + d, ze_in);
+            }
+#pragma unroll
+            for (int u = 0; u < kU; u++) {
+                const V up = __shfl_up_sync(0xffffffffu, c, 1), dn = __shfl_down_sync(0xffffffffu, c, 1);
+                if (zin && y + u < y1)
+                    use(id + u * a.nz, y + u, zr, c, (double)xm[u] + (double)xp[u], (double)ym + (double)yn[u],
+                        (double)(lane == 0 ? e[u] : up) + (double)(lane == 31 ? e[u] : dn), n[u]);
+                ym = c;
+                c = yn[u];
+            }
+            id += kU * a.nz;
+            ide += kU * a.nz;
+        }
+    }
+}
+
+// Phase B: the systems (2 + l) x_i - x_(i-1) - x_(i+1) = f_i of a group of
+// columns, l the column's hx^2 (lam_y + lam_z).  Elimination from both ends
+// towards the middle by two half-warps (the coefficients c_i = 1 / (2 + l -
+// c_(i-1)) are the same from either end), then substitution outwards.  e = 1 -
+// c is carried instead of c, e' = (l + e) / (1 + l + e): all terms positive,
+// so the smooth columns (l ~ 1e-3) keep full relative accuracy.  Bound by the
+// serial chain, mx / 2 steps of an add, a reciprocal and two products.
+template <typename T>
+__device__ __forceinline__ void solve_columns(const DirectArgs<T> &a, float *sm, int group) {
+    const int ncol = a.my * a.wz, c0 = group * a.cw, n = min(a.cw, ncol - c0), mx = a.mx, pitch = a.cpitch;
+    float *f = sm, *cc = sm + (size_t)mx * pitch;
+    const int quads = n >> 2, xs = kThreads / quads, xq = threadIdx.x / quads, q4 = 4 * (threadIdx.x - xq * quads);
+    float *const g = a.work + c0 + q4;
+    constexpr int kU = 8;  // rows in flight per thread
+    for (int x = xq < xs ? xq : mx; x < mx; x += kU * xs) {
+        float4 v[kU];
+#pragma unroll
+        for (int u = 0; u < kU; u++)
+            if (x + u * xs < mx) v[u] = __ldcg(reinterpret_cast<const float4 *>(g + (size_t)(x + u * xs) * ncol));
+#pragma unroll
+        for (int u = 0; u < kU; u++)
+            if (x + u * xs < mx) *reinterpret_cast<float4 *>(f + (x + u * xs) * pitch + q4) = v[u];
+    }
+    __syncthreads();
+    const int lane = threadIdx.x & 31, col = (threadIdx.x >> 5) * 16 + (lane & 15), side = lane >> 4;
+    const int h = mx >> 1;
+    if ((threadIdx.x >> 5) * 16 < n) {
+        // columns past the group's end (n is a multiple of four) run on what
+        // their place holds; nothing reads their results
+        const int gcol = c0 + min(col, n - 1), ky = gcol / a.wz;
+        const float l = __ldg(a.lamy + ky) + __ldg(a.lamz + gcol - ky * a.wz);
+        // byte addresses in shared memory: the column's rows from this side's
+        // end, and its coefficients
+        const int pb = 4 * pitch, step = side ? -pb : pb;
+        unsigned fp = (unsigned)__cvta_generic_to_shared(f + col + (side ? (mx - 1) * pitch : 0));
+        unsigned cp = (unsigned)__cvta_generic_to_shared(cc + col);
+        float e = 1.0f, y = 0.0f, rc = 0.0f;
+        auto forward = [&](float fv) {
+            const float t = l + e;
+            rc = rcp_fast(1.0f + t);
+            e = t * rc;
+            y = (fv + y) * rc;
+            sts(fp, y);
+            sts(cp, rc);  // both sides write the column's one coefficient
+            fp += step;
+            cp += pb;
+        };
+        int i = 0;
+        for (; i + 4 <= h; i += 4) {
+            const float f0 = lds(fp), f1 = lds(fp + step), f2 = lds(fp + 2 * step), f3 = lds(fp + 3 * step);
+            forward(f0);
+            forward(f1);
+            forward(f2);
+            forward(f3);
+        }
+        for (; i < h; i++) forward(lds(fp));
+        const float other = __shfl_xor_sync(0xffffffffu, y, 16);
+        float x;
+        if (mx & 1) {
+            // the middle node, between the two sides' last ones
+            x = (lds(fp) + y + other) / (l + 2.0f * e);
+            __syncwarp();
+            sts(fp, x);
+        } else {
+            // the other side's last node: x_other = (y_other + c y) / (1 - c^2)
+            x = (other + rc * y) / (e * (1.0f + rc));
+        }
+        __syncwarp();
+        auto back = [&](float cv, float yv) {
+            x = fmaf(cv, x, yv);
+            fp -= step;
+            sts(fp, x);
+        };
+        for (; i >= 4; i -= 4) {
+            const float c3 = lds(cp - pb), c2 = lds(cp - 2 * pb), c1 = lds(cp - 3 * pb), c0v = lds(cp - 4 * pb);
+            const float y3 = lds(fp - step), y2 = lds(fp - 2 * step), y1 = lds(fp - 3 * step), y0 = lds(fp - 4 * step);
+            back(c3, y3);
+            back(c2, y2);
+            back(c1, y1);
+            back(c0v, y0);
+            cp -= 4 * pb;
+        }
+        for (; i > 0; i--) {
+            back(lds(cp - pb), lds(fp - step));
+            cp -= pb;
+        }
+    }
+    __syncthreads();
+    for (int x = xq < xs ? xq : mx; x < mx; x += xs)
+        __stcg(reinterpret_cast<float4 *>(g + (size_t)x * ncol), *reinterpret_cast<const float4 *>(f + x * pitch + q4));
+    __syncthreads();
+}
+
+// What the last phase reads at a node: the residual, the solve's start, phi
+// and the solution before it.
+struct Node {
+    double r, start, phi, prev;
+};
+
+template <typename T, int RT, int NT>
+__device__ __forceinline__ void direct_body(const DirectArgs<T> &a, const int b) {
+    extern __shared__ __align__(16) float sm[];
+    __shared__ double s_tot[2];
+    const int tid = threadIdx.x;
+    int *err = a.status;
+    // shared memory: plane | z matrices | y matrices (| the inverse ones).
+    // Phase B's columns lie where the plane lies; matrices that do not fit
+    // beside them are loaded anew by each phase
+    float *P = sm, *tz = sm + a.front;
+    float *ty = a.shared_tab ? tz : tz + a.zlen;
+    const int one = a.zlen + (a.shared_tab ? 0 : a.ylen);
+    float *tzi = a.keep_tab ? tz + one : tz, *tyi = a.keep_tab ? ty + one : ty;
+    const int step = a.ctl[0];
+    const int hist = a.extrapolate ? a.ctl[2] : 0;
+    const long long sx = (long long)a.ny * a.nz;
+
+    auto load_dir = [&](bool inverse) {
+        if (a.keep_tab) return;
+        load_tab(tz, inverse ? a.wz_i : a.wz_f, a.zlen);
+        if (!a.shared_tab) load_tab(ty, inverse ? a.wy_i : a.wy_f, a.ylen);
+    };
+    if (a.keep_tab) {
+        load_tab(tz, a.wz_f, a.zlen);
+        load_tab(tzi, a.wz_i, a.zlen);
+        if (!a.shared_tab) {
+            load_tab(ty, a.wy_f, a.ylen);
+            load_tab(tyi, a.wy_i, a.ylen);
+        }
+    }
+    // the start: the extrapolation that the last solve left (none without
+    // earlier solutions), the boundary values of phi on the faces
+    const double *start = hist > 0 ? a.guess : a.phi;
+    auto load_start = [&](long long id, bool interior) { return (interior ? start : a.phi)[id]; };
+    auto load_delta = [&](long long id, bool) { return __ldcg(a.delta + id); };
+    auto to_plane = [&](int y, int z, double r) {
+        const int q = z - 1;
+        P[(y - 1) * a.ps + (q < a.hz ? q : a.off + q - a.hz)] = (float)r * a.scale;
+    };
+    auto totals = [&](double &u, double &v) {
+        if (tid < 32) {
+            double su = 0.0, sv = 0.0;
+            for (int q = tid; q < a.nblocks; q += 32) {
+                su += __ldcg(a.partials + 2 * q);
+                sv += __ldcg(a.partials + 2 * q + 1);
+            }
+            for (int o = 16; o > 0; o >>= 1) {
+                su += __shfl_xor_sync(0xffffffffu, su, o);
+                sv += __shfl_xor_sync(0xffffffffu, sv, o);
+            }
+            if (tid == 0) {
+                s_tot[0] = su;
+                s_tot[1] = sv;
+            }
+        }
+        __syncthreads();
+        u = s_tot[0];
+        v = s_tot[1];
+    };
+    // The first correction of a solve: phi := v, the solution before it moves
+    // to prev, and the next solve's start is extrapolated in time while all its
+    // terms are at hand -- 3 v - 3 phi + prev, or 2 v - phi while only one
+    // earlier solution is held (a cubic guess measured worse: it amplifies the
+    // step-to-step particle noise).  Reading that one field in the next solve's
+    // stencil instead of three moves 36 bytes a node fewer.
+    auto store_first = [&](long long id, double v, double phi, double prev) {
+        if (a.extrapolate) {
+            a.guess[id] = a.extrapolate == 2 && hist > 0 ? 3.0 * (v - phi) + prev : 2.0 * v - phi;
+            a.prev[id] = phi;
+        }
+        a.phi[id] = v;
+    };
+    // a later one adds its share of the extrapolation too
+    const double again = a.extrapolate == 2 && hist > 0 ? 3.0 : 2.0;
+
+    int its = 0;
+    double rel = 0.0, bsum = 0.0;
+    bool converged = false;
+    while (true) {
+        // ---- A: residual of the plane and its forward transforms -----------
+        double rr = 0.0, bb = 0.0;
+        load_dir(false);
+        // the stored plane's gaps are zero and stay so until phase B
+        const int gap0 = a.off - a.hz, gaps = a.wz - a.mz;
+        for (int e = tid; e < a.my * gaps; e += kThreads) {
+            const int r = e / gaps, q = e - r * gaps;
+            P[r * a.ps + (q < gap0 ? a.hz + q : a.wz - gaps + q)] = 0.0f;
+        }
+        for (int i = 1 + b; i <= a.mx; i += a.nblocks) {
+            if (its == 0) {
+                walk_plane<4>(
+                    a, i, load_start, [&](long long id) { return __ldg(a.rho + id); },
+                    [&](long long id, int y, int z, double c, double xs, double ys, double zs, T rho) {
+                        const double bv = a.src_c * (double)rho;
+                        const double r = bv + xs * a.dhx2i + ys * a.dhy2i + zs * a.dhz2i - a.ddiag * c;
+                        a.resid[id] = r;
+                        rr += r * r;
+                        bb += bv * bv;
+                        to_plane(y, z, r);
+                    });
+            } else {
+                walk_plane<4>(
+                    a, i, load_delta, [&](long long id) { return a.resid[id]; },
+                    [&](long long id, int y, int z, float c, double xs, double ys, double zs, double r0) {
+                        const double r = r0 + xs * a.dhx2i + ys * a.dhy2i + zs * a.dhz2i - a.ddiag * (double)c;
+                        a.resid[id] = r;
+                        to_plane(y, z, r);
+                    });
+            }
+            tab_wait();
+            __syncthreads();
+            butterfly_z(a, P);
+            transform_z<T, RT, NT>(a, P, tz);
+            butterfly_y(a, P);
+            transform_y<T, RT, NT>(a, P, ty, a.work + (size_t)(i - 1) * a.my * a.wz, a.wz, false);
+        }
+        if (its == 0) {
+            block_sum2(rr, bb);
+            if (tid == 0) {
+                a.partials[2 * b] = rr;
+                a.partials[2 * b + 1] = bb;
+            }
+        }
+        if (!grid_barrier(a.bar, a.nblocks, err, a.max_spin)) return;
+        if (its == 0) {
+            double u;
+            totals(u, bsum);
+            rel = bsum > 0.0 ? sqrt(u / bsum) : sqrt(u);
+            converged = rel <= a.tol;
+            if (converged || !(rel == rel)) {
+                for (int i = 1 + b; i <= a.mx; i += a.nblocks)
+                    for (int e = tid; e < a.my * a.mz; e += kThreads) {
+                        const long long id = i * sx + (long long)(1 + e / a.mz) * a.nz + 1 + e % a.mz;
+                        store_first(id, start[id], a.phi[id], a.prev[id]);
+                    }
+                break;
+            }
+        }
+        // ---- B: along x -------------------------------------------------------
+        const int groups = (a.my * a.wz + a.cw - 1) / a.cw;
+        for (int g = b; g < groups; g += a.nblocks) solve_columns(a, sm, g);
+        if (!grid_barrier(a.bar, a.nblocks, err, a.max_spin)) return;
+        // ---- C: inverse transforms -------------------------------------------
+        load_dir(true);
+        for (int i = 1 + b; i <= a.mx; i += a.nblocks) {
+            const float *src = a.work + (size_t)(i - 1) * a.my * a.wz;
+            // a row per group of lanes, eight rows in flight per thread
+            const int quads = a.wz >> 2, rs = kThreads / quads, rq = tid / quads, q4 = 4 * (tid - rq * quads);
+            for (int r = rq < rs ? rq : a.my; r < a.my; r += 8 * rs) {
+                float4 v[8];
+#pragma unroll
+                for (int u = 0; u < 8; u++)
+                    if (r + u * rs < a.my) v[u] = __ldcg(reinterpret_cast<const float4 *>(src + (r + u * rs) * a.wz + q4));
+#pragma unroll
+                for (int u = 0; u < 8; u++)
+                    if (r + u * rs < a.my) *reinterpret_cast<float4 *>(P + (r + u * rs) * a.ps + q4) = v[u];
+            }
+            tab_wait();
+            __syncthreads();
+            transform_z<T, RT, NT>(a, P, tzi);
+            butterfly_z(a, P);
+            transform_y<T, RT, NT>(a, P, tyi, P, a.ps, true);
+            const int hay = a.my - a.hy;
+            for (int j = tid >> 5; j < a.hy; j += kWarps)
+                for (int q = tid & 31; q < a.mz; q += 32) {
+                    const int c = q < a.hz ? q : a.off + q - a.hz;
+                    const float o = P[j * a.ps + c];
+                    float *d = a.delta + i * sx + q + 1;
+                    if (j < hay) {
+                        const float e = P[(a.my - 1 - j) * a.ps + c];
+                        __stcg(d + (long long)(j + 1) * a.nz, o + e);
+                        __stcg(d + (long long)(a.my - j) * a.nz, o - e);
+                    } else {
+                        __stcg(d + (long long)(j + 1) * a.nz, o);
+                    }
+                }
+            __syncthreads();
+        }
+        if (!grid_barrier(a.bar, a.nblocks, err, a.max_spin)) return;
+        // ---- D: phi += delta, the FP64 residual of the new phi ---------------
+        rr = bb = 0.0;
+        for (int i = 1 + b; i <= a.mx; i += a.nblocks)
+            if (its == 0)
+                walk_plane<4>(
+                    a, i, load_delta,
+                    [&](long long id) { return Node{a.resid[id], start[id], a.phi[id], a.prev[id]}; },
+                    [&](long long id, int, int, float c, double xs, double ys, double zs, const Node &n) {
+                        const double r = n.r + xs * a.dhx2i + ys * a.dhy2i + zs * a.dhz2i - a.ddiag * (double)c;
+                        rr += r * r;
+                        store_first(id, n.start + (double)c, n.phi, n.prev);
+                    });
+            else
+                walk_plane<4>(
+                    a, i, load_delta,
+                    [&](long long id) { return Node{a.resid[id], a.extrapolate ? a.guess[id] : 0.0, a.phi[id], 0.0}; },
+                    [&](long long id, int, int, float c, double xs, double ys, double zs, const Node &n) {
+                        const double r = n.r + xs * a.dhx2i + ys * a.dhy2i + zs * a.dhz2i - a.ddiag * (double)c;
+                        rr += r * r;
+                        a.phi[id] = n.phi + (double)c;
+                        if (a.extrapolate) a.guess[id] = n.start + again * (double)c;
+                    });
+        block_sum2(rr, bb);
+        if (tid == 0) a.partials[2 * b] = rr;
+        if (!grid_barrier(a.bar, a.nblocks, err, a.max_spin)) return;
+        double u, none;
+        totals(u, none);
+        rel = bsum > 0.0 ? sqrt(u / bsum) : sqrt(u);
+        converged = rel <= a.tol;
+        its++;
+        if (converged || its >= a.max_iter || !(rel == rel)) break;
+    }
+    if (b == 0 && tid == 0) {
+        a.status[1] = its;
+        a.status[2] = converged ? 1 : 0;
+        a.status[3] = its + 1;
+        a.metric[0] = rel;
+        a.ctl[1] = max(its, 1);
+        // solutions held before phi; a start from phi leaves none
+        a.ctl[2] = a.extrapolate ? min(a.ctl[2] + 1, 2) : 0;
+        if (a.its_ring) a.its_ring[step % a.ring] = converged ? its : -its;
+    }
+}
+
+// One solve, or several in one launch (kBatch): block blockIdx.x works on
+// instance binst[blockIdx.x], as its block blockIdx.x - bfirst[instance].
+template <typename T, int RT, int NT, bool kBatch>
+__global__ void __launch_bounds__(kThreads, 1) k_poisson_direct(DirectArgs<T> p) {
+    if constexpr (kBatch) {
+        __shared__ DirectArgs<T> inst;
+        const int q = p.binst[blockIdx.x];
+        if (threadIdx.x == 0) inst = p.batch[q];
+        __syncthreads();
+        direct_body<T, RT, NT>(inst, (int)blockIdx.x - p.bfirst[q]);
+    } else {
+        direct_body<T, RT, NT>(p, (int)blockIdx.x);
+    }
+}
+
+int up(int v, int q) { return (v + q - 1) / q * q; }
+
+// The tile counts of both transforms for row tiles of RT.
+int warp_tiles(const Geom &g, int off, int wz, int RT) {
+    auto tiles = [](int CG, int RG) { return 2 * ((CG + 7) / 8) * ((RG + 3) / 4); };
+    const int my = g.ny - 2, hy = (my + 1) / 2;
+    return std::max(tiles(off / 4, (my + RT - 1) / RT), tiles(wz / 4, (hy + RT - 1) / RT));
+}
+
+// One axis' matrix pair (odd and even wavenumbers), forward [position][k] and
+// inverse [k][position], zero-padded to `pitch` squares.
+void sine_tables(int m, int pitch, std::vector<float> &fwd, std::vector<float> &inv) {
+    const int h = (m + 1) / 2, ha = m - h;
+    fwd.assign((size_t)2 * pitch * pitch, 0.0f);
+    inv.assign((size_t)2 * pitch * pitch, 0.0f);
+    const double s = std::sqrt(2.0 / (m + 1));
+    for (int par = 0; par < 2; par++)
+        for (int p = 0; p < (par ? ha : h); p++)
+            for (int k = 0; k < (par ? ha : h); k++) {
+                const int j = par ? ha - 1 - p : p, w = 2 * k + 1 + par;
+                // the argument reduced exactly before the sine
+                const long long r = ((long long)(j + 1) * w) % (2ll * (m + 1));
+                const float v = (float)(s * std::sin(kPi * (double)r / (m + 1)));
+                fwd[((size_t)par * pitch + p) * pitch + k] = v;
+                inv[((size_t)par * pitch + k) * pitch + p] = v;
+            }
+}
+
+template <bool kBatch>
+const void *direct_kernel(int rt, int nt) {
+    if (rt == 4) return (const void *)k_poisson_direct<float, 4, 1, kBatch>;
+    return nt == 1   ? (const void *)k_poisson_direct<float, 8, 1, kBatch>
+           : nt == 2 ? (const void *)k_poisson_direct<float, 8, 2, kBatch>
+                     : (const void *)k_poisson_direct<float, 8, 3, kBatch>;
+}
+
+DirectArgs<float> direct_args(hv_ctx *c, const float *rho, int *ctl, int *its_ring, int ring, int nblocks) {
+    const PoissonDirect &d = c->fused.direct;
+    const Geom &g = c->geom;
+    DirectArgs<float> a;
+    std::memset(&a, 0, sizeof(a));
+    a.nx = g.nx;
+    a.ny = g.ny;
+    a.nz = g.nz;
+    a.mx = g.nx - 2;
+    a.my = g.ny - 2;
+    a.mz = g.nz - 2;
+    a.hy = (a.my + 1) / 2;
+    a.hz = (a.mz + 1) / 2;
+    a.off = d.off;
+    a.wz = d.wz;
+    a.ps = d.ps;
+    a.py = d.py;
+    a.zlen = 2 * d.off * d.off;
+    a.ylen = 2 * d.py * d.py;
+    a.shared_tab = d.shared_tab;
+    a.keep_tab = d.keep_tab;
+    a.front = d.front;
+    a.nblocks = nblocks;
+    // phase B: an equal share of the columns per block, in sixteens (a
+    // half-warp each from either end), as many as shared memory holds
+    const int ncol = a.my * a.wz;
+    a.cw = std::min(up((ncol + nblocks - 1) / nblocks, 16), d.cw_max);
+    a.cpitch = a.cw;
+    const double dx = 2.0 * g.dmx / g.nx, dy = 2.0 * g.dmy / g.ny, dz = 2.0 * g.dmz / g.nz;
+    a.dhx2i = 1.0 / (dx * dx);
+    a.dhy2i = 1.0 / (dy * dy);
+    a.dhz2i = 1.0 / (dz * dz);
+    a.ddiag = 2.0 * (a.dhx2i + a.dhy2i + a.dhz2i);
+    a.src_c = 4.0 * kPi * kE2;
+    a.scale = (float)(dx * dx);
+    a.tol = c->params.sor.tol;
+    a.max_iter = c->params.sor.max_iter;
+    a.extrapolate = c->fast.sor_warm_start == HV_WARM_EXTRAPOLATE ? 1 : c->fast.sor_warm_start == HV_WARM_QUADRATIC ? 2 : 0;
+    a.max_spin = c->fast.sor_wait_limit > 0 ? c->fast.sor_wait_limit : kDefaultSpin;
+    a.rho = rho;
+    a.phi = c->fused.phi64;
+    a.prev = c->fused.phi64_prev;
+    a.guess = c->fused.phi64_prev2;
+    a.resid = c->fused.sor.resid;
+    a.work = d.work;
+    a.delta = d.delta;
+    a.wz_f = d.tables;
+    a.wz_i = a.wz_f + a.zlen;
+    a.wy_f = a.wz_i + a.zlen;
+    a.wy_i = a.wy_f + a.ylen;
+    a.lamy = a.wy_i + a.ylen;
+    a.lamz = a.lamy + up(a.my, 4);
+    a.partials = d.partials;
+    a.bar = d.bar;
+    a.status = c->fused.sor.status;
+    a.metric = c->fused.sor.metric;
+    a.ctl = ctl;
+    a.its_ring = its_ring;
+    a.ring = ring;
+    return a;
+}
+
+}  // namespace
+
+// Plans the direct solve of a float context: it runs on every grid whose y-z
+// plane, with the transforms' matrices, fits in one block's shared memory and
+// registers (about 174 nodes per axis); larger planes keep the sweeps.
+hv_status poisson_plan(hv_ctx *c) {
+    PoissonDirect &d = c->fused.direct;
+    const Geom &g = c->geom;
+    d.ok = false;
+    if (c->prec != HV_F32) return HV_OK;
+    const int mx = g.nx - 2, my = g.ny - 2, mz = g.nz - 2;
+    const int hy = (my + 1) / 2, hz = (mz + 1) / 2;
+    d.off = up(hz, 8);
+    d.wz = d.off + up(mz - hz, 4);
+    d.py = up(hy, 8);
+    d.ps = d.wz;
+    while (d.ps % 32 != 4 && d.ps % 32 != 12 && d.ps % 32 != 20 && d.ps % 32 != 28) d.ps += 4;
+    d.rt = warp_tiles(g, d.off, d.wz, 4) <= kWarps ? 4 : 8;
+    d.nt = (warp_tiles(g, d.off, d.wz, d.rt) + kWarps - 1) / kWarps;
+    if (d.nt > 3) return HV_OK;
+    int optin = 0;
+    HV_CUDA(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, c->device));
+    const size_t limit = optin - 4096;  // the kernels' static shared memory
+    const size_t plane = (size_t)up(my, d.rt) * d.ps, zl = (size_t)2 * d.off * d.off, yl = (size_t)2 * d.py * d.py;
+    d.shared_tab = my == mz ? 1 : 0;
+    const size_t one = zl + (d.shared_tab ? 0 : yl);
+    // phase B's columns and their coefficients lie where the plane lies; the
+    // matrices follow, both directions where they fit, else over the columns
+    const int ncol = my * d.wz;
+    const size_t col = (size_t)(mx + mx / 2 + 1);
+    int want = std::min(up((ncol + c->sm_count - 1) / c->sm_count, 16), 256);
+    while (want > 16 && col * want * sizeof(float) > limit) want -= 16;
+    if (col * want * sizeof(float) > limit) return HV_OK;
+    d.cw_max = want;
+    const size_t both = std::max(plane, col * want) + 2 * one;
+    d.keep_tab = both * sizeof(float) <= limit ? 1 : 0;
+    const size_t words = d.keep_tab ? both : std::max(plane + one, col * want);
+    d.front = (int)(d.keep_tab ? both - 2 * one : plane);
+    d.smem = words * sizeof(float);
+    if (d.smem > limit) return HV_OK;
+    // one block per x plane, more where they shorten phase B
+    d.nblocks = std::min(c->sm_count, std::max(mx, (ncol + 31) / 32));
+    for (const void *k : {direct_kernel<false>(d.rt, d.nt), direct_kernel<true>(d.rt, d.nt)}) {
+        HV_TRY(allow_max_dynamic_smem(k, c->device));
+        int per_sm = 0;
+        HV_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, kThreads, d.smem));
+        if (per_sm < 1) return HV_OK;
+    }
+    std::vector<float> zf, zi, yf, yi, lam;
+    sine_tables(mz, d.off, zf, zi);
+    sine_tables(my, d.py, yf, yi);
+    const double dx = 2.0 * g.dmx / g.nx, dy = 2.0 * g.dmy / g.ny, dz = 2.0 * g.dmz / g.nz;
+    auto eigen = [](int m, int w) { const double s = std::sin(kPi * w / (2.0 * (m + 1))); return 4.0 * s * s; };
+    lam.assign((size_t)up(my, 4) + d.wz, 0.0f);
+    for (int r = 0; r < my; r++)
+        lam[r] = (float)(eigen(my, r < hy ? 2 * r + 1 : 2 * (r - hy) + 2) * (dx * dx) / (dy * dy));
+    for (int q = 0; q < mz; q++)
+        lam[up(my, 4) + (q < hz ? q : d.off + q - hz)] =
+            (float)(eigen(mz, q < hz ? 2 * q + 1 : 2 * (q - hz) + 2) * (dx * dx) / (dz * dz));
+    std::vector<float> all;
+    for (const auto *v : {&zf, &zi, &yf, &yi, &lam}) all.insert(all.end(), v->begin(), v->end());
+    // one allocation: the tables, the spectrum, the correction (zero on the
+    // faces), the partial sums and the barrier words
+    const size_t nw = (size_t)mx * ncol, np = 4 * (size_t)c->sm_count;
+    const size_t at_work = up((int)all.size(), 64), at_delta = at_work + (nw + 63) / 64 * 64;
+    const size_t at_part = at_delta + ((size_t)g.G + 63) / 64 * 64, words_all = at_part + np + 64;
+    HV_CUDA(cudaMalloc((void **)&d.tables, words_all * sizeof(float)));
+    d.work = d.tables + at_work;
+    d.delta = d.tables + at_delta;
+    d.partials = reinterpret_cast<double *>(d.tables + at_part);
+    d.bar = reinterpret_cast<unsigned *>(d.tables + at_part + np);
+    HV_CUDA(cudaMemsetAsync(d.delta, 0, (words_all - at_delta) * sizeof(float), c->stream));
+    HV_CUDA(cudaMemcpyAsync(d.tables, all.data(), all.size() * sizeof(float), cudaMemcpyHostToDevice, c->stream));
+    HV_CUDA(cudaStreamSynchronize(c->stream));
+    d.ok = true;
+    return HV_OK;
+}
+
+void poisson_release(hv_ctx *c) {
+    PoissonDirect &d = c->fused.direct;
+    if (d.tables) cudaFree(d.tables);
+    d = PoissonDirect();
+}
+
+// Whether this context's solves take the direct form: float, the
+// relative-residual rule, and the default solver options (the corrected cycles
+// on, the tagged exchange not replaced by phase counters).
+bool poisson_direct_runs(const hv_ctx *c) {
+    return c->prec == HV_F32 && c->fused.direct.ok && c->fast.sor_coarse &&
+           c->fast.sor_exchange == HV_SOR_EXCHANGE_AUTO && c->params.sor.criterion == HV_SOR_REL_RESIDUAL;
+}
+
+hv_status poisson_launch(hv_ctx *c, const float *rho, int *ctl, int *its_ring, int ring, bool step_solve) {
+    const PoissonDirect &d = c->fused.direct;
+    DirectArgs<float> a = direct_args(c, rho, ctl, its_ring, ring, d.nblocks);
+    if (!step_solve) a.extrapolate = 0;
+    void *args[] = {&a};
+    HV_CUDA(cudaLaunchCooperativeKernel(direct_kernel<false>(d.rt, d.nt), dim3(d.nblocks), dim3(kThreads), args,
+                                        d.smem, c->stream));
+    return HV_OK;
+}
+
+// The barrier words of a solve that gave up are not back at zero.
+hv_status poisson_clear(hv_ctx *c) {
+    if (c->fused.direct.bar) HV_CUDA(cudaMemsetAsync(c->fused.direct.bar, 0, sizeof(unsigned) * 2, c->stream));
+    return HV_OK;
+}
+
+}  // namespace hv

@@ -43,6 +43,7 @@
 #include <cstring>
 #include <vector>
 
+#include "grid_sync.cuh"
 #include "hv_internal.h"
 
 namespace hv {
@@ -57,11 +58,6 @@ constexpr int kSorThreads = 1024;
 // at 128^3 (2.9e-7) and three on the other grids; measured on the GPU at
 // 128^3, 13 sweeps at 1.8 took three cycles in 999 of 1000 solves.
 constexpr double kCoarseOmega = 1.7;
-// default bounds of the device-side waits (hv_fast_options.sor_wait_limit
-// replaces both): polls of a grid barrier or a neighbour's phase counter before
-// the wait gives up (~1 s), and polls of one tagged mirror entry
-constexpr long long kDefaultSpin = 1ll << 24;
-constexpr long long kDefaultPoll = 1ll << 22;
 #ifndef HV_SOR_POLL_NS
 #define HV_SOR_POLL_NS 64
 #endif
@@ -106,46 +102,6 @@ struct SorArgs {
     const int *binst, *bfirst;
 };
 
-__device__ __forceinline__ unsigned ld_relaxed(const unsigned *p) {
-    unsigned v;
-    asm volatile("ld.relaxed.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
-    return v;
-}
-__device__ __forceinline__ void st_release(unsigned *p, unsigned v) {
-    asm volatile("st.release.gpu.global.u32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
-}
-__device__ __forceinline__ void fence_acq_rel() { asm volatile("fence.acq_rel.gpu;" ::: "memory"); }
-__device__ __forceinline__ int ld_volatile(const int *p) { return *(const volatile int *)p; }
-
-// Grid barrier for co-resident blocks; false when a wait timed out or another
-// block reported an error.
-__device__ bool grid_barrier(unsigned *bar, int nblocks, int *err, long long max_spin) {
-    __shared__ int ok;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        ok = 1;
-        unsigned gen = ld_relaxed(bar + 1);
-        fence_acq_rel();
-        unsigned arrived = atomicAdd(bar, 1u) + 1u;
-        if (arrived == (unsigned)nblocks) {
-            atomicExch(bar, 0u);
-            st_release(bar + 1, gen + 1u);
-        } else {
-            long long spin = 0;
-            while (ld_relaxed(bar + 1) == gen) {
-                if (++spin > max_spin || ld_volatile(err)) {
-                    atomicExch(err, 1);
-                    ok = 0;
-                    break;
-                }
-            }
-        }
-        fence_acq_rel();
-    }
-    __syncthreads();
-    return ok;
-}
-
 // Waits until every neighbouring block has published `target` phases: lane q
 // of warp 0 polls neighbour q with relaxed loads, then one acquire fence; the
 // block barrier extends the ordering to every thread.
@@ -185,32 +141,6 @@ __device__ bool wait_neighbours(const SorArgs<T, S> &a, int bx, int by, unsigned
 __device__ __forceinline__ void publish(unsigned *phase_slot, unsigned value) {
     __syncthreads();
     if (threadIdx.x == 0) st_release(phase_slot, value);
-}
-
-// Deterministic block sum of two doubles (fixed shuffle tree, fixed warp order);
-// the result is valid in thread 0.
-__device__ void block_sum2(double &u, double &v) {
-    __shared__ double su[kSorThreads / 32], sv[kSorThreads / 32];
-    for (int o = 16; o > 0; o >>= 1) {
-        u += __shfl_xor_sync(0xffffffffu, u, o);
-        v += __shfl_xor_sync(0xffffffffu, v, o);
-    }
-    const int w = threadIdx.x >> 5, l = threadIdx.x & 31;
-    __syncthreads();
-    if (l == 0) {
-        su[w] = u;
-        sv[w] = v;
-    }
-    __syncthreads();
-    if (w == 0) {
-        const int nw = blockDim.x >> 5;
-        u = l < nw ? su[l] : 0.0;
-        v = l < nw ? sv[l] : 0.0;
-        for (int o = 16; o > 0; o >>= 1) {
-            u += __shfl_xor_sync(0xffffffffu, u, o);
-            v += __shfl_xor_sync(0xffffffffu, v, o);
-        }
-    }
 }
 
 template <typename S>
@@ -1693,7 +1623,7 @@ hv_status sor_fast_clear_error(hv_ctx *c) {
     const SorFast &f = c->fused.sor;
     HV_CUDA(cudaMemsetAsync(f.status, 0, sizeof(int) * 4, c->stream));
     HV_CUDA(cudaMemsetAsync(f.phase, 0, sizeof(unsigned) * (f.nblocks + 2), c->stream));
-    return HV_OK;
+    return poisson_clear(c);
 }
 
 hv_status sor_fast_plan(hv_ctx *c) {

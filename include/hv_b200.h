@@ -341,19 +341,22 @@ typedef struct hv_fast_options {
                              (about a second).  The context stays usable after
                              a timeout                                         */
     int sor_coarse;       /* 1 (the default): each cycle of the fused float
-                             solve starts its correction from the correction
-                             equation solved exactly on a coarse grid (every
-                             F-th node, F the smallest power of two leaving at
-                             most 15 interior coarse nodes per axis; grids of
-                             fewer than 48^3 nodes or whose axes F does not
-                             divide, double solves, the max-update rule and
-                             batched waves of generic sweeps go without), and
-                             runs sor_coarse_sweeps red+black iterations after
-                             it; 0: plain SOR cycles.  The stopping rule is
-                             unchanged, so only the iterations per solve
-                             change                                            */
-    int sor_coarse_sweeps;/* red+black iterations after each coarse correction
-                             (default 12)                                      */
+                             solve finds its correction exactly: on the run's
+                             own grid (sine transforms along y and z, an
+                             elimination along x) where the y-z plane fits in
+                             one block's shared memory -- up to about 170 nodes
+                             on y and z -- and each cycle then counts as one
+                             iteration; on larger planes on a coarse grid
+                             (every F-th node, F the smallest power of two
+                             leaving at most 15 interior coarse nodes per axis)
+                             followed by sor_coarse_sweeps red+black
+                             iterations.  Double solves, the max-update rule
+                             and the phase-counter exchange run plain SOR
+                             cycles, as everything does with 0.  The stopping
+                             rule is unchanged, so only the iterations per
+                             solve change                                      */
+    int sor_coarse_sweeps;/* red+black iterations after each coarse-grid
+                             correction (default 12)                           */
     int deposit_aggregate;/* 1 (the default): the float atomic deposit of the
                              fused particle step sums the CIC weights of
                              neighbouring lanes with the same base node (the
