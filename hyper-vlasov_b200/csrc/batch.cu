@@ -15,7 +15,9 @@
 // How many blocks each instance's solve uses is a plan choice: fewer blocks
 // pack more instances into a wave, more blocks make each solve faster.
 // hv_batch_plan takes a cap; hv_batch_autotune times candidate caps on trial
-// steps and keeps the fastest, then the particle step's block size.
+// steps and keeps the fastest, then the particle step's block size.  The cap
+// shapes the sweeps only: direct solves (k_poisson.cu), the float default,
+// share the SMs by their work.
 #include <algorithm>
 #include <cstring>
 #include <numeric>
@@ -34,6 +36,7 @@ struct hv_batch {
     std::vector<cudaEvent_t> ev_a, ev_c;  // per instance: end of its phase A / C
     cudaEvent_t ev_fork_a = nullptr, ev_fork_c = nullptr;
     std::vector<SorWave> waves;
+    std::vector<int> blocks;              // blocks of each instance's solve
     int cap = -1;                         // SOR block cap of the current plan (0: own plans)
     cudaGraphExec_t graph = nullptr;
     int graph_len = 0;
@@ -172,25 +175,32 @@ hv_status hv_batch_plan(hv_batch *b, int sor_max_blocks) {
             return HV_ERR_UNSUPPORTED;
         }
     }
-    // first fit by decreasing block count into waves of at most one block per SM
+    // instances whose solves take the direct form share launches of all SMs;
+    // the others' sweeps go, first fit by decreasing block count, into waves of
+    // at most one block per SM
     std::vector<int> order(n);
     std::iota(order.begin(), order.end(), 0);
     std::stable_sort(order.begin(), order.end(),
                      [&](int x, int y) { return b->ctx[x]->fused.sor.nblocks > b->ctx[y]->fused.sor.nblocks; });
     std::vector<std::vector<int>> groups;
     std::vector<int> used;
+    std::vector<bool> direct;
     for (int i : order) {
-        const int nb = b->ctx[i]->fused.sor.nblocks;
+        const bool d = poisson_direct_runs(b->ctx[i]);
+        const int nb = d ? 1 : b->ctx[i]->fused.sor.nblocks;
         size_t g = 0;
-        while (g < groups.size() && used[g] + nb > b->sm_count) g++;
+        while (g < groups.size() && (direct[g] != d || used[g] + nb > b->sm_count)) g++;
         if (g == groups.size()) {
             groups.emplace_back();
             used.push_back(0);
+            direct.push_back(d);
         }
         groups[g].push_back(i);
         used[g] += nb;
     }
-    for (auto &grp : groups) {
+    b->blocks.assign(n, 0);
+    for (size_t q = 0; q < groups.size(); q++) {
+        const std::vector<int> &grp = groups[q];
         std::vector<hv_ctx *> cs;
         std::vector<const float *> rho;
         std::vector<int *> ctl, its;
@@ -205,11 +215,15 @@ hv_status hv_batch_plan(hv_batch *b, int sor_max_blocks) {
             its.push_back(it);
         }
         b->waves.emplace_back();
-        hv_status st = sor_wave_build(b->waves.back(), cs, rho, ctl, its, ring);
+        std::vector<int> blocks;
+        hv_status st = direct[q] ? poisson_wave_build(b->waves.back(), cs, rho, ctl, its, ring, blocks)
+                                 : sor_wave_build(b->waves.back(), cs, rho, ctl, its, ring);
         if (st != HV_OK) {
             set_last_error("batch: a wave of solves cannot be launched together");
             return st;
         }
+        for (size_t k = 0; k < grp.size(); k++)
+            b->blocks[grp[k]] = direct[q] ? blocks[k] : b->ctx[grp[k]]->fused.sor.nblocks;
     }
     b->cap = sor_max_blocks;
     return HV_OK;
@@ -323,7 +337,7 @@ hv_status hv_batch_tiles(const hv_batch *b, int *sor_planes, int *sor_rows, int 
         const hv_ctx *c = b->ctx[i];
         if (sor_planes) sor_planes[i] = c->fused.sor.P;
         if (sor_rows) sor_rows[i] = c->fused.sor.R;
-        if (sor_blocks) sor_blocks[i] = c->fused.sor.nblocks;
+        if (sor_blocks) sor_blocks[i] = b->blocks[i];
         if (particle_block) particle_block[i] = c->fused.pblock;
     }
     return HV_OK;

@@ -116,6 +116,7 @@ struct PoissonDirect {
     bool ok = false;           // the plane and its matrices fit on chip
     int off = 0, wz = 0, ps = 0, py = 0;  // stored plane: second half's column, columns, pitch; y matrices' pitch
     int rt = 0, nt = 0;        // kernel form: rows of a thread's tile, tiles per warp
+    int nt8 = 0;               // tiles per warp with eight rows (launches shared with larger planes)
     int shared_tab = 0, keep_tab = 0, front = 0, cw_max = 0, nblocks = 0;
     size_t smem = 0;
     float *tables = nullptr;   // sine matrices of z and y, both directions, and the eigenvalues (owns the
@@ -282,11 +283,17 @@ struct SorWave {
     void *args = nullptr;            // device: the instances' kernel arguments
     int *binst = nullptr, *bfirst = nullptr;  // device: block -> instance, instance -> first block
     std::vector<hv_ctx *> ctx;
+    bool direct = false;             // the direct solve's launch (k_poisson.cu), not the sweeps'
 };
 hv_status sor_wave_build(SorWave &w, const std::vector<hv_ctx *> &cs, const std::vector<const float *> &rho,
                          const std::vector<int *> &ctl, const std::vector<int *> &its_ring, int ring);
 hv_status sor_wave_launch(const SorWave &w, cudaStream_t st);
 void sor_wave_release(SorWave &w);
+// the same for direct solves; blocks receives each instance's share
+hv_status poisson_wave_build(SorWave &w, const std::vector<hv_ctx *> &cs, const std::vector<const float *> &rho,
+                             const std::vector<int *> &ctl, const std::vector<int *> &its_ring, int ring,
+                             std::vector<int> &blocks);
+hv_status poisson_wave_launch(const SorWave &w, cudaStream_t st);
 // Lets a kernel launch with up to the device's opt-in shared memory per block.
 // The attribute belongs to the function, which every context shares, so it is
 // raised to the maximum once rather than set to one plan's need.

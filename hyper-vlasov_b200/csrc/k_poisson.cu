@@ -757,13 +757,14 @@ hv_status poisson_plan(hv_ctx *c) {
     d.py = up(hy, 8);
     d.ps = d.wz;
     while (d.ps % 32 != 4 && d.ps % 32 != 12 && d.ps % 32 != 20 && d.ps % 32 != 28) d.ps += 4;
+    d.nt8 = (warp_tiles(g, d.off, d.wz, 8) + kWarps - 1) / kWarps;
+    if (d.nt8 > 3) return HV_OK;
     d.rt = warp_tiles(g, d.off, d.wz, 4) <= kWarps ? 4 : 8;
-    d.nt = (warp_tiles(g, d.off, d.wz, d.rt) + kWarps - 1) / kWarps;
-    if (d.nt > 3) return HV_OK;
+    d.nt = d.rt == 4 ? 1 : d.nt8;
     int optin = 0;
     HV_CUDA(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, c->device));
     const size_t limit = optin - 4096;  // the kernels' static shared memory
-    const size_t plane = (size_t)up(my, d.rt) * d.ps, zl = (size_t)2 * d.off * d.off, yl = (size_t)2 * d.py * d.py;
+    const size_t plane = (size_t)up(my, 8) * d.ps, zl = (size_t)2 * d.off * d.off, yl = (size_t)2 * d.py * d.py;
     d.shared_tab = my == mz ? 1 : 0;
     const size_t one = zl + (d.shared_tab ? 0 : yl);
     // phase B's columns and their coefficients lie where the plane lies; the
@@ -773,9 +774,15 @@ hv_status poisson_plan(hv_ctx *c) {
     int want = std::min(up((ncol + c->sm_count - 1) / c->sm_count, 16), 256);
     while (want > 16 && col * want * sizeof(float) > limit) want -= 16;
     if (col * want * sizeof(float) > limit) return HV_OK;
+    auto total = [&](int w) { return (std::max(plane, col * w) + 2 * one) * sizeof(float); };
+    d.keep_tab = total(want) <= limit ? 1 : 0;
+    // room for wider groups where it costs nothing: a solve that shares its
+    // launch has fewer blocks (16 warps eliminate 256 columns at once)
+    while (want < std::min(256, up(ncol, 16)) &&
+           (d.keep_tab ? total(want + 16) : col * (want + 16) * sizeof(float)) <= limit)
+        want += 16;
     d.cw_max = want;
-    const size_t both = std::max(plane, col * want) + 2 * one;
-    d.keep_tab = both * sizeof(float) <= limit ? 1 : 0;
+    const size_t both = total(want) / sizeof(float);
     const size_t words = d.keep_tab ? both : std::max(plane + one, col * want);
     d.front = (int)(d.keep_tab ? both - 2 * one : plane);
     d.smem = words * sizeof(float);
@@ -839,6 +846,81 @@ hv_status poisson_launch(hv_ctx *c, const float *rho, int *ctl, int *its_ring, i
     void *args[] = {&a};
     HV_CUDA(cudaLaunchCooperativeKernel(direct_kernel<false>(d.rt, d.nt), dim3(d.nblocks), dim3(kThreads), args,
                                         d.smem, c->stream));
+    return HV_OK;
+}
+
+// Several direct solves in one cooperative launch: the blocks of the SMs are
+// shared out by the instances' work, so that they end together.
+hv_status poisson_wave_build(SorWave &w, const std::vector<hv_ctx *> &cs, const std::vector<const float *> &rho,
+                             const std::vector<int *> &ctl, const std::vector<int *> &its_ring, int ring,
+                             std::vector<int> &blocks) {
+    sor_wave_release(w);
+    const int n = (int)cs.size(), sms = cs[0]->sm_count;
+    if (n > sms) return HV_ERR_UNSUPPORTED;
+    // time of an instance ~ planes per block x work of a plane (the walks, and
+    // the transforms, as much again for 64 rows and columns)
+    auto most = [&](int i) { return cs[i]->fused.direct.nblocks; };
+    auto cost = [&](int i) {
+        const Geom &g = cs[i]->geom;
+        const double plane = (double)g.ny * g.nz * (1.0 + (g.ny + g.nz) / 128.0);
+        return plane * ((g.nx - 2 + blocks[i] - 1) / blocks[i]);
+    };
+    blocks.assign(n, 1);
+    for (int left = sms - n; left > 0;) {
+        int worst = -1;
+        for (int i = 0; i < n; i++)
+            if (blocks[i] < most(i) && (worst < 0 || cost(i) > cost(worst))) worst = i;
+        if (worst < 0) break;
+        // enough blocks for one plane per block fewer, or what is left
+        const int mx = cs[worst]->geom.nx - 2, per = (mx + blocks[worst] - 1) / blocks[worst];
+        const int next = per > 1 ? (mx + per - 2) / (per - 1) : most(worst);
+        const int add = std::min(left, std::max(1, std::min(next, most(worst)) - blocks[worst]));
+        blocks[worst] += add;
+        left -= add;
+    }
+    std::vector<DirectArgs<float>> args;
+    std::vector<int> binst, bfirst(n);
+    int rt = 4, nt = 1;
+    size_t smem = 0;
+    for (int i = 0; i < n; i++) {
+        const PoissonDirect &d = cs[i]->fused.direct;
+        args.push_back(direct_args(cs[i], rho[i], ctl[i], its_ring[i], ring, blocks[i]));
+        bfirst[i] = (int)binst.size();
+        binst.insert(binst.end(), blocks[i], i);
+        if (d.rt == 8) rt = 8;
+        smem = std::max(smem, d.smem);
+    }
+    if (rt == 8)
+        for (hv_ctx *c : cs) nt = std::max(nt, c->fused.direct.nt8);
+    w.kern = direct_kernel<true>(rt, nt);
+    HV_TRY(allow_max_dynamic_smem(w.kern, cs[0]->device));
+    int per_sm = 0;
+    HV_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, w.kern, kThreads, smem));
+    if ((long long)per_sm * sms < (long long)binst.size()) return HV_ERR_UNSUPPORTED;
+    HV_CUDA(cudaMalloc(&w.args, sizeof(DirectArgs<float>) * n));
+    HV_CUDA(cudaMalloc((void **)&w.binst, sizeof(int) * binst.size()));
+    HV_CUDA(cudaMalloc((void **)&w.bfirst, sizeof(int) * n));
+    HV_CUDA(cudaMemcpy(w.args, args.data(), sizeof(DirectArgs<float>) * n, cudaMemcpyHostToDevice));
+    HV_CUDA(cudaMemcpy(w.binst, binst.data(), sizeof(int) * binst.size(), cudaMemcpyHostToDevice));
+    HV_CUDA(cudaMemcpy(w.bfirst, bfirst.data(), sizeof(int) * n, cudaMemcpyHostToDevice));
+    // a cudaMemcpy from pageable memory may return before its DMA ends; the
+    // wave's kernels run later on other streams
+    HV_CUDA(cudaDeviceSynchronize());
+    w.ctx = cs;
+    w.nblocks = (int)binst.size();
+    w.smem = smem;
+    w.direct = true;
+    return HV_OK;
+}
+
+hv_status poisson_wave_launch(const SorWave &w, cudaStream_t st) {
+    DirectArgs<float> p;
+    std::memset(&p, 0, sizeof(p));
+    p.batch = reinterpret_cast<const DirectArgs<float> *>(w.args);
+    p.binst = w.binst;
+    p.bfirst = w.bfirst;
+    void *args[] = {&p};
+    HV_CUDA(cudaLaunchCooperativeKernel(w.kern, dim3(w.nblocks), dim3(kThreads), args, w.smem, st));
     return HV_OK;
 }
 

@@ -1862,6 +1862,7 @@ hv_status sor_wave_build(SorWave &w, const std::vector<hv_ctx *> &cs, const std:
 // The waves run tagged forms only: each instance's barrier counter is back at
 // zero after its solve, and the batch's start resets it (run_begin).
 hv_status sor_wave_launch(const SorWave &w, cudaStream_t st) {
+    if (w.direct) return poisson_wave_launch(w, st);
     SorArgs<float, float> p;
     std::memset(&p, 0, sizeof(p));
     p.batch = reinterpret_cast<const SorArgs<float, float> *>(w.args);
