@@ -89,6 +89,19 @@ TapTable build_taps(const hv_world &w, double sigma_r) {
     }
     t.count = (int)t.packed.size();
     for (int a = 0; a < 3; a++) t.lim[a] = lim64[a];
+    // the same taps as runs of consecutive c, and the first run of each a
+    const auto unpack = [&](int i, int sh) { return ((t.packed[i] >> sh) & 1023) - 512; };
+    std::vector<int> runs;
+    t.slabs.assign(2 * t.lim[0] + 2, 0);
+    for (int i = 0; i < t.count;) {
+        int n = 1;
+        while (i + n < t.count && t.packed[i + n] == t.packed[i] + n) n++;
+        runs.insert(runs.end(), {unpack(i, 10), unpack(i, 0), n, i});
+        for (int a = unpack(i, 20) + t.lim[0] + 1; a < (int)t.slabs.size(); a++) t.slabs[a] = (int)runs.size() / 4;
+        i += n;
+    }
+    t.runs = (int)runs.size() / 4;
+    t.slabs.insert(t.slabs.begin(), runs.begin(), runs.end());
     return t;
 }
 
@@ -100,6 +113,16 @@ template <>
 State<float> &state<float>(hv_ctx *c) { return c->d32; }
 
 namespace {
+
+// The tap runs and slabs on the device.
+hv_status upload_runs(hv_ctx *c) {
+    if (c->taps_runs) cudaFree(c->taps_runs);
+    c->taps_runs = nullptr;
+    const std::vector<int> &v = c->taps.slabs;
+    HV_CUDA(cudaMalloc((void **)&c->taps_runs, sizeof(int) * (v.size() + 4)));
+    HV_CUDA(cudaMemcpyAsync(c->taps_runs, v.data(), sizeof(int) * v.size(), cudaMemcpyHostToDevice, c->stream));
+    return HV_OK;
+}
 
 template <typename T>
 hv_status alloc_state(hv_ctx *c) {
@@ -508,6 +531,7 @@ hv_status hv_ctx_create(const hv_world *world, int protons, int neutrons, hv_pre
                         c->stream) != cudaSuccess)
         return fail(cuda_status(cudaGetLastError(), "taps upload"));
     st = prec == HV_F64 ? alloc_state<double>(c) : alloc_state<float>(c);
+    if (st == HV_OK) st = upload_runs(c);
     if (st != HV_OK) return fail(st);
     const int n = c->total > 0 ? c->total : 1;
     Scratch &s = c->scratch;
@@ -515,7 +539,6 @@ hv_status hv_ctx_create(const hv_world *world, int protons, int neutrons, hv_pre
     s.cub_tmp_bytes = sorted_deposit_tmp_bytes(n);
     if (cudaMalloc((void **)&c->perm, sizeof(int) * n) != cudaSuccess ||
         cudaMalloc((void **)&s.partials, sizeof(double) * s.partials_len) != cudaSuccess ||
-        cudaMalloc((void **)&s.maxbits, sizeof(unsigned long long) * 4) != cudaSuccess ||
         cudaMalloc((void **)&s.result, sizeof(double) * 64) != cudaSuccess ||
         cudaMallocHost((void **)&s.h_result, sizeof(double) * 64) != cudaSuccess ||
         cudaMalloc((void **)&s.keys, sizeof(unsigned int) * n) != cudaSuccess ||
@@ -543,7 +566,7 @@ hv_status hv_ctx_destroy(hv_ctx *c) {
     free_state(c->d64);
     free_state(c->d32);
     Scratch &s = c->scratch;
-    void *ptrs[] = {c->perm, c->taps_dev, s.partials, s.maxbits, s.result, s.keys, s.keys_alt, s.vals, s.vals_alt,
+    void *ptrs[] = {c->perm, c->taps_dev, s.partials, s.sor, c->taps_runs, s.result, s.keys, s.keys_alt, s.vals, s.vals_alt,
                     s.cell_start, s.cub_tmp, s.sort_tmp};
     for (void *p : ptrs)
         if (p) cudaFree(p);
@@ -572,6 +595,8 @@ hv_status hv_ctx_set_params(hv_ctx *c, const hv_run_params *p) {
         }
         c->taps = t;
         c->taps_count = t.count;
+        HV_CUDA(cudaStreamSynchronize(c->stream));
+        HV_TRY(upload_runs(c));
         if (t.count > 0) {
             HV_CUDA(cudaMemcpyAsync(c->taps_dev, t.packed.data(), sizeof(int) * t.count, cudaMemcpyHostToDevice, c->stream));
             if (c->d64.taps_w)

@@ -50,6 +50,11 @@ struct TapTable {
     std::vector<int> packed;
     std::vector<double> w64;
     std::vector<float> w32;
+    // runs of consecutive c: (b, c of the first tap, taps, index of the first)
+    // each, `runs` of them, then the first run of every a from -lim[0] on and
+    // their number
+    int runs = 0;
+    std::vector<int> slabs;
 };
 TapTable build_taps(const hv_world &w, double sigma_r);
 
@@ -71,7 +76,7 @@ struct State {
 struct Scratch {
     double *partials = nullptr;     // deterministic reduction partials
     size_t partials_len = 0;
-    unsigned long long *maxbits = nullptr;  // SOR max|dphi| as ordered bits
+    void *sor = nullptr;            // plain SOR: saved values, partial results, barrier, outcome
     double *result = nullptr;       // small device results (reductions)
     double *h_result = nullptr;     // pinned host mirror of result
     // sorted-deposit buffers
@@ -213,6 +218,7 @@ struct hv_ctx {
     hv::TapTable taps;
     int taps_count = 0;
     int *taps_dev = nullptr;
+    int *taps_runs = nullptr;  // taps.slabs
     hv::Scratch scratch;
     hv::Fused fused;
     hv::Profile prof;

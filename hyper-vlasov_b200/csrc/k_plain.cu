@@ -3,8 +3,11 @@
 // that a*b+c stays two rounded operations, as in the reference built with
 // -ffp-contract=off; with identical inputs the HV_F64 results of deposit
 // (sorted mode), FDM, merge, SOR, gather and push are bit-identical to it.
+#include <algorithm>
+
 #include <cub/device/device_radix_sort.cuh>
 
+#include "grid_sync.cuh"
 #include "hv_internal.h"
 
 namespace hv {
@@ -183,6 +186,73 @@ __global__ void k_smooth_direct(Geom g, int ntaps, int lx, int ly, int lz, const
     dst[i] = rho_f * term;  // physics.hpp:229-232
 }
 
+// The same sums, in the same order, four consecutive z per thread: the source
+// rows that a block's outputs reach at one x offset are staged in shared
+// memory with zeros outside the grid (adding w * 0 changes no sum), and along
+// a run of taps a thread's four source values shift through registers, one new
+// load a tap.  Stored by z mod 4, so that consecutive threads read consecutive
+// words.  A tap then costs a thread two shared loads and eight operations
+// instead of four times two global loads, the index arithmetic and two
+// operations: 64^3 in double, half-width 4, 533 -> 95 us.
+constexpr int kRowThreads = 128;
+struct RowTile {
+    int qz, ty, pitch, words, wmax;  // quads of a z row, y rows of a block, words of a quarter row, of a slab, weights
+};
+
+template <typename T>
+__global__ void __launch_bounds__(kRowThreads) k_smooth_rows(Geom g, RowTile rt, int lx, int ly, int lz, int runs,
+                                                             const int *__restrict__ tab, const T *__restrict__ w,
+                                                             T term, const T *__restrict__ src, T *dst) {
+    extern __shared__ __align__(16) unsigned char row_smem[];
+    T *rows = reinterpret_cast<T *>(row_smem), *ws = rows + rt.words;
+    const int nx = g.nx, ny = g.ny, nz = g.nz, tid = threadIdx.x;
+    const int ix = blockIdx.y, y0 = blockIdx.x * rt.ty, nrows = rt.ty + 2 * ly, width = nz + 2 * lz;
+    const T *s = src + (blockIdx.z ? g.G : 0);
+    const int4 *run = reinterpret_cast<const int4 *>(tab);
+    const int *slab = tab + 4 * runs;
+    const int r = tid / rt.qz, q = tid - r * rt.qz;
+    const bool mine = r < rt.ty && y0 + r < ny;
+    T acc0 = T(0), acc1 = T(0), acc2 = T(0), acc3 = T(0);
+    for (int a = -lx; a <= lx; a++) {
+        const int r0 = slab[a + lx], r1 = slab[a + lx + 1], jx = ix + a;
+        if (r0 == r1 || jx < 0 || jx >= nx) continue;
+        const int t0 = run[r0].w, t1 = run[r1 - 1].w + run[r1 - 1].z;
+        __syncthreads();
+        for (int e = tid; e < t1 - t0; e += kRowThreads) ws[e] = w[t0 + e];
+        for (int e = tid; e < nrows * width; e += kRowThreads) {
+            const int rr = e / width, zz = e - rr * width, jy = y0 - ly + rr, jz = zz - lz;
+            const bool in = jy >= 0 && jy < ny && jz >= 0 && jz < nz;
+            rows[(rr * 4 + (zz & 3)) * rt.pitch + (zz >> 2)] =
+                in ? s[((long long)jx * ny + jy) * nz + jz] : T(0);
+        }
+        __syncthreads();
+        if (!mine) continue;
+        for (int k = r0; k < r1; k++) {
+            const int4 v = run[k];
+            const T *row = rows + (r + ly + v.x) * 4 * rt.pitch + q;
+            const T *wk = ws + v.w - t0;
+            int z = v.y + lz;  // padded position of the first tap for z = 4 q
+            auto at = [&](int p) { return row[(p & 3) * rt.pitch + (p >> 2)]; };
+            T v0 = at(z), v1 = at(z + 1), v2 = at(z + 2);
+            for (int t = 0; t < v.z; t++) {
+                const T v3 = at(z + 3 + t), wt = wk[t];
+                acc0 += v0 * wt;
+                acc1 += v1 * wt;
+                acc2 += v2 * wt;
+                acc3 += v3 * wt;
+                v0 = v1;
+                v1 = v2;
+                v2 = v3;
+            }
+        }
+    }
+    if (!mine) return;
+    T *d = dst + (blockIdx.z ? g.G : 0) + ((long long)ix * ny + y0 + r) * nz + 4 * q;
+    const T out[4] = {acc0, acc1, acc2, acc3};
+    for (int u = 0; u < 4; u++)
+        if (4 * q + u < nz) d[u] = out[u] * term;  // physics.hpp:229-232
+}
+
 // ---- Skyrme (include/physics.hpp:272-281, physics_formulas.hpp:70-77) ------
 template <typename T>
 __device__ __forceinline__ T skyrme_u(T A, T B, T C, T gamma, T rho_p, T rho_n, T tau) {
@@ -218,106 +288,196 @@ __global__ void k_boundary(Geom g, int Z, T *phi) {
     phi[id] = (T)(A(1.44) * Z / r);
 }
 
-// ---- red-black SOR half sweep (include/physics.hpp:99-157) ----------------
-__device__ __forceinline__ void atomic_max_bits(unsigned long long *m, double v) {
-    atomicMax(m, (unsigned long long)__double_as_longlong(v));
+// ---- red-black SOR (include/physics.hpp:99-157) ---------------------------
+// One cooperative launch per solve; the stopping rule is tested after every
+// iteration, as the reference's loop does, but on the device and one half
+// sweep late.  A black update has its node's final neighbours at hand, so it
+// forms the node's residual too; a red node's residual of iteration t needs
+// the black values of t, which the red half sweep of t + 1 reads anyway.  The
+// test of iteration t therefore runs while the black half sweep of t + 1
+// does; when t met the rule, both half sweeps of t + 1 are taken back from the
+// values they saved.  An iteration is two half sweeps and two grid barriers;
+// the arithmetic of every kept value is the reference's.
+//
+// Bound by the latency of a half sweep (operands from L2, three divisions) and
+// of the barrier.  A step of the plain double path, mostly this solve: 208Pb
+// 64^3 15.4 -> 4.0 ms, 40Ca 32^3 2.6 -> 0.56 ms (five launches, a serial sum
+// and a synchronisation an iteration before).
+constexpr int kSorBlock = 512;
+
+template <typename T>
+struct PlainSor {
+    int nx, ny, nz, half, count;  // count: colour points, (nx - 2)(ny - 2) half
+    T omega, inv_dx2, hx2, hy2, hz2, src_c, tol_t;
+    double ix2, iy2, iz2, diag, bsrc, tol;
+    int criterion, max_iter, nblocks;
+    long long max_spin;
+    T *phi, *saved;
+    const T *rho;
+    double *partials;             // [nblocks][2]
+    unsigned *bar;
+    int *status;                  // [0] error, [1] iterations, [2] 1 converged, 2 not finite
+    double *metric;
+};
+
+template <typename T>
+__device__ __forceinline__ T nan_max(T a, T b) {
+    return (b > a || b != b) ? b : a;
 }
-__device__ __forceinline__ void atomic_max_bits(unsigned long long *m, float v) {
-    atomicMax(m, (unsigned long long)__float_as_uint(v));
+
+// Node of colour point t, or -1 (the last point of a short line).
+template <typename T>
+__device__ __forceinline__ int colour_node(const PlainSor<T> &a, int color, int t) {
+    const int l = t / a.half, kk = t - l * a.half, li = l / (a.ny - 2);
+    const int j = 1 + l - li * (a.ny - 2), i = 1 + li;
+    const int k = 1 + ((i + j + 1 + color) & 1) + 2 * kk;
+    return k < a.nz - 1 ? (i * a.ny + j) * a.nz + k : -1;
 }
 
 template <typename T>
-__global__ void k_sor_half(Geom g, int color, T omega, T inv_dx2, T hx2, T hy2, T hz2, T src_c,
-                           T *phi, const T *__restrict__ rho, unsigned long long *maxbits) {
-    const int nx = g.nx, ny = g.ny, nz = g.nz;
-    const int half = (nz - 1) / 2;  // upper bound of colour points per (i, j) line
-    long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    long long lines = (long long)(nx - 2) * (ny - 2);
-    T diff = T(0.0);
-    if (t < lines * half) {
-        int kk = (int)(t % half);
-        long long l = t / half;
-        int j = 1 + (int)(l % (ny - 2)), i = 1 + (int)(l / (ny - 2));
-        int k = 1 + ((i + j + 1 + color) & 1) + 2 * kk;
-        if (k < nz - 1) {
-            const long long sx = (long long)ny * nz, sy = nz;
-            long long id = i * sx + j * sy + k;
-            T r = rho[id];
-            T phi_x = (phi[id + sx] + phi[id - sx]) / hx2;
-            T phi_y = (phi[id + sy] + phi[id - sy]) / hy2;
-            T phi_z = (phi[id + 1] + phi[id - 1]) / hz2;
-            T phi_star = (phi_x + phi_y + phi_z + src_c * r) * inv_dx2;
-            T phi_old = phi[id];
-            T nv = (T(1.0) - omega) * phi_old + omega * phi_star;
-            phi[id] = nv;
-            diff = fabs(nv - phi_old);
-        }
-    }
-    // block max, then one atomic per block (max is order independent)
-    __shared__ T red[kBlock / 32];
-    for (int o = 16; o > 0; o >>= 1) {
-        T other = __shfl_xor_sync(0xffffffffu, diff, o);
-        diff = (other > diff || other != other) ? other : diff;
-    }
-    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = diff;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        T m = red[0];
-        for (int w = 1; w < kBlock / 32; w++) m = (red[w] > m || red[w] != red[w]) ? red[w] : m;
-        atomic_max_bits(maxbits, m);
-    }
-}
-
-// ||b + lap_h phi||^2 and ||b||^2 over interior nodes, in double; one partial
-// pair per block (fixed grid, fixed order: deterministic).
-template <typename T>
-__global__ void k_residual_partials(Geom g, double ix2, double iy2, double iz2, double src_c,
-                                    const T *__restrict__ phi, const T *__restrict__ rho,
-                                    double *partials) {
-    const int nx = g.nx, ny = g.ny, nz = g.nz;
-    const long long sx = (long long)ny * nz, sy = nz;
-    const long long n_int = (long long)(nx - 2) * (ny - 2) * (nz - 2);
-    const double diag = 2.0 * ix2 + 2.0 * iy2 + 2.0 * iz2;
+__global__ void __launch_bounds__(kSorBlock, 2) k_sor_plain(PlainSor<T> a) {
+    __shared__ int s_stop;
+    __shared__ double s_metric;
+    __shared__ T s_max[kSorBlock / 32];
+    const int tid = threadIdx.x, b = blockIdx.x, stride = a.nblocks * kSorBlock, first = b * kSorBlock + tid;
+    const int sx = a.ny * a.nz, sy = a.nz;
+    const bool rel = a.criterion == HV_SOR_REL_RESIDUAL;
+    // the first point of each colour, decoded once (most grids: the only one)
+    const int node0[2] = {first < a.count ? colour_node(a, 0, first) : -1,
+                          first < a.count ? colour_node(a, 1, first) : -1};
     double rr = 0.0, bb = 0.0;
-    for (long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x; t < n_int;
-         t += (long long)gridDim.x * blockDim.x) {
-        int k = 1 + (int)(t % (nz - 2));
-        long long l = t / (nz - 2);
-        int j = 1 + (int)(l % (ny - 2)), i = 1 + (int)(l / (ny - 2));
-        long long id = i * sx + j * sy + k;
-        double b = src_c * (double)rho[id];
-        double lap = ((double)phi[id + sx] + (double)phi[id - sx]) * ix2 +
-                     ((double)phi[id + sy] + (double)phi[id - sy]) * iy2 +
-                     ((double)phi[id + 1] + (double)phi[id - 1]) * iz2 - diag * (double)phi[id];
-        double r = b + lap;
-        rr += r * r;
-        bb += b * b;
-    }
-    __shared__ double s_rr[kBlock], s_bb[kBlock];
-    s_rr[threadIdx.x] = rr;
-    s_bb[threadIdx.x] = bb;
-    __syncthreads();
-    for (int o = kBlock / 2; o > 0; o >>= 1) {
-        if (threadIdx.x < o) {
-            s_rr[threadIdx.x] += s_rr[threadIdx.x + o];
-            s_bb[threadIdx.x] += s_bb[threadIdx.x + o];
+    T diff = T(0);
+
+    auto sweep = [&](int color, bool sources) {
+        for (int t = first; t < a.count; t += stride) {
+            const int id = t == first ? node0[color] : colour_node(a, color, t);
+            if (id < 0) continue;
+            const T r = __ldg(a.rho + id);
+            const T xp = __ldcg(a.phi + id + sx), xm = __ldcg(a.phi + id - sx);
+            const T yp = __ldcg(a.phi + id + sy), ym = __ldcg(a.phi + id - sy);
+            const T zp = __ldcg(a.phi + id + 1), zm = __ldcg(a.phi + id - 1);
+            const T old = __ldcg(a.phi + id);
+            const T phi_x = (xp + xm) / a.hx2, phi_y = (yp + ym) / a.hy2, phi_z = (zp + zm) / a.hz2;
+            const T star = (phi_x + phi_y + phi_z + a.src_c * r) * a.inv_dx2;
+            const T nv = (T(1.0) - a.omega) * old + a.omega * star;
+            a.saved[id] = old;
+            __stcg(a.phi + id, nv);
+            if (rel) {
+                // b + lap_h phi in double: of the iterate before at a red node,
+                // of this one at a black node
+                const double bv = a.bsrc * (double)r;
+                const double lap = ((double)xp + (double)xm) * a.ix2 + ((double)yp + (double)ym) * a.iy2 +
+                                   ((double)zp + (double)zm) * a.iz2 - a.diag * (double)(color ? nv : old);
+                const double res = bv + lap;
+                rr += res * res;
+                if (sources) bb += bv * bv;
+            } else {
+                diff = nan_max(diff, (T)fabs(nv - old));
+            }
         }
-        __syncthreads();
+    };
+    auto take_back = [&](int color) {
+        for (int t = first; t < a.count; t += stride) {
+            const int id = t == first ? node0[color] : colour_node(a, color, t);
+            if (id >= 0) a.phi[id] = a.saved[id];
+        }
+    };
+    // warp 0: the test of iteration `t` from the blocks' partial results
+    auto test = [&](int t) {
+        double u = 0.0, v = 0.0;
+        for (int q = tid; q < a.nblocks; q += 32) {
+            const double p = __ldcg(a.partials + 2 * q);
+            if (rel) {
+                u += p;
+                v += __ldcg(a.partials + 2 * q + 1);
+            } else {
+                u = nan_max(u, p);
+            }
+        }
+        for (int o = 16; o > 0; o >>= 1) {
+            const double p = __shfl_xor_sync(0xffffffffu, u, o), q = __shfl_xor_sync(0xffffffffu, v, o);
+            u = rel ? u + p : nan_max(u, p);
+            v += q;
+        }
+        if (tid == 0) {
+            const double m = !rel ? u : v > 0.0 ? sqrt(u / v) : sqrt(u);
+            const bool ok = rel ? m <= a.tol : (T)m < a.tol_t;
+            s_metric = m;
+            s_stop = m != m ? 2 : ok ? 1 : t >= a.max_iter ? 3 : 0;
+        }
+    };
+
+    int it = 0;
+    while (true) {
+        it++;
+        if (!rel && it > 1 && tid < 32) test(it - 1);
+        // rr still holds the black nodes' residual of iteration it - 1
+        if (!rel) diff = T(0);
+        sweep(0, it == 1);
+        if (rel) {
+            double u = rr, v = bb;
+            block_sum2(u, v);
+            if (tid == 0) {
+                a.partials[2 * b] = u;
+                a.partials[2 * b + 1] = v;
+            }
+            rr = 0.0;
+        } else if (it > 1) {
+            __syncthreads();
+            if (s_stop) {
+                take_back(0);
+                break;
+            }
+        }
+        if (!grid_barrier(a.bar, a.nblocks, a.status, a.max_spin)) return;
+        if (rel && it > 1 && tid < 32) test(it - 1);
+        sweep(1, it == 1);
+        if (rel) {
+            __syncthreads();
+            if (it > 1 && s_stop) {
+                take_back(0);
+                take_back(1);
+                break;
+            }
+        } else {
+            T m = diff;
+            for (int o = 16; o > 0; o >>= 1) m = nan_max(m, __shfl_xor_sync(0xffffffffu, m, o));
+            if ((tid & 31) == 0) s_max[tid >> 5] = m;
+            __syncthreads();
+            if (tid == 0) {
+                for (int w = 1; w < kSorBlock / 32; w++) m = nan_max(m, s_max[w]);
+                a.partials[2 * b] = (double)m;
+            }
+        }
+        if (!grid_barrier(a.bar, a.nblocks, a.status, a.max_spin)) return;
     }
-    if (threadIdx.x == 0) {
-        partials[2 * blockIdx.x] = s_rr[0];
-        partials[2 * blockIdx.x + 1] = s_bb[0];
+    if (b == 0 && tid == 0) {
+        a.status[1] = it - 1;
+        a.status[2] = s_stop == 3 ? 0 : s_stop;
+        a.metric[0] = s_metric;
     }
 }
 
 // Sums `width`-wide rows of partials (nblocks rows) in fixed order.
+// The rows come to shared memory first, all loads at once: the sums' serial
+// chain then waits for additions, not for memory (18 us before, 3 after).
+constexpr int kSumRows = 1024;
 __global__ void k_sum_partials(const double *__restrict__ partials, int nblocks, int width,
                                double *out) {
-    int c = threadIdx.x;
-    if (c >= width) return;
+    __shared__ double sh[kSumRows * 6];
+    const int c = threadIdx.x;
     double s = 0.0;
-    for (int b = 0; b < nblocks; b++) s += partials[(long long)b * width + c];
-    out[c] = s;
+    for (int b0 = 0; b0 < nblocks; b0 += kSumRows) {
+        const int n = min(kSumRows, nblocks - b0);
+        for (int e = threadIdx.x; e < n * width; e += blockDim.x) sh[e] = partials[(long long)b0 * width + e];
+        __syncthreads();
+        if (c < width) {
+#pragma unroll 8
+            for (int b = 0; b < n; b++) s += sh[b * width + c];
+        }
+        __syncthreads();
+    }
+    if (c < width) out[c] = s;
 }
 
 // ---- merge, FDM, gather, push, excite ------------------------------------
@@ -497,6 +657,24 @@ hv_status launch_smooth(hv_ctx *c, const T *rho_raw, T *rho) {
     const T term = (T(1.0) / p.part_per_nucleon) *
                    (T(1.0) / std::pow(T(2.0) * T(kPi) * sig * sig, T(1.5)));
     const T *w = reinterpret_cast<const T *>(sizeof(T) == 8 ? (void *)c->d64.taps_w : (void *)c->d32.taps_w);
+    // staged rows where a block's slab fits in the default shared memory (z
+    // rows of at most 512 nodes and stencils of up to ~12 nodes at 128^3 in
+    // double), else tap by tap
+    const Geom &g = c->geom;
+    const int *lim = c->taps.lim;
+    RowTile rt;
+    rt.qz = (g.nz + 3) / 4;
+    rt.ty = std::max(1, std::min(kRowThreads / rt.qz, g.ny));
+    rt.pitch = (4 * rt.qz + 2 * lim[2] + 3) / 4 + 1;
+    rt.words = (rt.ty + 2 * lim[1]) * 4 * rt.pitch;
+    rt.wmax = (2 * lim[1] + 1) * (2 * lim[2] + 1);
+    const size_t smem = sizeof(T) * (size_t)(rt.words + rt.wmax);
+    if (rt.qz <= kRowThreads && smem <= 48 * 1024 && c->taps.runs > 0) {
+        k_smooth_rows<T><<<dim3((g.ny + rt.ty - 1) / rt.ty, g.nx, 2), kRowThreads, smem, c->stream>>>(
+            g, rt, lim[0], lim[1], lim[2], c->taps.runs, c->taps_runs, w, term, rho_raw, rho);
+        HV_CUDA(cudaGetLastError());
+        return HV_OK;
+    }
     k_smooth_direct<T><<<blocks_for(2 * c->geom.G), kBlock, 0, c->stream>>>(
         c->geom, c->taps_count, c->taps.lim[0], c->taps.lim[1], c->taps.lim[2], c->taps_dev, w, term, rho_raw, rho);
     HV_CUDA(cudaGetLastError());
@@ -525,76 +703,61 @@ hv_status launch_sor_plain(hv_ctx *c, T *phi, const T *rho, int *iters, double *
     const T dx = T(2.0) * T(g.dmx) / g.nx, dy = T(2.0) * T(g.dmy) / g.ny, dz = T(2.0) * T(g.dmz) / g.nz;
     const T hx2 = dx * dx, hy2 = dy * dy, hz2 = dz * dz;
     const T inv_dx2 = T(1.0) / (T(2.0) / hx2 + T(2.0) / hy2 + T(2.0) / hz2);
-    const T omega = T(sp.omega);
-    const T src_c = T(4.0) * T(kPi) * T(1.44);
-    const long long lines = (long long)(g.nx - 2) * (g.ny - 2);
-    const int half = (g.nz - 1) / 2;
-    const int nb = blocks_for(lines * half);
+    // the solver's work space, kept by the context: the saved values, the
+    // partial results, the barrier, the outcome
+    Scratch &sc = c->scratch;
+    const size_t nsaved = ((size_t)g.G * sizeof(T) + 255) / 256 * 256, npart = 2 * 2 * (size_t)c->sm_count;
+    if (!sc.sor) {
+        HV_CUDA(cudaMalloc(&sc.sor, nsaved + npart * sizeof(double) + 256));
+    }
+    char *base = static_cast<char *>(sc.sor);
+    PlainSor<T> a;
+    a.nx = g.nx;
+    a.ny = g.ny;
+    a.nz = g.nz;
+    a.half = (g.nz - 1) / 2;  // upper bound of colour points per (i, j) line
+    a.count = (int)((long long)(g.nx - 2) * (g.ny - 2) * a.half);
+    a.omega = T(sp.omega);
+    a.inv_dx2 = inv_dx2;
+    a.hx2 = hx2;
+    a.hy2 = hy2;
+    a.hz2 = hz2;
+    a.src_c = T(4.0) * T(kPi) * T(1.44);
+    a.tol_t = T(sp.tol);
+    a.tol = sp.tol;
     // residual in double from double spacings
     const double ddx = 2.0 * g.dmx / g.nx, ddy = 2.0 * g.dmy / g.ny, ddz = 2.0 * g.dmz / g.nz;
-    const int rb = 2 * c->sm_count;
-    double m = 0.0;
-    int it = 0;
-    bool converged = false;
-    for (it = 0; it < sp.max_iter;) {
-        if (sp.criterion == HV_SOR_MAX_UPDATE)
-            HV_CUDA(cudaMemsetAsync(c->scratch.maxbits, 0, sizeof(unsigned long long), c->stream));
-        for (int color = 0; color < 2; color++) {
-            k_sor_half<T><<<nb, kBlock, 0, c->stream>>>(g, color, omega, inv_dx2, hx2, hy2, hz2, src_c, phi, rho,
-                                                       c->scratch.maxbits);
-        }
-        HV_CUDA(cudaGetLastError());
-        it++;
-        if (sp.criterion == HV_SOR_MAX_UPDATE) {
-            unsigned long long bits = 0;
-            HV_CUDA(cudaMemcpyAsync(&bits, c->scratch.maxbits, sizeof(bits), cudaMemcpyDeviceToHost, c->stream));
-            HV_CUDA(cudaStreamSynchronize(c->stream));
-            T md;
-            if (sizeof(T) == 8) {
-                double d;
-                memcpy(&d, &bits, 8);
-                md = (T)d;
-            } else {
-                unsigned int u = (unsigned int)bits;
-                float f;
-                memcpy(&f, &u, 4);
-                md = (T)f;
-            }
-            m = (double)md;
-            if (md != md) {
-                if (iters) *iters = it;
-                if (metric) *metric = m;
-                return HV_ERR_NONFINITE;
-            }
-            if (md < T(sp.tol)) {  // physics.hpp:152
-                converged = true;
-                break;
-            }
-        } else {
-            k_residual_partials<T><<<rb, kBlock, 0, c->stream>>>(g, 1.0 / (ddx * ddx), 1.0 / (ddy * ddy),
-                                                                 1.0 / (ddz * ddz), 4.0 * kPi * 1.44, phi, rho,
-                                                                 c->scratch.partials);
-            k_sum_partials<<<1, 32, 0, c->stream>>>(c->scratch.partials, rb, 2, c->scratch.result);
-            HV_CUDA(cudaGetLastError());
-            HV_CUDA(cudaMemcpyAsync(c->scratch.h_result, c->scratch.result, 2 * sizeof(double),
-                                    cudaMemcpyDeviceToHost, c->stream));
-            HV_CUDA(cudaStreamSynchronize(c->stream));
-            double rr = c->scratch.h_result[0], bb = c->scratch.h_result[1];
-            m = bb > 0.0 ? std::sqrt(rr / bb) : std::sqrt(rr);
-            if (m != m) {
-                if (iters) *iters = it;
-                if (metric) *metric = m;
-                return HV_ERR_NONFINITE;
-            }
-            if (m <= sp.tol) {
-                converged = true;
-                break;
-            }
-        }
+    a.ix2 = 1.0 / (ddx * ddx);
+    a.iy2 = 1.0 / (ddy * ddy);
+    a.iz2 = 1.0 / (ddz * ddz);
+    a.diag = 2.0 * a.ix2 + 2.0 * a.iy2 + 2.0 * a.iz2;
+    a.bsrc = 4.0 * kPi * 1.44;
+    a.criterion = sp.criterion;
+    a.max_iter = sp.max_iter;
+    // a thread per colour point up to two blocks per SM
+    a.nblocks = std::min(2 * c->sm_count, std::max(1, div_up(a.count, kSorBlock)));
+    a.max_spin = kDefaultSpin;
+    a.phi = phi;
+    a.saved = reinterpret_cast<T *>(base);
+    a.rho = rho;
+    a.partials = reinterpret_cast<double *>(base + nsaved);
+    a.bar = reinterpret_cast<unsigned *>(a.partials + npart);
+    a.status = reinterpret_cast<int *>(a.bar + 2);
+    a.metric = reinterpret_cast<double *>(a.bar + 8);
+    HV_CUDA(cudaMemsetAsync(a.bar, 0, 64, c->stream));
+    void *args[] = {&a};
+    HV_CUDA(cudaLaunchCooperativeKernel((const void *)k_sor_plain<T>, dim3(a.nblocks), dim3(kSorBlock), args, 0,
+                                        c->stream));
+    HV_CUDA(cudaMemcpyAsync(sc.h_result, a.bar, 64, cudaMemcpyDeviceToHost, c->stream));
+    HV_CUDA(cudaStreamSynchronize(c->stream));
+    const int *st = reinterpret_cast<const int *>(sc.h_result) + 2;
+    if (st[0]) {
+        set_last_error("SOR: a bounded device-side wait timed out");
+        return HV_ERR_TIMEOUT;
     }
-    if (iters) *iters = it;
-    if (metric) *metric = m;
-    return converged ? HV_OK : HV_ERR_NOT_CONVERGED;
+    if (iters) *iters = st[1];
+    if (metric) *metric = sc.h_result[4];
+    return st[2] == 1 ? HV_OK : st[2] == 2 ? HV_ERR_NONFINITE : HV_ERR_NOT_CONVERGED;
 }
 
 template <typename T>
@@ -655,7 +818,7 @@ template <typename T>
 hv_status launch_observe(hv_ctx *c, const T *x, const T *y, const T *z, hv_observables *out) {
     const int nb = 2 * c->sm_count;
     k_observe_partials<T><<<nb, kBlock, 0, c->stream>>>(c->geom, c->protons, c->total, x, y, z, c->scratch.partials);
-    k_sum_partials<<<1, 32, 0, c->stream>>>(c->scratch.partials, nb, 6, c->scratch.result);
+    k_sum_partials<<<1, 512, 0, c->stream>>>(c->scratch.partials, nb, 6, c->scratch.result);
     HV_CUDA(cudaGetLastError());
     HV_CUDA(cudaMemcpyAsync(c->scratch.h_result, c->scratch.result, 6 * sizeof(double), cudaMemcpyDeviceToHost,
                             c->stream));
