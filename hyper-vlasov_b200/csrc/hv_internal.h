@@ -274,11 +274,14 @@ hv_status fused_run(hv_ctx *c, int n_steps, hv_observables *obs);
 hv_status fused_autotune(hv_ctx *c, int trial, hv_autotune_report *rep);
 void fused_invalidate(hv_ctx *c);
 
-// Direct Coulomb solve of float contexts (k_poisson.cu)
+// Direct Coulomb solve (k_poisson.cu)
 hv_status poisson_plan(hv_ctx *c);
 void poisson_release(hv_ctx *c);
 bool poisson_direct_runs(const hv_ctx *c);
-hv_status poisson_launch(hv_ctx *c, const float *rho, int *ctl, int *its_ring, int ring, bool step_solve);
+template <typename T>
+hv_status poisson_launch(hv_ctx *c, const T *rho, int *ctl, int *its_ring, int ring, bool step_solve);
+hv_status poisson_launch_adjoint(hv_ctx *c, const double *src, const double *norm, double *mu, double *mu_prev,
+                                 double *mu_guess, int *ctl);
 hv_status poisson_clear(hv_ctx *c);
 
 // Several float SOR solves run by one cooperative launch (k_sor_fast.cu).

@@ -845,8 +845,7 @@ hv_status enqueue_phase_c(hv_ctx *c) {
 // The Coulomb solve: the direct correction where it runs, else the sweeps.
 template <typename T>
 hv_status launch_coulomb(hv_ctx *c, const T *rho, int *its_ring, bool step_solve) {
-    if constexpr (sizeof(T) == 4)
-        if (poisson_direct_runs(c)) return poisson_launch(c, rho, ctl_of(c), its_ring, kRing, step_solve);
+    if (poisson_direct_runs(c)) return poisson_launch<T>(c, rho, ctl_of(c), its_ring, kRing, step_solve);
     return sor_fast_launch<T>(c, rho, ctl_of(c), its_ring, kRing, step_solve);
 }
 

@@ -47,6 +47,11 @@
 namespace hv {
 namespace {
 
+// Double solves take the direct form when their rule is at least this tight: it
+// then pins phi far below what the way to it could show (the correction is in
+// float, the residual and phi in double).  At looser rules the point where the
+// sweeps stop is part of a double run's result, and stays.
+constexpr double kDoubleTol = 1e-9;
 constexpr int kThreads = 512;
 constexpr int kWarps = kThreads / 32;
 
@@ -62,6 +67,8 @@ struct DirectArgs {
     int front;                    // floats of shared memory before the matrices
     double dhx2i, dhy2i, dhz2i, ddiag, src_c, tol;
     float scale;                  // hx^2: the elimination's equations are scaled by it
+    const double *norm;           // largest |source| (null: taken as 1): the float correction works on
+                                  // values of its order, whatever the caller's units
     int max_iter, extrapolate;
     long long max_spin;
     const T *rho;
@@ -420,6 +427,13 @@ __device__ __forceinline__ void direct_body(const DirectArgs<T> &a, const int b)
     const int step = a.ctl[0];
     const int hist = a.extrapolate ? a.ctl[2] : 0;
     const long long sx = (long long)a.ny * a.nz;
+    double unit = 1.0;  // the power of two of the largest source
+    if (a.norm) {
+        const double m = *a.norm;
+        unit = m > 0.0 && m < 1e300 ? exp2(floor(log2(m))) : 1.0;
+    }
+    const double to_float = (double)a.scale / unit;
+    const double cx = a.dhx2i * unit, cy = a.dhy2i * unit, cz = a.dhz2i * unit, cd = a.ddiag * unit;
 
     auto load_dir = [&](bool inverse) {
         if (a.keep_tab) return;
@@ -441,7 +455,7 @@ __device__ __forceinline__ void direct_body(const DirectArgs<T> &a, const int b)
     auto load_delta = [&](long long id, bool) { return __ldcg(a.delta + id); };
     auto to_plane = [&](int y, int z, double r) {
         const int q = z - 1;
-        P[(y - 1) * a.ps + (q < a.hz ? q : a.off + q - a.hz)] = (float)r * a.scale;
+        P[(y - 1) * a.ps + (q < a.hz ? q : a.off + q - a.hz)] = (float)(r * to_float);
     };
     auto totals = [&](double &u, double &v) {
         if (tid < 32) {
@@ -508,7 +522,7 @@ __device__ __forceinline__ void direct_body(const DirectArgs<T> &a, const int b)
                 walk_plane<4>(
                     a, i, load_delta, [&](long long id) { return a.resid[id]; },
                     [&](long long id, int y, int z, float c, double xs, double ys, double zs, double r0) {
-                        const double r = r0 + xs * a.dhx2i + ys * a.dhy2i + zs * a.dhz2i - a.ddiag * (double)c;
+                        const double r = r0 + xs * cx + ys * cy + zs * cz - cd * (double)c;
                         a.resid[id] = r;
                         to_plane(y, z, r);
                     });
@@ -591,19 +605,19 @@ __device__ __forceinline__ void direct_body(const DirectArgs<T> &a, const int b)
                     a, i, load_delta,
                     [&](long long id) { return Node{a.resid[id], start[id], a.phi[id], a.prev[id]}; },
                     [&](long long id, int, int, float c, double xs, double ys, double zs, const Node &n) {
-                        const double r = n.r + xs * a.dhx2i + ys * a.dhy2i + zs * a.dhz2i - a.ddiag * (double)c;
+                        const double r = n.r + xs * cx + ys * cy + zs * cz - cd * (double)c;
                         rr += r * r;
-                        store_first(id, n.start + (double)c, n.phi, n.prev);
+                        store_first(id, n.start + unit * (double)c, n.phi, n.prev);
                     });
             else
                 walk_plane<4>(
                     a, i, load_delta,
                     [&](long long id) { return Node{a.resid[id], a.extrapolate ? a.guess[id] : 0.0, a.phi[id], 0.0}; },
                     [&](long long id, int, int, float c, double xs, double ys, double zs, const Node &n) {
-                        const double r = n.r + xs * a.dhx2i + ys * a.dhy2i + zs * a.dhz2i - a.ddiag * (double)c;
+                        const double r = n.r + xs * cx + ys * cy + zs * cz - cd * (double)c;
                         rr += r * r;
-                        a.phi[id] = n.phi + (double)c;
-                        if (a.extrapolate) a.guess[id] = n.start + again * (double)c;
+                        a.phi[id] = n.phi + unit * (double)c;
+                        if (a.extrapolate) a.guess[id] = n.start + again * unit * (double)c;
                     });
         block_sum2(rr, bb);
         if (tid == 0) a.partials[2 * b] = rr;
@@ -670,18 +684,19 @@ void sine_tables(int m, int pitch, std::vector<float> &fwd, std::vector<float> &
             }
 }
 
-template <bool kBatch>
+template <typename T, bool kBatch>
 const void *direct_kernel(int rt, int nt) {
-    if (rt == 4) return (const void *)k_poisson_direct<float, 4, 1, kBatch>;
-    return nt == 1   ? (const void *)k_poisson_direct<float, 8, 1, kBatch>
-           : nt == 2 ? (const void *)k_poisson_direct<float, 8, 2, kBatch>
-                     : (const void *)k_poisson_direct<float, 8, 3, kBatch>;
+    if (rt == 4) return (const void *)k_poisson_direct<T, 4, 1, kBatch>;
+    return nt == 1   ? (const void *)k_poisson_direct<T, 8, 1, kBatch>
+           : nt == 2 ? (const void *)k_poisson_direct<T, 8, 2, kBatch>
+                     : (const void *)k_poisson_direct<T, 8, 3, kBatch>;
 }
 
-DirectArgs<float> direct_args(hv_ctx *c, const float *rho, int *ctl, int *its_ring, int ring, int nblocks) {
+template <typename T>
+DirectArgs<T> direct_args(hv_ctx *c, const T *rho, int *ctl, int *its_ring, int ring, int nblocks) {
     const PoissonDirect &d = c->fused.direct;
     const Geom &g = c->geom;
-    DirectArgs<float> a;
+    DirectArgs<T> a;
     std::memset(&a, 0, sizeof(a));
     a.nx = g.nx;
     a.ny = g.ny;
@@ -749,7 +764,7 @@ hv_status poisson_plan(hv_ctx *c) {
     PoissonDirect &d = c->fused.direct;
     const Geom &g = c->geom;
     d.ok = false;
-    if (c->prec != HV_F32) return HV_OK;
+    if (c->prec == HV_F64 && c->params.sor.tol > kDoubleTol) return HV_OK;
     const int mx = g.nx - 2, my = g.ny - 2, mz = g.nz - 2;
     const int hy = (my + 1) / 2, hz = (mz + 1) / 2;
     d.off = up(hz, 8);
@@ -789,7 +804,10 @@ hv_status poisson_plan(hv_ctx *c) {
     if (d.smem > limit) return HV_OK;
     // one block per x plane, more where they shorten phase B
     d.nblocks = std::min(c->sm_count, std::max(mx, (ncol + 31) / 32));
-    for (const void *k : {direct_kernel<false>(d.rt, d.nt), direct_kernel<true>(d.rt, d.nt)}) {
+    const bool f64 = c->prec == HV_F64;
+    for (const void *k : {f64 ? direct_kernel<double, false>(d.rt, d.nt) : direct_kernel<float, false>(d.rt, d.nt),
+                          f64 ? nullptr : direct_kernel<float, true>(d.rt, d.nt)}) {
+        if (!k) continue;
         HV_TRY(allow_max_dynamic_smem(k, c->device));
         int per_sm = 0;
         HV_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, kThreads, d.smem));
@@ -831,22 +849,44 @@ void poisson_release(hv_ctx *c) {
     d = PoissonDirect();
 }
 
-// Whether this context's solves take the direct form: float, the
-// relative-residual rule, and the default solver options (the corrected cycles
-// on, the tagged exchange not replaced by phase counters).
+// Whether this context's solves take the direct form: the relative-residual
+// rule and the default solver options (the corrected cycles on, the tagged
+// exchange not replaced by phase counters).
 bool poisson_direct_runs(const hv_ctx *c) {
-    return c->prec == HV_F32 && c->fused.direct.ok && c->fast.sor_coarse &&
-           c->fast.sor_exchange == HV_SOR_EXCHANGE_AUTO && c->params.sor.criterion == HV_SOR_REL_RESIDUAL;
+    return c->fused.direct.ok && c->fast.sor_coarse && c->fast.sor_exchange == HV_SOR_EXCHANGE_AUTO &&
+           c->params.sor.criterion == HV_SOR_REL_RESIDUAL;
 }
 
-hv_status poisson_launch(hv_ctx *c, const float *rho, int *ctl, int *its_ring, int ring, bool step_solve) {
+namespace {
+template <typename T>
+hv_status launch_one(hv_ctx *c, DirectArgs<T> &a) {
     const PoissonDirect &d = c->fused.direct;
-    DirectArgs<float> a = direct_args(c, rho, ctl, its_ring, ring, d.nblocks);
-    if (!step_solve) a.extrapolate = 0;
     void *args[] = {&a};
-    HV_CUDA(cudaLaunchCooperativeKernel(direct_kernel<false>(d.rt, d.nt), dim3(d.nblocks), dim3(kThreads), args,
+    HV_CUDA(cudaLaunchCooperativeKernel(direct_kernel<T, false>(d.rt, d.nt), dim3(d.nblocks), dim3(kThreads), args,
                                         d.smem, c->stream));
     return HV_OK;
+}
+}  // namespace
+
+template <typename T>
+hv_status poisson_launch(hv_ctx *c, const T *rho, int *ctl, int *its_ring, int ring, bool step_solve) {
+    DirectArgs<T> a = direct_args<T>(c, rho, ctl, its_ring, ring, c->fused.direct.nblocks);
+    if (!step_solve) a.extrapolate = 0;
+    return launch_one(c, a);
+}
+template hv_status poisson_launch<float>(hv_ctx *, const float *, int *, int *, int, bool);
+template hv_status poisson_launch<double>(hv_ctx *, const double *, int *, int *, int, bool);
+
+// The adjoint's transposed solve, lap mu = -4 pi e^2 src, with its own history
+// and control words; norm: the largest |src|.
+hv_status poisson_launch_adjoint(hv_ctx *c, const double *src, const double *norm, double *mu, double *mu_prev,
+                                 double *mu_guess, int *ctl) {
+    DirectArgs<double> a = direct_args<double>(c, src, ctl, nullptr, 0, c->fused.direct.nblocks);
+    a.phi = mu;
+    a.prev = mu_prev;
+    a.guess = mu_guess;
+    a.norm = norm;
+    return launch_one(c, a);
 }
 
 // Several direct solves in one cooperative launch: the blocks of the SMs are
@@ -884,7 +924,7 @@ hv_status poisson_wave_build(SorWave &w, const std::vector<hv_ctx *> &cs, const 
     size_t smem = 0;
     for (int i = 0; i < n; i++) {
         const PoissonDirect &d = cs[i]->fused.direct;
-        args.push_back(direct_args(cs[i], rho[i], ctl[i], its_ring[i], ring, blocks[i]));
+        args.push_back(direct_args<float>(cs[i], rho[i], ctl[i], its_ring[i], ring, blocks[i]));
         bfirst[i] = (int)binst.size();
         binst.insert(binst.end(), blocks[i], i);
         if (d.rt == 8) rt = 8;
@@ -892,7 +932,7 @@ hv_status poisson_wave_build(SorWave &w, const std::vector<hv_ctx *> &cs, const 
     }
     if (rt == 8)
         for (hv_ctx *c : cs) nt = std::max(nt, c->fused.direct.nt8);
-    w.kern = direct_kernel<true>(rt, nt);
+    w.kern = direct_kernel<float, true>(rt, nt);
     HV_TRY(allow_max_dynamic_smem(w.kern, cs[0]->device));
     int per_sm = 0;
     HV_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, w.kern, kThreads, smem));

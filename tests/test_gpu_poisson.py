@@ -93,3 +93,50 @@ def test_direct_solve_stops_at_the_iteration_cap(hv):
         obs = s.run(2, hv.HV_PATH_FUSED)
     assert np.all(obs["sor_iterations"] == 1)
     assert np.all(obs["flags"] & 1)
+
+
+@pytest.mark.parametrize("n", [(3, 4, 5), (32, 32, 32), (75, 61, 50), (64, 64, 64), (20, 127, 128)])
+def test_direct_double_solve_matches_the_double_solution(hv, n):
+    """A double context with a rule of 1e-11 takes the direct form.  The solve
+    leaves |r|_2 <= 1e-11 |b|_2, so phi is off by at most |r|_2 over the
+    smallest eigenvalue (and a few roundings of phi)."""
+    from dataclasses import replace
+    tol = 1e-11
+    w = replace(hv.CA40_SMALL, sor_tol=tol, dt=0.25)
+    p = hv.workload_particles(w, np.float64)
+    lam = sum((2.0 - 2.0 * np.cos(np.pi / (m - 1))) * (m / (2.0 * d)) ** 2 for m, d in zip(n, HALF_BOX))
+    with hv.Session(_world(n), w.protons, w.neutrons, w.run_params(), hv.HV_F64) as s:
+        s.upload_particles(*p)
+        for steps in (0, 4):
+            obs = s.run(steps, hv.HV_PATH_FUSED)
+            rho = s.download_field(hv.HV_FIELD_DENSITY).reshape(2, *n)
+            phi = s.download_field(hv.HV_FIELD_COULOMB).reshape(n)
+            ref = exact_phi(n, w.Z, rho[0])
+            b = 4.0 * np.pi * 1.44 * np.linalg.norm(rho[0][1:-1, 1:-1, 1:-1])
+            assert np.abs(phi - ref).max() < tol * b / lam + 1e-13 * np.abs(ref).max(), (n, steps)
+        assert not np.any(obs["flags"] & 1)
+        assert np.all(obs["sor_iterations"] <= 5), obs["sor_iterations"]
+
+
+def test_direct_adjoint_solve_does_not_depend_on_the_objective_scale(hv):
+    """The transposed solves' correction is in float on values scaled to their
+    largest source: the gradient of an objective scaled by 2^-140 (below
+    float's range) is the scaled gradient, and no solve stops unconverged."""
+    from dataclasses import replace
+
+    from hv_b200.adjoint import AdjointRun
+    steps = 6
+    w = replace(hv.CA40_SMALL, ppn=40, sor_tol=1e-12, deposit_mode=hv.HV_DEPOSIT_SORTED)
+    p = hv.workload_particles(w, np.float64)
+    wts = np.random.default_rng(3).standard_normal(steps)
+    run = AdjointRun(w, p, steps, checkpoint_every=3, path=hv.HV_PATH_FUSED)
+    try:
+        run.forward((w.t0, w.t3, w.sigma, w.a_sym))
+        g1 = run.backward(wts)
+        g2 = run.backward(wts * 2.0 ** -140)
+        _, its, unconverged = run.session.adjoint_stats()
+    finally:
+        run.close()
+    assert unconverged == 0 and 0 < its <= 6 * (steps + 1)
+    # each solve's own tolerance, 1e-12, is all that may differ
+    assert np.max(np.abs(g2 * 2.0 ** 140 - g1)) <= 1e-9 * np.abs(g1).max()
