@@ -16,6 +16,7 @@
 namespace hv {
 
 size_t sorted_deposit_tmp_bytes(int total);  // k_plain.cu
+size_t sorted_deposit_entry_bytes(int total, hv_precision prec);
 
 static thread_local std::string g_last_error;
 
@@ -113,6 +114,16 @@ template <>
 State<float> &state<float>(hv_ctx *c) { return c->d32; }
 
 namespace {
+
+// The sorted deposit's entries, once the parameters ask for that mode (steps
+// are captured into graphs, so nothing is allocated when it runs).
+hv_status alloc_entries(hv_ctx *c) {
+    if (c->params.deposit_mode != HV_DEPOSIT_SORTED || c->scratch.entries) return HV_OK;
+    const size_t bytes = sorted_deposit_entry_bytes(c->total, c->prec);
+    HV_CUDA(cudaMalloc(&c->scratch.entries, bytes));
+    HV_CUDA(cudaMemsetAsync(c->scratch.entries, 0, bytes, c->stream));
+    return HV_OK;
+}
 
 // The tap runs and slabs on the device.
 hv_status upload_runs(hv_ctx *c) {
@@ -532,6 +543,7 @@ hv_status hv_ctx_create(const hv_world *world, int protons, int neutrons, hv_pre
         return fail(cuda_status(cudaGetLastError(), "taps upload"));
     st = prec == HV_F64 ? alloc_state<double>(c) : alloc_state<float>(c);
     if (st == HV_OK) st = upload_runs(c);
+    if (st == HV_OK) st = alloc_entries(c);
     if (st != HV_OK) return fail(st);
     const int n = c->total > 0 ? c->total : 1;
     Scratch &s = c->scratch;
@@ -566,7 +578,7 @@ hv_status hv_ctx_destroy(hv_ctx *c) {
     free_state(c->d64);
     free_state(c->d32);
     Scratch &s = c->scratch;
-    void *ptrs[] = {c->perm, c->taps_dev, s.partials, s.sor, c->taps_runs, s.result, s.keys, s.keys_alt, s.vals, s.vals_alt,
+    void *ptrs[] = {c->perm, c->taps_dev, s.partials, s.sor, s.entries, c->taps_runs, s.result, s.keys, s.keys_alt, s.vals, s.vals_alt,
                     s.cell_start, s.cub_tmp, s.sort_tmp};
     for (void *p : ptrs)
         if (p) cudaFree(p);
@@ -606,6 +618,8 @@ hv_status hv_ctx_set_params(hv_ctx *c, const hv_run_params *p) {
         }
         HV_CUDA(cudaStreamSynchronize(c->stream));
     }
+    HV_CUDA(cudaSetDevice(c->device));
+    HV_TRY(alloc_entries(c));
     HV_CUDA(cudaStreamSynchronize(c->stream));
     fused_release(c);  // plans and graphs depend on the parameters
     return HV_OK;

@@ -83,6 +83,7 @@ struct Scratch {
     unsigned int *keys = nullptr, *keys_alt = nullptr;
     int *vals = nullptr, *vals_alt = nullptr;
     int *cell_start = nullptr;      // [2G + 1]
+    void *entries = nullptr;        // sorted particles (allocated when the deposit mode is the sorted one)
     void *cub_tmp = nullptr;
     size_t cub_tmp_bytes = 0;
     void *sort_tmp = nullptr;       // total x 8 bytes: the slot re-sort's gather buffer, and the stage of
