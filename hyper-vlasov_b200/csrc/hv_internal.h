@@ -86,6 +86,9 @@ struct Scratch {
     void *entries = nullptr;        // sorted particles (allocated when the deposit mode is the sorted one)
     void *cub_tmp = nullptr;
     size_t cub_tmp_bytes = 0;
+    void *dens = nullptr;           // per-particle densities: work space, and both results
+    size_t dens_bytes = 0;
+    void *dens_out = nullptr;
     void *sort_tmp = nullptr;       // total x 8 bytes: the slot re-sort's gather buffer, and the stage of
                                     // uploads and downloads in permuted slot order
 };

@@ -113,19 +113,63 @@ __global__ void k_sorted_positions(int total, int protons, const int *__restrict
     sp[s] = v;
 }
 
-// exp(-d2 * e): in float as exp2f(d2 * c) with c = -e log2(e), in double exp.
-__device__ __forceinline__ float gauss(float d2, float e, float c) { return exp2f(d2 * c); }
-__device__ __forceinline__ double gauss(double d2, double e, double) { return exp(-d2 * e); }
+// 2^v for v in [-12, 0]
+__device__ __forceinline__ float exp2_near(float v) {
+    float r;
+    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(v));
+    return r;
+}
+
+// exp(-t) for t in [0, 8], by table (Tang 1989): t log2(e) = n/64 + r' with
+// 2^(-n/64) from 64 doubles and an integer exponent, and exp of the rest, at
+// most ln(2)/128, by its Taylor polynomial of degree 5 (next term 4e-17).
+// Half the double operations of exp.
+struct ExpTable {
+    const double *t;  // 2^(-j/64), j < 64
+    __device__ __forceinline__ double operator()(double v) const {
+        const double shift = 6755399441055744.0;  // 1.5 * 2^52: rounds to an integer in the low word
+        const double q = fma(v, 92.33248261689366, shift);  // 64 / ln 2
+        const int n = __double2loint(q);
+        const double k = q - shift;
+        // r = k ln(2)/64 - v, ln(2)/64 as the sum of two doubles
+        const double r = fma(k, 3.623510646634843e-19, fma(k, 0.010830424696249145, -v));
+        double p = fma(r, 1.0 / 120.0, 1.0 / 24.0);
+        p = fma(p, r, 1.0 / 6.0);
+        p = fma(p, r, 0.5);
+        p = fma(p, r, 1.0);
+        p = fma(p, r, 1.0);
+        const double s = t[n & 63];
+        const double e = __hiloint2double(__double2hiint(s) - ((n >> 6) << 20), __double2loint(s));
+        return p * e;
+    }
+};
+
+// exp(-d2 e): in float 2^(d2 c) with c = -e log2(e), in double by table.
+__device__ __forceinline__ float gauss(float d2, float, float c, const ExpTable &) { return exp2_near(d2 * c); }
+__device__ __forceinline__ double gauss(double d2, double e, double, const ExpTable &t) { return t(d2 * e); }
 
 // Sums over the cells that the cutoff sphere of particle s (sorted order)
 // reaches, results to the particle's own slot.  Per (x, y) row of cells, only
 // the z range of cells within `reach` of the particle is scanned (a sorted,
 // contiguous slot range); reach is the cutoff radius with a margin for the
 // rounding of d^2 in T, whose test decides.
+//
+// Bound by issue slots (23 instructions a scanned partner) and, in double, by
+// the double operations of the exponential.  208Pb, whole calls: 416,000
+// particles in float 8.4 -> 7.8 ms, 104,000 in double 2.9 -> 2.3 ms (exp2f and
+// exp before).  One list for a whole warp, or two particles a thread, measured
+// slower: a warp or thread that crosses from one row of cells into the next
+// then scans the whole nucleus and is waited for.
 template <typename T>
-__global__ void k_pair_densities(int total, Cells cl, double edge, double reach, T exp_term, T exp2_term, T cutoff,
-                                 T term, const int *__restrict__ idx, const int *__restrict__ start,
+__global__ void __launch_bounds__(kBlock) k_pair_densities(int total, Cells cl, double edge, double reach, T exp_term,
+                                                           T exp2_term, T cutoff, T term, const int *__restrict__ idx, const int *__restrict__ start,
                                  const typename Vec4<T>::type *__restrict__ sp, T *dp, T *dn) {
+    __shared__ double powers[64];
+    if (sizeof(T) == 8) {
+        if (threadIdx.x < 64) powers[threadIdx.x] = exp2(-(double)threadIdx.x / 64.0);
+        __syncthreads();
+    }
+    const ExpTable table{powers};
     const int s = blockIdx.x * blockDim.x + threadIdx.x;
     if (s >= total) return;
     const typename Vec4<T>::type me = sp[s];
@@ -151,7 +195,7 @@ __global__ void k_pair_densities(int total, Cells cl, double edge, double reach,
                 const T ex = xi - o.x, ey = yi - o.y, ez = zi - o.z;
                 const T d2 = ex * ex + ey * ey + ez * ez;
                 if (d2 > cutoff) continue;
-                const T f = gauss(d2, exp_term, exp2_term);
+                const T f = gauss(d2, exp_term, exp2_term, table);
                 a += o.w * f;        // protons
                 b += f - o.w * f;    // neutrons
             }
@@ -164,6 +208,21 @@ __global__ void k_pair_densities(int total, Cells cl, double edge, double reach,
 
 }  // namespace
 
+// The work space of these calls, kept by the context and grown when a call
+// needs more (stream-ordered allocations were mapped anew by every call: up to
+// 6 ms beside a 2.4 ms kernel).
+static hv_status dens_work(hv_ctx *c, size_t bytes) {
+    Scratch &sc = c->scratch;
+    if (sc.dens_bytes >= bytes) return HV_OK;
+    HV_CUDA(cudaStreamSynchronize(c->stream));
+    if (sc.dens) cudaFree(sc.dens);
+    sc.dens = nullptr;
+    sc.dens_bytes = 0;
+    HV_CUDA(cudaMalloc(&sc.dens, bytes));
+    sc.dens_bytes = bytes;
+    return HV_OK;
+}
+
 template <typename T>
 hv_status particle_densities_at(hv_ctx *c, int N, int protons, const T *px, const T *py, const T *pz, T *dp_dev,
                                 T *dn_dev) {
@@ -171,12 +230,10 @@ hv_status particle_densities_at(hv_ctx *c, int N, int protons, const T *px, cons
     cudaStream_t s = c->stream;
     // bounding box
     const int bb = std::min(nb(N), 4 * c->sm_count);
-    double *part = nullptr;
-    HV_CUDA(cudaMallocAsync((void **)&part, sizeof(double) * 6 * bb, s));
+    double *part = c->scratch.partials;  // 32 doubles per SM and more
     k_bbox_partials<T><<<bb, kBlock, 0, s>>>(N, px, py, pz, part);
     std::vector<double> hp((size_t)6 * bb);
     HV_CUDA(cudaMemcpyAsync(hp.data(), part, sizeof(double) * 6 * bb, cudaMemcpyDeviceToHost, s));
-    HV_CUDA(cudaFreeAsync(part, s));
     HV_CUDA(cudaStreamSynchronize(s));
     double lo[3] = {1e300, 1e300, 1e300}, hi[3] = {-1e300, -1e300, -1e300};
     for (int b = 0; b < bb; b++)
@@ -201,22 +258,29 @@ hv_status particle_densities_at(hv_ctx *c, int N, int protons, const T *px, cons
     for (int a = 0; a < 3; a++) cl.lo[a] = lo[a];
     cl.inv = 1.0 / edge;
     const int ncells = cl.n[0] * cl.n[1] * cl.n[2];
-    // sort particles by cell
-    unsigned *keys = nullptr, *keys2 = nullptr;
-    int *idx = nullptr, *idx2 = nullptr, *start = nullptr;
-    typename Vec4<T>::type *sp = nullptr;
-    void *tmp = nullptr;
-    size_t tmp_bytes = 0;
+    // sort particles by cell; the context's own sort buffers hold as many
+    // particles as it has
+    Scratch &sc = c->scratch;
     int bits = 1;
     while ((1ll << bits) < ncells + 1) bits++;
-    HV_CUDA(cub::DeviceRadixSort::SortPairs(nullptr, tmp_bytes, keys, keys2, idx, idx2, N, 0, bits, s));
-    HV_CUDA(cudaMallocAsync((void **)&keys, sizeof(unsigned) * N, s));
-    HV_CUDA(cudaMallocAsync((void **)&keys2, sizeof(unsigned) * N, s));
-    HV_CUDA(cudaMallocAsync((void **)&idx, sizeof(int) * N, s));
-    HV_CUDA(cudaMallocAsync((void **)&idx2, sizeof(int) * N, s));
-    HV_CUDA(cudaMallocAsync((void **)&start, sizeof(int) * (ncells + 1), s));
-    HV_CUDA(cudaMallocAsync((void **)&sp, sizeof(typename Vec4<T>::type) * N, s));
-    HV_CUDA(cudaMallocAsync(&tmp, tmp_bytes, s));
+    const bool own = N <= c->total;
+    size_t tmp_bytes = sc.cub_tmp_bytes;
+    if (!own)
+        HV_CUDA(cub::DeviceRadixSort::SortPairs(nullptr, tmp_bytes, (unsigned *)nullptr, (unsigned *)nullptr,
+                                                (int *)nullptr, (int *)nullptr, N, 0, bits, s));
+    auto up = [](size_t n) { return (n + 255) / 256 * 256; };
+    const size_t n4 = up(4 * (size_t)N), nst = up(sizeof(int) * ((size_t)ncells + 1)),
+                 nsp = up(sizeof(typename Vec4<T>::type) * (size_t)N);
+    HV_TRY(dens_work(c, nsp + nst + (own ? 0 : 4 * n4 + up(tmp_bytes))));
+    char *w = static_cast<char *>(sc.dens);
+    typename Vec4<T>::type *sp = reinterpret_cast<typename Vec4<T>::type *>(w);
+    int *start = reinterpret_cast<int *>(w + nsp);
+    w += nsp + nst;
+    unsigned *keys = own ? sc.keys : reinterpret_cast<unsigned *>(w);
+    unsigned *keys2 = own ? sc.keys_alt : reinterpret_cast<unsigned *>(w + n4);
+    int *idx = own ? sc.vals : reinterpret_cast<int *>(w + 2 * n4);
+    int *idx2 = own ? sc.vals_alt : reinterpret_cast<int *>(w + 3 * n4);
+    void *tmp = own ? sc.cub_tmp : w + 4 * n4;
     k_cell_of<T><<<nb(N), kBlock, 0, s>>>(N, cl, px, py, pz, keys, idx);
     HV_CUDA(cub::DeviceRadixSort::SortPairs(tmp, tmp_bytes, keys, keys2, idx, idx2, N, 0, bits, s));
     k_cell_ranges<<<nb(N + 1), kBlock, 0, s>>>(N, ncells, keys2, start);
@@ -226,11 +290,9 @@ hv_status particle_densities_at(hv_ctx *c, int N, int protons, const T *px, cons
     const T exp2_term = T(-1.4426950408889634) * exp_term;  // -log2(e) / (2 sigma_r^2)
     const T term = (T(1.0) / c->params.part_per_nucleon) * (T(1.0) / std::pow(T(2.0) * T(kPi) * sr * sr, T(1.5)));
     const double reach = 4.0 * sig * (1.0 + 1e-5);
-    k_pair_densities<T><<<nb(N), kBlock, 0, s>>>(N, cl, edge, reach, exp_term, exp2_term, cutoff, term, idx2, start, sp, dp_dev,
-                                                 dn_dev);
+    k_pair_densities<T><<<nb(N), kBlock, 0, s>>>(N, cl, edge, reach, exp_term, exp2_term, cutoff, term, idx2, start, sp,
+                                                 dp_dev, dn_dev);
     HV_CUDA(cudaGetLastError());
-    void *bufs[] = {keys, keys2, idx, idx2, start, sp, tmp};
-    for (void *p : bufs) HV_CUDA(cudaFreeAsync(p, s));
     return HV_OK;
 }
 
@@ -248,9 +310,9 @@ extern "C" hv_status hv_particle_densities(hv_ctx *c, void *density_p, void *den
     HV_CUDA(cudaSetDevice(c->device));
     if (c->total == 0) return HV_OK;
     const size_t es = c->prec == HV_F64 ? 8 : 4, bytes = es * c->total;
-    void *dp = nullptr, *dn = nullptr;
-    HV_CUDA(cudaMallocAsync(&dp, bytes, c->stream));
-    HV_CUDA(cudaMallocAsync(&dn, bytes, c->stream));
+    Scratch &sc = c->scratch;
+    if (!sc.dens_out) HV_CUDA(cudaMalloc(&sc.dens_out, 2 * bytes));
+    void *dp = sc.dens_out, *dn = static_cast<char *>(sc.dens_out) + bytes;
     hv_status st = c->prec == HV_F64
                        ? particle_densities_at<double>(c, c->total, c->protons, c->d64.x, c->d64.y, c->d64.z,
                                                        (double *)dp, (double *)dn)
@@ -258,8 +320,6 @@ extern "C" hv_status hv_particle_densities(hv_ctx *c, void *density_p, void *den
                                                       (float *)dp, (float *)dn);
     if (st == HV_OK) st = download_slots(c, dp, density_p);
     if (st == HV_OK) st = download_slots(c, dn, density_n);
-    cudaFreeAsync(dp, c->stream);
-    cudaFreeAsync(dn, c->stream);
     HV_CUDA(cudaStreamSynchronize(c->stream));
     return st;
 }
