@@ -231,6 +231,44 @@ __global__ void k_slot_keys(Geom g, int protons, int total, const T *__restrict_
     vals[i] = i;
 }
 
+// What a slot re-sort moves: x, y, z, kx, ky, kz and the caller permutation.
+template <typename T>
+struct SlotArrays {
+    T *v[6];
+    int *perm;
+};
+
+template <typename T>
+__global__ void k_gather_slots(int n, const int *__restrict__ from, SlotArrays<T> in, SlotArrays<T> out) {
+    const int s = blockIdx.x * blockDim.x + threadIdx.x;
+    if (s >= n) return;
+    const int i = from[s];
+    T v[6];
+#pragma unroll
+    for (int q = 0; q < 6; q++) v[q] = in.v[q][i];
+    const int p = in.perm[i];
+#pragma unroll
+    for (int q = 0; q < 6; q++) out.v[q][s] = v[q];
+    out.perm[s] = p;
+}
+
+template <typename T>
+__global__ void k_copy_slots(int n, SlotArrays<T> in, SlotArrays<T> out) {
+    const int s0 = blockIdx.x * 1024 + threadIdx.x;
+#pragma unroll
+    for (int u = 0; u < 4; u++) {
+        const int s = s0 + 256 * u;
+        if (s >= n) break;
+        T v[6];
+#pragma unroll
+        for (int q = 0; q < 6; q++) v[q] = in.v[q][s];
+        const int p = in.perm[s];
+#pragma unroll
+        for (int q = 0; q < 6; q++) out.v[q][s] = v[q];
+        out.perm[s] = p;
+    }
+}
+
 template <typename T>
 hv_status sort_slots_typed(hv_ctx *c, State<T> &s) {
     const int n = c->total;
@@ -244,16 +282,17 @@ hv_status sort_slots_typed(hv_ctx *c, State<T> &s) {
     size_t bytes = sc.cub_tmp_bytes;
     HV_CUDA(cub::DeviceRadixSort::SortPairs(sc.cub_tmp, bytes, sc.keys, sc.keys_alt, sc.vals, sc.vals_alt, n, 0,
                                             end_bit, c->stream));
-    // every per-particle array and the caller permutation follow the new order
-    T *tmp = reinterpret_cast<T *>(sc.sort_tmp);
-    T *arrs[] = {s.x, s.y, s.z, s.kx, s.ky, s.kz, s.fx, s.fy, s.fz};
-    for (T *a : arrs) {
-        k_permute<T><<<div_up(n, 256), 256, 0, c->stream>>>(n, sc.vals_alt, a, tmp);
-        HV_CUDA(cudaMemcpyAsync(a, tmp, sizeof(T) * (size_t)n, cudaMemcpyDeviceToDevice, c->stream));
-    }
-    int *ptmp = reinterpret_cast<int *>(sc.sort_tmp);
-    k_permute<int><<<div_up(n, 256), 256, 0, c->stream>>>(n, sc.vals_alt, c->perm, ptmp);
-    HV_CUDA(cudaMemcpyAsync(c->perm, ptmp, sizeof(int) * (size_t)n, cudaMemcpyDeviceToDevice, c->stream));
+    // positions, wavenumbers and the caller permutation follow the new order:
+    // gathered into a kept buffer, copied back in one go.  (The forces are not
+    // carried: a fused run writes them at its end, from the field.)
+    const size_t stride = ((size_t)n + 63) / 64 * 64;
+    if (!sc.sort_stage) HV_CUDA(cudaMalloc(&sc.sort_stage, stride * (6 * sizeof(T) + sizeof(int))));
+    SlotArrays<T> a{{s.x, s.y, s.z, s.kx, s.ky, s.kz}, c->perm}, b;
+    T *stage = static_cast<T *>(sc.sort_stage);
+    for (int q = 0; q < 6; q++) b.v[q] = stage + q * stride;
+    b.perm = reinterpret_cast<int *>(stage + 6 * stride);
+    k_gather_slots<T><<<div_up(n, 256), 256, 0, c->stream>>>(n, sc.vals_alt, a, b);
+    k_copy_slots<T><<<div_up(n, 1024), 256, 0, c->stream>>>(n, b, a);
     HV_CUDA(cudaGetLastError());
     c->permuted = true;
     return HV_OK;
@@ -578,7 +617,7 @@ hv_status hv_ctx_destroy(hv_ctx *c) {
     free_state(c->d64);
     free_state(c->d32);
     Scratch &s = c->scratch;
-    void *ptrs[] = {c->perm, c->taps_dev, s.partials, s.sor, s.entries, s.dens, s.dens_out, c->taps_runs, s.result, s.keys, s.keys_alt, s.vals, s.vals_alt,
+    void *ptrs[] = {c->perm, c->taps_dev, s.partials, s.sor, s.sort_stage, s.entries, s.dens, s.dens_out, c->taps_runs, s.result, s.keys, s.keys_alt, s.vals, s.vals_alt,
                     s.cell_start, s.cub_tmp, s.sort_tmp};
     for (void *p : ptrs)
         if (p) cudaFree(p);

@@ -52,6 +52,38 @@ static __device__ bool grid_barrier(unsigned *bar, int nblocks, int *err, long l
     return ok;
 }
 
+// The same with half the round trips: one counter that only grows.  Each block
+// adds one (a release) and polls for the sum of all; `target` is the count that
+// ends the barrier, advanced by every call.  bar[1] holds the count at which
+// the launch before ended: every block takes it as its first target's base
+// (epoch_base) before its first barrier, and block 0 leaves the final count
+// there after the last one (epoch_end).  A solve that gave up leaves the words
+// inconsistent; the host zeroes them before the next run.
+// Per barrier on 126 blocks: 2.1 us against 3.1.
+__device__ __forceinline__ unsigned epoch_base(const unsigned *bar) { return ld_relaxed(bar + 1); }
+__device__ __forceinline__ void epoch_end(unsigned *bar, unsigned target) { bar[1] = target; }
+static __device__ bool epoch_barrier(unsigned *bar, unsigned &target, int nblocks, int *err, long long max_spin) {
+    __shared__ int ok;
+    target += (unsigned)nblocks;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        int good = 1;
+        asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(bar) : "memory");
+        long long spin = 0;
+        while ((int)(ld_relaxed(bar) - target) < 0) {
+            if (++spin > max_spin || ((spin & 15) == 0 && ld_volatile(err))) {
+                atomicExch(err, 1);
+                good = 0;
+                break;
+            }
+        }
+        fence_acq_rel();
+        ok = good;
+    }
+    __syncthreads();
+    return ok;
+}
+
 // Deterministic block sum of two doubles (fixed shuffle tree, fixed warp order)
 // for blocks of whole warps, at most 32; the result is valid in thread 0.
 static __device__ void block_sum2(double &u, double &v) {

@@ -89,7 +89,8 @@ struct Scratch {
     void *dens = nullptr;           // per-particle densities: work space, and both results
     size_t dens_bytes = 0;
     void *dens_out = nullptr;
-    void *sort_tmp = nullptr;       // total x 8 bytes: the slot re-sort's gather buffer, and the stage of
+    void *sort_stage = nullptr;     // the slot re-sort's gathered arrays
+    void *sort_tmp = nullptr;       // total x 8 bytes: the stage of
                                     // uploads and downloads in permuted slot order
 };
 
@@ -133,7 +134,7 @@ struct PoissonDirect {
     float *work = nullptr;     // the planes' spectrum
     float *delta = nullptr;    // correction per node, zero on the faces
     double *partials = nullptr;
-    unsigned *bar = nullptr;   // [0] arrivals, [1] generation
+    unsigned *bar = nullptr;   // [0] arrivals, [1] their count at the last solve's end
 };
 
 // Decomposed smoothing plan (k_smooth_fast.cu).

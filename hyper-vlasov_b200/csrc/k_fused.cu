@@ -33,9 +33,7 @@ namespace {
 constexpr int kPBlock = 256;      // default threads per block of the particle step
 constexpr int kPBlockMax = 512;   // largest of the autotuner's candidates
 constexpr int kPGridMax = 16;     // most blocks per SM of the particle step
-constexpr int kForceRows = 8;     // y rows per thread of the forces kernel on every row
-constexpr int kForceRowsGated = 4; // the same where only rows holding raw density are computed:
-                                   // shorter walks, as few blocks work (an eighth on 208Pb 128^3)
+constexpr int kForceRows = 4;     // y rows per thread of the forces kernel
 constexpr int kRing = 64;  // observable rows kept on the device
 
 // control words (Fused::ctl)
@@ -555,24 +553,23 @@ inline long long skyrme_threads(long long G) {
 // group of four rows.
 template <typename T>
 __global__ void k_forces_f4(Geom g, T idx, T idy, T idz, const T *__restrict__ U, const double *__restrict__ phi,
-                            T *F4, int *advance, const T *__restrict__ raw, int rows,
-                            const unsigned *__restrict__ occ) {
+                            T *F4, int *advance, const T *__restrict__ raw, const unsigned *__restrict__ occ) {
     // the step's last kernel also advances the step counter (advance: the
     // control words; null for the initial solve)
     if (advance && blockIdx.x == 0 && blockIdx.y == 0 && blockIdx.z == 0 && threadIdx.x == 0) {
         advance[CTL_STEP] += 1;
         advance[CTL_CLOSE] = 1;
     }
-    // block (row group, x plane, species), threads along z: each thread walks
-    // `rows` consecutive y rows at its z, keeping the y-1, y and y+1 values
-    // of U + phi in registers, so a node loads five values, not seven
+    // block (group of kForceRows y rows, x plane, species), threads along z.  A
+    // thread loads every value its rows' differences need before it forms the
+    // first one, so that the kernel waits for memory once, not once per row
     const int ii = blockIdx.y;
     const bool prot = blockIdx.z == 0;
     const int nx = g.nx, ny = g.ny, nz = g.nz;
     const long long sx = (long long)ny * nz, sy = nz;
     const T *Us = U + (prot ? 0 : g.G);
     auto u = [&](long long q) { return prot ? Us[q] + (T)phi[q] : Us[q]; };
-    const int j0 = blockIdx.x * rows, j1 = min(j0 + rows, ny);
+    const int j0 = blockIdx.x * kForceRows, j1 = min(j0 + kForceRows, ny);
     if (occ) {
         if (!((occ[blockIdx.z * nx + ii] >> blockIdx.x) & 1u)) return;
     } else if (raw) {
@@ -583,22 +580,35 @@ __global__ void k_forces_f4(Geom g, T idx, T idy, T idz, const T *__restrict__ U
         if (!__syncthreads_or(any)) return;
     }
     for (int k = threadIdx.x; k < nz; k += blockDim.x) {
-        long long id = (long long)ii * sx + (long long)j0 * sy + k;
-        T um = j0 > 0 ? u(id - sy) : T(0);
-        T uc = u(id);
-        for (int j = j0; j < j1; j++, id += sy) {
-            const T up = j + 1 < ny ? u(id + sy) : T(0);
+        const long long plane = (long long)ii * sx + k;
+        T c[kForceRows + 2], xm[kForceRows], xp[kForceRows], zm[kForceRows], zp[kForceRows];
+#pragma unroll
+        for (int q = 0; q < kForceRows + 2; q++) c[q] = u(plane + min(max(j0 + q - 1, 0), ny - 1) * sy);
+#pragma unroll
+        for (int q = 0; q < kForceRows; q++) {
+            // neighbours past a face repeat the node: the one-sided formulas skip them
+            const long long id = plane + min(j0 + q, ny - 1) * sy;
+            xm[q] = u(ii > 0 ? id - sx : id);
+            xp[q] = u(ii < nx - 1 ? id + sx : id);
+            zm[q] = u(k > 0 ? id - 1 : id);
+            zp[q] = u(k < nz - 1 ? id + 1 : id);
+        }
+#pragma unroll
+        for (int q = 0; q < kForceRows; q++) {
+            const int j = j0 + q;
+            if (j >= j1) break;
+            const T uc = c[q + 1];
             T gx, gy, gz;
-            if (ii == 0) gx = (u(id + sx) - uc) * idx;
-            else if (ii == nx - 1) gx = (uc - u(id - sx)) * idx;
-            else gx = (u(id + sx) - u(id - sx)) * (T(0.5) * idx);
-            if (j == 0) gy = (up - uc) * idy;
-            else if (j == ny - 1) gy = (uc - um) * idy;
-            else gy = (up - um) * (T(0.5) * idy);
-            if (k == 0) gz = (u(id + 1) - uc) * idz;
-            else if (k == nz - 1) gz = (uc - u(id - 1)) * idz;
-            else gz = (u(id + 1) - u(id - 1)) * (T(0.5) * idz);
-            const long long i = (prot ? 0 : g.G) + id;
+            if (ii == 0) gx = (xp[q] - uc) * idx;
+            else if (ii == nx - 1) gx = (uc - xm[q]) * idx;
+            else gx = (xp[q] - xm[q]) * (T(0.5) * idx);
+            if (j == 0) gy = (c[q + 2] - uc) * idy;
+            else if (j == ny - 1) gy = (uc - c[q]) * idy;
+            else gy = (c[q + 2] - c[q]) * (T(0.5) * idy);
+            if (k == 0) gz = (zp[q] - uc) * idz;
+            else if (k == nz - 1) gz = (uc - zm[q]) * idz;
+            else gz = (zp[q] - zm[q]) * (T(0.5) * idz);
+            const long long i = (prot ? 0 : g.G) + plane + (long long)j * sy;
             if constexpr (sizeof(T) == 4) {
                 reinterpret_cast<float4 *>(F4)[i] = make_float4(-gx, -gy, -gz, 0.0f);
             } else {
@@ -608,16 +618,14 @@ __global__ void k_forces_f4(Geom g, T idx, T idy, T idz, const T *__restrict__ U
                 o[2] = -gz;
                 o[3] = T(0);
             }
-            um = uc;
-            uc = up;
         }
     }
 }
 
-// k_forces_f4's launch: one block per (group of `rows` y rows, x plane,
+// k_forces_f4's launch: one block per (group of kForceRows y rows, x plane,
 // species), threads along z
-inline dim3 forces_grid(const Geom &g, int rows) {
-    return dim3((unsigned)((g.ny + rows - 1) / rows), (unsigned)g.nx, 2u);
+inline dim3 forces_grid(const Geom &g) {
+    return dim3((unsigned)((g.ny + kForceRows - 1) / kForceRows), (unsigned)g.nx, 2u);
 }
 inline dim3 forces_block(const Geom &g) { return dim3((unsigned)std::min(128, (g.nz + 31) / 32 * 32)); }
 
@@ -825,18 +833,21 @@ hv_status enqueue_phase_c(hv_ctx *c) {
     // with the reference's division, which can put a particle on a cell face
     // into the neighbouring cell of the gather's (a product by the reciprocal),
     // so its steps compute every row.
-    const T *raw = (sizeof(T) == 4 && c->params.deposit_mode != HV_DEPOSIT_SORTED) ? s.rho_raw : nullptr;
+    // Below 72^3 nodes the whole field costs less than the wait for the test
+    // of the raw density (64^3: 5 us against 12).
+    const T *raw = (sizeof(T) == 4 && c->params.deposit_mode != HV_DEPOSIT_SORTED && g.G >= 72ll * 72 * 72)
+                       ? s.rho_raw
+                       : nullptr;
     {
         ProfScope ps(c, HV_K_FORCES);
-        const int rows = raw ? kForceRowsGated : kForceRows;
         // the 128^3 FFT smoothing's occupancy bits: 32 groups of four rows
         const unsigned *occ = (raw && f.smooth.fft128 && f.smooth.occ && smooth_fft_runs(c) &&
-                               g.ny == 32 * kForceRowsGated)
+                               g.ny == 32 * kForceRows)
                                   ? f.smooth.occ
                                   : nullptr;
-        k_forces_f4<T><<<forces_grid(g, rows), forces_block(g), 0, c->stream>>>(g, idx, idy, idz, s.U, f.phi64,
+        k_forces_f4<T><<<forces_grid(g), forces_block(g), 0, c->stream>>>(g, idx, idy, idz, s.U, f.phi64,
                                                                         reinterpret_cast<T *>(f.F4), ctl, raw,
-                                                                        rows, occ);
+                                                                        occ);
     }
     HV_CUDA(cudaGetLastError());
     return HV_OK;
@@ -924,8 +935,8 @@ hv_status initial_typed(hv_ctx *c) {
     HV_TRY(launch_coulomb<T>(c, s.rho, nullptr, false));
     const T idx = T(1.0) / (T(2.0) * T(g.dmx) / g.nx), idy = T(1.0) / (T(2.0) * T(g.dmy) / g.ny),
             idz = T(1.0) / (T(2.0) * T(g.dmz) / g.nz);
-    k_forces_f4<T><<<forces_grid(g, kForceRows), forces_block(g), 0, c->stream>>>(
-        g, idx, idy, idz, s.U, f.phi64, reinterpret_cast<T *>(f.F4), nullptr, nullptr, kForceRows, nullptr);
+    k_forces_f4<T><<<forces_grid(g), forces_block(g), 0, c->stream>>>(
+        g, idx, idy, idz, s.U, f.phi64, reinterpret_cast<T *>(f.F4), nullptr, nullptr, nullptr);
     HV_CUDA(cudaGetLastError());
     int status[3] = {0, 0, 0};
     HV_CUDA(cudaMemcpyAsync(status, f.sor.status, sizeof(int) * 3, cudaMemcpyDeviceToHost, c->stream));
@@ -1190,8 +1201,8 @@ hv_status run_end(hv_ctx *c, int n_steps, int exc) {
         // same U and phi (before the merge below adds phi to U)
         const T idx = T(1.0) / (T(2.0) * T(g.dmx) / g.nx), idy = T(1.0) / (T(2.0) * T(g.dmy) / g.ny),
                 idz = T(1.0) / (T(2.0) * T(g.dmz) / g.nz);
-        k_forces_f4<T><<<forces_grid(g, kForceRows), forces_block(g), 0, c->stream>>>(
-            g, idx, idy, idz, S.U, f.phi64, reinterpret_cast<T *>(f.F4), nullptr, nullptr, kForceRows, nullptr);
+        k_forces_f4<T><<<forces_grid(g), forces_block(g), 0, c->stream>>>(
+            g, idx, idy, idz, S.U, f.phi64, reinterpret_cast<T *>(f.F4), nullptr, nullptr, nullptr);
     }
     if (c->total > 0)
         k_close_kick<T><<<nblk(c->total, 256), 256, 0, c->stream>>>(g, c->protons, c->total, S.x, S.y, S.z, S.kx, S.ky,

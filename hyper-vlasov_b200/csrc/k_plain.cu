@@ -454,6 +454,7 @@ __global__ void __launch_bounds__(kSorBlock, 2) k_sor_plain(PlainSor<T> a) {
         }
     };
 
+    unsigned target = 0;  // the host zeroes the barrier before each launch
     int it = 0;
     while (true) {
         it++;
@@ -476,7 +477,7 @@ __global__ void __launch_bounds__(kSorBlock, 2) k_sor_plain(PlainSor<T> a) {
                 break;
             }
         }
-        if (!grid_barrier(a.bar, a.nblocks, a.status, a.max_spin)) return;
+        if (!epoch_barrier(a.bar, target, a.nblocks, a.status, a.max_spin)) return;
         if (rel && it > 1 && tid < 32) test(it - 1);
         sweep(1, it == 1);
         if (rel) {
@@ -496,7 +497,7 @@ __global__ void __launch_bounds__(kSorBlock, 2) k_sor_plain(PlainSor<T> a) {
                 a.partials[2 * b] = (double)m;
             }
         }
-        if (!grid_barrier(a.bar, a.nblocks, a.status, a.max_spin)) return;
+        if (!epoch_barrier(a.bar, target, a.nblocks, a.status, a.max_spin)) return;
     }
     if (b == 0 && tid == 0) {
         a.status[1] = it - 1;

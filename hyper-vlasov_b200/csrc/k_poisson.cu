@@ -493,6 +493,7 @@ __device__ __forceinline__ void direct_body(const DirectArgs<T> &a, const int b)
     // a later one adds its share of the extrapolation too
     const double again = a.extrapolate == 2 && hist > 0 ? 3.0 : 2.0;
 
+    unsigned target = epoch_base(a.bar);
     int its = 0;
     double rel = 0.0, bsum = 0.0;
     bool converged = false;
@@ -541,7 +542,7 @@ __device__ __forceinline__ void direct_body(const DirectArgs<T> &a, const int b)
                 a.partials[2 * b + 1] = bb;
             }
         }
-        if (!grid_barrier(a.bar, a.nblocks, err, a.max_spin)) return;
+        if (!epoch_barrier(a.bar, target, a.nblocks, err, a.max_spin)) return;
         if (its == 0) {
             double u;
             totals(u, bsum);
@@ -559,7 +560,7 @@ __device__ __forceinline__ void direct_body(const DirectArgs<T> &a, const int b)
         // ---- B: along x -------------------------------------------------------
         const int groups = (a.my * a.wz + a.cw - 1) / a.cw;
         for (int g = b; g < groups; g += a.nblocks) solve_columns(a, sm, g);
-        if (!grid_barrier(a.bar, a.nblocks, err, a.max_spin)) return;
+        if (!epoch_barrier(a.bar, target, a.nblocks, err, a.max_spin)) return;
         // ---- C: inverse transforms -------------------------------------------
         load_dir(true);
         for (int i = 1 + b; i <= a.mx; i += a.nblocks) {
@@ -596,7 +597,7 @@ __device__ __forceinline__ void direct_body(const DirectArgs<T> &a, const int b)
                 }
             __syncthreads();
         }
-        if (!grid_barrier(a.bar, a.nblocks, err, a.max_spin)) return;
+        if (!epoch_barrier(a.bar, target, a.nblocks, err, a.max_spin)) return;
         // ---- D: phi += delta, the FP64 residual of the new phi ---------------
         rr = bb = 0.0;
         for (int i = 1 + b; i <= a.mx; i += a.nblocks)
@@ -621,7 +622,7 @@ __device__ __forceinline__ void direct_body(const DirectArgs<T> &a, const int b)
                     });
         block_sum2(rr, bb);
         if (tid == 0) a.partials[2 * b] = rr;
-        if (!grid_barrier(a.bar, a.nblocks, err, a.max_spin)) return;
+        if (!epoch_barrier(a.bar, target, a.nblocks, err, a.max_spin)) return;
         double u, none;
         totals(u, none);
         rel = bsum > 0.0 ? sqrt(u / bsum) : sqrt(u);
@@ -630,6 +631,7 @@ __device__ __forceinline__ void direct_body(const DirectArgs<T> &a, const int b)
         if (converged || its >= a.max_iter || !(rel == rel)) break;
     }
     if (b == 0 && tid == 0) {
+        epoch_end(a.bar, target);
         a.status[1] = its;
         a.status[2] = converged ? 1 : 0;
         a.status[3] = its + 1;
