@@ -127,8 +127,9 @@ struct PoissonDirect {
     int off = 0, wz = 0, ps = 0, py = 0;  // stored plane: second half's column, columns, pitch; y matrices' pitch
     int rt = 0, nt = 0;        // kernel form: rows of a thread's tile, tiles per warp
     int nt8 = 0;               // tiles per warp with eight rows (launches shared with larger planes)
-    int shared_tab = 0, keep_tab = 0, front = 0, cw_max = 0, nblocks = 0;
-    size_t smem = 0;
+    int shared_tab = 0, nblocks = 0;
+    int plane = 0, one = 0;    // floats of the stored plane, of one direction's matrices
+    size_t limit = 0, smem = 0;
     float *tables = nullptr;   // sine matrices of z and y, both directions, and the eigenvalues (owns the
                                // allocation the pointers below lie in)
     float *work = nullptr;     // the planes' spectrum

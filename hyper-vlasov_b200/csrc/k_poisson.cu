@@ -427,13 +427,20 @@ __device__ __forceinline__ void direct_body(const DirectArgs<T> &a, const int b)
     const int step = a.ctl[0];
     const int hist = a.extrapolate ? a.ctl[2] : 0;
     const long long sx = (long long)a.ny * a.nz;
-    double unit = 1.0;  // the power of two of the largest source
-    if (a.norm) {
-        const double m = *a.norm;
-        unit = m > 0.0 && m < 1e300 ? exp2(floor(log2(m))) : 1.0;
+    // the power of two of the largest source: the unit of the correction
+    // (double contexts only; a float context's sources are densities)
+    double unit = 1.0;
+    if constexpr (sizeof(T) == 8) {
+        if (a.norm) {
+            const double m = *a.norm;
+            unit = m > 0.0 && m < 1e300 ? exp2(floor(log2(m))) : 1.0;
+        }
     }
-    const double to_float = (double)a.scale / unit;
-    const double cx = a.dhx2i * unit, cy = a.dhy2i * unit, cz = a.dhz2i * unit, cd = a.ddiag * unit;
+    auto lap = [&](double xs, double ys, double zs, float c) {
+        const double v = xs * a.dhx2i + ys * a.dhy2i + zs * a.dhz2i - a.ddiag * (double)c;
+        return sizeof(T) == 8 ? unit * v : v;
+    };
+    auto value = [&](float c) { return sizeof(T) == 8 ? unit * (double)c : (double)c; };
 
     auto load_dir = [&](bool inverse) {
         if (a.keep_tab) return;
@@ -455,7 +462,7 @@ __device__ __forceinline__ void direct_body(const DirectArgs<T> &a, const int b)
     auto load_delta = [&](long long id, bool) { return __ldcg(a.delta + id); };
     auto to_plane = [&](int y, int z, double r) {
         const int q = z - 1;
-        P[(y - 1) * a.ps + (q < a.hz ? q : a.off + q - a.hz)] = (float)(r * to_float);
+        P[(y - 1) * a.ps + (q < a.hz ? q : a.off + q - a.hz)] = sizeof(T) == 8 ? (float)(r / unit) * a.scale : (float)r * a.scale;
     };
     auto totals = [&](double &u, double &v) {
         if (tid < 32) {
@@ -523,7 +530,7 @@ __device__ __forceinline__ void direct_body(const DirectArgs<T> &a, const int b)
                 walk_plane<4>(
                     a, i, load_delta, [&](long long id) { return a.resid[id]; },
                     [&](long long id, int y, int z, float c, double xs, double ys, double zs, double r0) {
-                        const double r = r0 + xs * cx + ys * cy + zs * cz - cd * (double)c;
+                        const double r = r0 + lap(xs, ys, zs, c);
                         a.resid[id] = r;
                         to_plane(y, z, r);
                     });
@@ -606,19 +613,19 @@ __device__ __forceinline__ void direct_body(const DirectArgs<T> &a, const int b)
                     a, i, load_delta,
                     [&](long long id) { return Node{a.resid[id], start[id], a.phi[id], a.prev[id]}; },
                     [&](long long id, int, int, float c, double xs, double ys, double zs, const Node &n) {
-                        const double r = n.r + xs * cx + ys * cy + zs * cz - cd * (double)c;
+                        const double r = n.r + lap(xs, ys, zs, c);
                         rr += r * r;
-                        store_first(id, n.start + unit * (double)c, n.phi, n.prev);
+                        store_first(id, n.start + value(c), n.phi, n.prev);
                     });
             else
                 walk_plane<4>(
                     a, i, load_delta,
                     [&](long long id) { return Node{a.resid[id], a.extrapolate ? a.guess[id] : 0.0, a.phi[id], 0.0}; },
                     [&](long long id, int, int, float c, double xs, double ys, double zs, const Node &n) {
-                        const double r = n.r + xs * cx + ys * cy + zs * cz - cd * (double)c;
+                        const double r = n.r + lap(xs, ys, zs, c);
                         rr += r * r;
-                        a.phi[id] = n.phi + unit * (double)c;
-                        if (a.extrapolate) a.guess[id] = n.start + again * unit * (double)c;
+                        a.phi[id] = n.phi + value(c);
+                        if (a.extrapolate) a.guess[id] = n.start + again * value(c);
                     });
         block_sum2(rr, bb);
         if (tid == 0) a.partials[2 * b] = rr;
@@ -686,6 +693,33 @@ void sine_tables(int m, int pitch, std::vector<float> &fwd, std::vector<float> &
             }
 }
 
+// Shared memory of a solve with nblocks blocks.  Phase B's columns, an equal
+// share per block in sixteens (a half-warp each from either end; at most 256,
+// all 16 warps), and their coefficients lie where the plane lies; the matrices
+// follow, both directions where they fit, else over the columns.  No more is
+// asked for than that: what is left of the SM's 256 KB caches the walks' loads
+// (128^3: 114 us with 149 KB, 123 with 220).
+struct Layout {
+    bool ok;
+    int cw, front, keep_tab;
+    size_t smem;
+};
+Layout layout(const PoissonDirect &d, const Geom &g, int nblocks) {
+    const int mx = g.nx - 2, ncol = (g.ny - 2) * d.wz;
+    const size_t col = (size_t)(mx + mx / 2 + 1), plane = d.plane, one = d.one;
+    int cw = std::min(up((ncol + nblocks - 1) / nblocks, 16), 256);
+    while (cw > 16 && col * cw * sizeof(float) > d.limit) cw -= 16;
+    auto total = [&](int w) { return (std::max(plane, col * w) + 2 * one) * sizeof(float); };
+    while (cw > 64 && total(cw) > d.limit) cw -= 16;
+    Layout l;
+    l.cw = cw;
+    l.keep_tab = total(cw) <= d.limit ? 1 : 0;
+    l.front = (int)(l.keep_tab ? std::max(plane, col * cw) : plane);
+    l.smem = l.keep_tab ? total(cw) : std::max(plane + one, col * cw) * sizeof(float);
+    l.ok = l.smem <= d.limit;
+    return l;
+}
+
 template <typename T, bool kBatch>
 const void *direct_kernel(int rt, int nt) {
     if (rt == 4) return (const void *)k_poisson_direct<T, 4, 1, kBatch>;
@@ -715,13 +749,11 @@ DirectArgs<T> direct_args(hv_ctx *c, const T *rho, int *ctl, int *its_ring, int 
     a.zlen = 2 * d.off * d.off;
     a.ylen = 2 * d.py * d.py;
     a.shared_tab = d.shared_tab;
-    a.keep_tab = d.keep_tab;
-    a.front = d.front;
+    const Layout lay = layout(d, g, nblocks);
+    a.keep_tab = lay.keep_tab;
+    a.front = lay.front;
     a.nblocks = nblocks;
-    // phase B: an equal share of the columns per block, in sixteens (a
-    // half-warp each from either end), as many as shared memory holds
-    const int ncol = a.my * a.wz;
-    a.cw = std::min(up((ncol + nblocks - 1) / nblocks, 16), d.cw_max);
+    a.cw = lay.cw;
     a.cpitch = a.cw;
     const double dx = 2.0 * g.dmx / g.nx, dy = 2.0 * g.dmy / g.ny, dz = 2.0 * g.dmz / g.nz;
     a.dhx2i = 1.0 / (dx * dx);
@@ -784,28 +816,15 @@ hv_status poisson_plan(hv_ctx *c) {
     const size_t plane = (size_t)up(my, 8) * d.ps, zl = (size_t)2 * d.off * d.off, yl = (size_t)2 * d.py * d.py;
     d.shared_tab = my == mz ? 1 : 0;
     const size_t one = zl + (d.shared_tab ? 0 : yl);
-    // phase B's columns and their coefficients lie where the plane lies; the
-    // matrices follow, both directions where they fit, else over the columns
     const int ncol = my * d.wz;
-    const size_t col = (size_t)(mx + mx / 2 + 1);
-    int want = std::min(up((ncol + c->sm_count - 1) / c->sm_count, 16), 256);
-    while (want > 16 && col * want * sizeof(float) > limit) want -= 16;
-    if (col * want * sizeof(float) > limit) return HV_OK;
-    auto total = [&](int w) { return (std::max(plane, col * w) + 2 * one) * sizeof(float); };
-    d.keep_tab = total(want) <= limit ? 1 : 0;
-    // room for wider groups where it costs nothing: a solve that shares its
-    // launch has fewer blocks (16 warps eliminate 256 columns at once)
-    while (want < std::min(256, up(ncol, 16)) &&
-           (d.keep_tab ? total(want + 16) : col * (want + 16) * sizeof(float)) <= limit)
-        want += 16;
-    d.cw_max = want;
-    const size_t both = total(want) / sizeof(float);
-    const size_t words = d.keep_tab ? both : std::max(plane + one, col * want);
-    d.front = (int)(d.keep_tab ? both - 2 * one : plane);
-    d.smem = words * sizeof(float);
-    if (d.smem > limit) return HV_OK;
     // one block per x plane, more where they shorten phase B
     d.nblocks = std::min(c->sm_count, std::max(mx, (ncol + 31) / 32));
+    d.plane = (int)plane;
+    d.one = (int)one;
+    d.limit = limit;
+    const Layout lay = layout(d, g, d.nblocks);
+    if (!lay.ok) return HV_OK;
+    d.smem = lay.smem;
     const bool f64 = c->prec == HV_F64;
     for (const void *k : {f64 ? direct_kernel<double, false>(d.rt, d.nt) : direct_kernel<float, false>(d.rt, d.nt),
                           f64 ? nullptr : direct_kernel<float, true>(d.rt, d.nt)}) {
@@ -930,7 +949,7 @@ hv_status poisson_wave_build(SorWave &w, const std::vector<hv_ctx *> &cs, const 
         bfirst[i] = (int)binst.size();
         binst.insert(binst.end(), blocks[i], i);
         if (d.rt == 8) rt = 8;
-        smem = std::max(smem, d.smem);
+        smem = std::max(smem, layout(d, cs[i]->geom, blocks[i]).smem);
     }
     if (rt == 8)
         for (hv_ctx *c : cs) nt = std::max(nt, c->fused.direct.nt8);
