@@ -152,6 +152,8 @@ struct SmoothFast {
     size_t smem = 0;
     int per = 0;               // R = max(A, B, W): the kernel instantiation
     int xsplit = 1;            // x segments per column tile (the plan's choice)
+    float *discs = nullptr;    // disc sums of every plane (the two-launch form; null where the FFT form runs)
+    int *flags = nullptr;      // behind them: tile planes that hold density
     // FFT form (power-of-two axes up to 128): the circular convolution by the
     // stencil's spectrum, exact while no density lies within (A, B, W) of a
     // face, and made exact otherwise by subtracting the wrapped pairs

@@ -15,6 +15,7 @@
 #include <cstring>
 
 #include "hv_internal.h"
+#include "skyrme.cuh"
 
 namespace hv {
 
@@ -25,7 +26,8 @@ hv_status sor_fast_launch(hv_ctx *c, const T *rho, int *ctl, int *its_ring, int 
 hv_status sor_fast_clear_error(hv_ctx *c);
 hv_status smooth_fast_plan(hv_ctx *c);
 void smooth_fast_release(hv_ctx *c);
-hv_status smooth_fast_launch(hv_ctx *c, const float *rho_raw, float *rho, const int *wcount);
+hv_status smooth_fast_launch(hv_ctx *c, const float *rho_raw, float *rho, const int *wcount, float *U,
+                             bool *potential);
 bool smooth_fft_runs(const hv_ctx *c);
 
 namespace {
@@ -465,31 +467,6 @@ __global__ void k_close_kick(Geom g, int protons, int total, const T *__restrict
     fz[i] = az;
 }
 
-// Skyrme potential (include/physics.hpp:272-281, physics_formulas.hpp:70-77).
-// In float, t^gamma is CUDA's fast power intrinsic (exp2 of gamma log2 t on
-// the special-function units) and the divisions by rho0 are products by its
-// reciprocal: the accurate pow and two divisions made this kernel compute-
-// bound (58 % SM, 11 % DRAM in ncu).  The results move by float rounding;
-// the FP32 form's accuracy is checked on D(t).  The double form (the fused
-// FP64 path) keeps pow and the divisions.
-template <typename T>
-__device__ __forceinline__ void skyrme_node(T A, T B, T C, T gamma, T rp, T rn, T &up, T &un) {
-    if constexpr (sizeof(T) == 4) {
-        const float inv_rho0 = 1.0f / 0.16f;
-        const float t = (rp + rn) * inv_rho0;
-        const float base = A * t + B * __powf(t, gamma);
-        const float iso = 2.0f * C * ((rn - rp) * inv_rho0);
-        up = base - iso;
-        un = base + iso;
-    } else {
-        const T t = (rp + rn) / T(0.16);
-        const T base = A * t + B * pow(t, gamma);
-        const T iso = T(2.0) * C * ((rn - rp) / T(0.16));
-        up = base - iso;
-        un = base + iso;
-    }
-}
-
 // The smoothed density is also clamped at zero here, in place: the FFT
 // smoothing's wrap correction subtracts from the edge slabs after the
 // transform's own clamp, and may leave rounding-level negatives there (the
@@ -737,6 +714,30 @@ void prof_collect(hv_ctx *c) {
     cudaGetLastError();
 }
 
+// The smoothed density and the Skyrme potential of the raw density; wcount: the
+// wrap list's count (null: none kept).
+template <typename T>
+hv_status enqueue_density_and_potential(hv_ctx *c, const int *wcount) {
+    State<T> &s = st<T>(c);
+    const hv_skyrme &sk = c->params.skyrme;
+    bool potential = false;
+    {
+        ProfScope ps(c, HV_K_SMOOTH);
+        if (sizeof(T) == 4 && c->fused.smooth.ok)
+            HV_TRY(smooth_fast_launch(c, reinterpret_cast<const float *>(s.rho_raw), reinterpret_cast<float *>(s.rho),
+                                      wcount, reinterpret_cast<float *>(s.U), &potential));
+        else
+            HV_TRY(launch_smooth<T>(c, s.rho_raw, s.rho));
+    }
+    if (!potential) {
+        ProfScope ps(c, HV_K_SKYRME);
+        k_skyrme_fast<T><<<nblk(skyrme_threads<T>(c->geom.G), 256), 256, 0, c->stream>>>(
+            c->geom.G, T(sk.A), T(sk.B), T(sk.C), T(sk.gamma), s.rho, s.U);
+    }
+    HV_CUDA(cudaGetLastError());
+    return HV_OK;
+}
+
 // Enqueues one fused step on the context stream (graph-capturable).
 // A step in three parts, so that several contexts can interleave them (the
 // batched driver): A = particle step, smoothing, Skyrme; the SOR; C = forces
@@ -802,22 +803,7 @@ hv_status enqueue_phase_a(hv_ctx *c) {
         ProfScope ps(c, HV_K_PARTICLE);
         HV_TRY(launch_deposit_sorted<T>(c, s.x, s.y, s.z, s.rho_raw));
     }
-    {
-        ProfScope ps(c, HV_K_SMOOTH);
-        if (sizeof(T) == 4 && f.smooth.ok)
-            HV_TRY(smooth_fast_launch(c, reinterpret_cast<const float *>(s.rho_raw), reinterpret_cast<float *>(s.rho),
-                                      wcount));
-        else
-            HV_TRY(launch_smooth<T>(c, s.rho_raw, s.rho));
-    }
-    const hv_skyrme &sk = p.skyrme;
-    {
-        ProfScope ps(c, HV_K_SKYRME);
-        k_skyrme_fast<T><<<nblk(skyrme_threads<T>(g.G), 256), 256, 0, c->stream>>>(g.G, T(sk.A), T(sk.B), T(sk.C),
-                                                                                   T(sk.gamma), s.rho, s.U);
-    }
-    HV_CUDA(cudaGetLastError());
-    return HV_OK;
+    return enqueue_density_and_potential<T>(c, wcount);
 }
 
 template <typename T>
@@ -905,15 +891,7 @@ hv_status initial_typed(hv_ctx *c) {
         HV_TRY(launch_deposit_atomic<T>(c, s.x, s.y, s.z, s.rho_raw));
     // no wrap list here (the deposit is not the particle step's): density at
     // a face takes the direct form
-    if (sizeof(T) == 4 && f.smooth.ok)
-        HV_TRY(smooth_fast_launch(c, reinterpret_cast<const float *>(s.rho_raw), reinterpret_cast<float *>(s.rho),
-                                  nullptr));
-    else
-        HV_TRY(launch_smooth<T>(c, s.rho_raw, s.rho));
-    const hv_skyrme &sk = p.skyrme;
-    k_skyrme_fast<T><<<nblk(skyrme_threads<T>(g.G), 256), 256, 0, c->stream>>>(g.G, T(sk.A), T(sk.B), T(sk.C),
-                                                                               T(sk.gamma), s.rho, s.U);
-    HV_CUDA(cudaGetLastError());
+    HV_TRY(enqueue_density_and_potential<T>(c, nullptr));
     // the boundary counts as set only once the solve has succeeded: a solve
     // that gave up leaves phi64 unfinished and the plain phi without the
     // monopole boundary, so the next attempt must start from the boundary again

@@ -266,14 +266,16 @@ __global__ void __launch_bounds__(kRowThreads) k_smooth_rows(Geom g, RowTile rt,
         const int t0 = run[r0].w, t1 = run[r1 - 1].w + run[r1 - 1].z;
         __syncthreads();
         for (int e = tid; e < t1 - t0; e += kRowThreads) ws[e] = w[t0 + e];
+        int some = 0;
         for (int e = tid; e < nrows * width; e += kRowThreads) {
             const int rr = e / width, zz = e - rr * width, jy = y0 - ly + rr, jz = zz - lz;
             const bool in = jy >= 0 && jy < ny && jz >= 0 && jz < nz;
-            rows[(rr * 4 + (zz & 3)) * rt.pitch + (zz >> 2)] =
-                in ? s[((long long)jx * ny + jy) * nz + jz] : T(0);
+            const T v = in ? s[((long long)jx * ny + jy) * nz + jz] : T(0);
+            some |= v != T(0);
+            rows[(rr * 4 + (zz & 3)) * rt.pitch + (zz >> 2)] = v;
         }
-        __syncthreads();
-        if (!mine) continue;
+        // rows without density add w * 0 to every sum
+        if (!__syncthreads_or(some) || !mine) continue;
         for (int k = r0; k < r1; k++) {
             const int4 v = run[k];
             const T *row = rows + (r + ly + v.x) * 4 * rt.pitch + q;

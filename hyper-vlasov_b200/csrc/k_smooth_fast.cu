@@ -26,6 +26,7 @@
 #include <vector>
 
 #include "hv_internal.h"
+#include "skyrme.cuh"
 
 namespace hv {
 namespace {
@@ -67,6 +68,8 @@ struct MarchArgs {
     float gx[kMaxR + 1], gy[kMaxR + 1], gz[kMaxR + 1];
     int bm[kMaxR + 1];                        // largest |b| with a tap for each |a| (-1: none)
     int wt[(kMaxR + 1) * (kMaxR + 1)];        // w(|a|, |b|) at |a| (kMaxR + 1) + |b| (-1: none)
+    int zoff[(kMaxR + 1) * (kMaxR + 1)];      // place of Z_w(|a|, |b|) in the block's z-runs (0: none)
+    float gyt[(kMaxR + 1) * (kMaxR + 1)];     // g(b) where (a, b) has taps, else 0
     const float *src;                         // 2G
     float *dst;                               // 2G
     const int *edge;                          // [nx] edge flags of the FFT form: run only if one
@@ -202,6 +205,8 @@ __device__ void wrap_correct(const MarchArgs &a) {
 // Y_|a| = sum_|b|<=bm(a) g(b) Z_w(|a|,|b|)(y + b) and adds g(a) Y_|a| to the
 // outputs x = xi -+ a, held in a thread-private ring of 2A + 1 planes in shared
 // memory.  Output plane xo is complete after plane xo + A and is written then.
+// Planes that hold no density in the tile and its halo are passed over: most of
+// the box around a nucleus.
 // R >= A, B, W is the halo and the unrolled extent of the loops over |a|, |b|
 // and w; the tables hold -1 (no tap) and zero weights beyond A, B, W.
 template <int R>
@@ -245,15 +250,18 @@ __global__ void __launch_bounds__(kMThreads) k_smooth_march(const __grid_constan
     load_plane<R, kPer>(a, src, xfirst, Y0, K0, v);
     int slot = xfirst % ring;  // ring slot of plane xi
     for (int xi = xfirst; xi <= X1 - 1 + A; xi++, slot = slot + 1 == ring ? 0 : slot + 1) {
-        const bool have = xi <= xlast;
+        bool have = xi <= xlast;
+        int some = 0;
         if (have) {
 #pragma unroll
             for (int i = 0; i < kPer; i++) {
                 const int e = tid + i * kMThreads;
                 if (e < rows * cols) s_rho[e] = v[i];
+                some |= v[i] != 0.0f;
             }
         }
-        __syncthreads();
+        // a plane without density here adds nothing to any output
+        have = __syncthreads_or(some) && have;
         if (have) {
             // z-runs of every staged row
             for (int e = tid; e < rows * kMBK; e += kMThreads) {
@@ -273,21 +281,29 @@ __global__ void __launch_bounds__(kMThreads) k_smooth_march(const __grid_constan
         __syncthreads();
         if (have) {
             const float *zc = s_z + (j + R) * kMBK + k;  // this column's row, width 0
-            constexpr int zstride = rows * kMBK;
 #pragma unroll
             for (int aa = 0; aa <= R; aa++) {
-                const int bm = a.bm[aa];
-                if (bm < 0) continue;
                 const int xo1 = xi - aa, xo2 = xi + aa;
                 const bool h1 = xo1 >= X0 && xo1 < X1, h2 = aa > 0 && xo2 >= X0 && xo2 < X1;
                 if (!h1 && !h2) continue;
-                const int *wr = a.wt + aa * (kMaxR + 1);
-                float y0 = a.gy[0] * zc[wr[0] * zstride], y1 = 0.0f;
+                // pairs that the sphere of R + 1 nodes cannot hold are left out at
+                // compile time, those it could but the taps lack have weight zero:
+                // no branch stands between the loads
+                const int *zo = a.zoff + aa * (kMaxR + 1);
+                const float *gb = a.gyt + aa * (kMaxR + 1);
+                float p0[R + 1], p1[R + 1];
+#pragma unroll
+                for (int b = 0; b <= R; b++) {
+                    if (b > 0 && aa * aa + b * b >= (R + 1) * (R + 1)) continue;
+                    const float *pb = zc + zo[b];
+                    p0[b] = pb[b * kMBK];
+                    p1[b] = b > 0 ? pb[-b * kMBK] : 0.0f;
+                }
+                float y0 = gb[0] * p0[0], y1 = 0.0f;
 #pragma unroll
                 for (int b = 1; b <= R; b++) {
-                    if (b > bm) break;
-                    const float *pb = zc + wr[b] * zstride;
-                    const float t = a.gy[b] * (pb[b * kMBK] + pb[-b * kMBK]);
+                    if (aa * aa + b * b >= (R + 1) * (R + 1)) continue;
+                    const float t = gb[b] * (p0[b] + p1[b]);
                     if (b & 1) y0 += t;
                     else y1 += t;
                 }
@@ -305,6 +321,156 @@ __global__ void __launch_bounds__(kMThreads) k_smooth_march(const __grid_constan
             if (out_ok) a.dst[sp * a.G + ((long long)xo * a.ny + y) * a.nz + z] = *acc * a.term;
             *acc = 0.0f;
         }
+    }
+}
+
+// ---- the same sums in two launches -----------------------------------------
+// The march is a chain: a block's planes follow one another, ~2 us each, and a
+// segment of x pays for 2A planes it does not own.  Here every (tile, x plane,
+// species) is a block of its own.  k_smooth_discs forms the disc sums Y_|a| of
+// a plane's tile, as the march does, and stores them; k_smooth_planes adds
+// g(a) Y_|a|(x + a) over a per node, for both species, and writes the Skyrme
+// potential along with the density.  A tile plane without density (most of the
+// box around a nucleus) stores a flag only and is not read.
+// Smoothing and potential, per step: 64^3 (half-width 4) 31 + 7 us by the march
+// and its own kernel -> 19, 75 x 61 x 50 (half-width 6) 50 + 7 -> 26.  Bound by
+// the latency of one block's stages and of the sums' loads.
+struct DiscArgs {
+    float *y;     // [species][x][A + 1][ny nz]
+    int *flag;    // [species][x][tiles]: the tile plane holds density
+    float *rho, *U;
+    float cA, cB, cC, gamma;  // Skyrme coefficients
+};
+
+template <int R>
+__global__ void __launch_bounds__(kMThreads) k_smooth_discs(const __grid_constant__ MarchArgs a, const DiscArgs d) {
+    extern __shared__ __align__(16) float sm[];
+    constexpr int rows = kMBY + 2 * R, cols = kMBK + 2 * R;
+    constexpr int kPer = (rows * cols + kMThreads - 1) / kMThreads;
+    float *s_rho = sm, *s_z = s_rho + rows * cols;
+    const int tid = threadIdx.x, tz = (a.nz + kMBK - 1) / kMBK;
+    const int Y0 = (blockIdx.x / tz) * kMBY, K0 = (blockIdx.x % tz) * kMBK, xi = blockIdx.y, sp = blockIdx.z;
+    float v[kPer];
+    load_plane<R, kPer>(a, a.src + sp * a.G, xi, Y0, K0, v);
+    int some = 0;
+#pragma unroll
+    for (int i = 0; i < kPer; i++) {
+        const int e = tid + i * kMThreads;
+        if (e < rows * cols) s_rho[e] = v[i];
+        some |= v[i] != 0.0f;
+    }
+    some = __syncthreads_or(some);
+    if (tid == 0) d.flag[(sp * a.nx + xi) * gridDim.x + blockIdx.x] = some;
+    if (!some) return;
+    // z-runs of every staged row
+    for (int e = tid; e < rows * kMBK; e += kMThreads) {
+        const int r = e / kMBK, kk = e - r * kMBK;
+        const float *line = s_rho + r * cols + kk + R;
+        float zsum = a.gz[0] * line[0];
+        s_z[r * kMBK + kk] = zsum;
+#pragma unroll
+        for (int w = 1; w <= R; w++) {
+            zsum += a.gz[w] * (line[w] + line[-w]);
+            s_z[(w * rows + r) * kMBK + kk] = zsum;
+        }
+    }
+    __syncthreads();
+    const int j = tid / kMBK, k = tid % kMBK, y = Y0 + j, z = K0 + k;
+    const float *zc = s_z + (j + R) * kMBK + k;
+    const long long plane = (long long)a.ny * a.nz;
+    float *out = d.y + ((long long)(sp * a.nx + xi) * (a.A + 1)) * plane + (long long)y * a.nz + z;
+    const bool ok = y < a.ny && z < a.nz;
+#pragma unroll
+    for (int aa = 0; aa <= R; aa++) {
+        if (aa > a.A) break;
+        // as in k_smooth_march
+        const int *zo = a.zoff + aa * (kMaxR + 1);
+        const float *gb = a.gyt + aa * (kMaxR + 1);
+        float p0[R + 1], p1[R + 1];
+#pragma unroll
+        for (int b = 0; b <= R; b++) {
+            if (b > 0 && aa * aa + b * b >= (R + 1) * (R + 1)) continue;
+            const float *pb = zc + zo[b];
+            p0[b] = pb[b * kMBK];
+            p1[b] = b > 0 ? pb[-b * kMBK] : 0.0f;
+        }
+        float y0 = gb[0] * p0[0], y1 = 0.0f;
+#pragma unroll
+        for (int b = 1; b <= R; b++) {
+            if (aa * aa + b * b >= (R + 1) * (R + 1)) continue;
+            const float t = gb[b] * (p0[b] + p1[b]);
+            if (b & 1) y0 += t;
+            else y1 += t;
+        }
+        if (ok) out[aa * plane] = y0 + y1;
+    }
+}
+
+__global__ void __launch_bounds__(kMThreads) k_smooth_planes(const __grid_constant__ MarchArgs a, const DiscArgs d) {
+    const int tz = (a.nz + kMBK - 1) / kMBK;
+    const int y = (blockIdx.x / tz) * kMBY + threadIdx.x / kMBK, z = (blockIdx.x % tz) * kMBK + threadIdx.x % kMBK;
+    const int x = blockIdx.y;
+    const long long plane = (long long)a.ny * a.nz, yz = (long long)y * a.nz + z;
+    __shared__ int s_flag[2][2 * kMaxR + 9];  // read up to a batch past the end
+    const int n = 2 * a.A + 1;
+    for (int e = threadIdx.x; e < 2 * n; e += kMThreads) {
+        const int sp = e / n, xi = x + e - sp * n - a.A;
+        s_flag[sp][e - sp * n] = xi >= 0 && xi < a.nx ? d.flag[(sp * a.nx + xi) * gridDim.x + blockIdx.x] : 0;
+    }
+    __syncthreads();
+    if (y >= a.ny || z >= a.nz) return;
+    float r[2] = {0.0f, 0.0f};
+    const long long sstride = (long long)a.nx * (a.A + 1) * plane;
+    const float *src = d.y + (long long)(x - a.A) * (a.A + 1) * plane + yz;
+    // in the order the march adds the planes, the loads of nine ahead
+    constexpr int kU = 9;
+    for (int q0 = 0; q0 < n; q0 += kU) {
+        float v[2][kU];
+#pragma unroll
+        for (int u = 0; u < kU; u++) {
+            const int q = q0 + u, aa = abs(q - a.A);
+            const float *at = src + ((long long)q * (a.A + 1) + aa) * plane;
+            v[0][u] = q < n && s_flag[0][q] ? __ldg(at) : 0.0f;
+            v[1][u] = q < n && s_flag[1][q] ? __ldg(at + sstride) : 0.0f;
+        }
+#pragma unroll
+        for (int u = 0; u < kU; u++) {
+            const float g = q0 + u < n ? a.gx[abs(q0 + u - a.A)] : 0.0f;
+            r[0] += g * v[0][u];
+            r[1] += g * v[1][u];
+        }
+    }
+    r[0] *= a.term;
+    r[1] *= a.term;
+    d.rho[x * plane + yz] = r[0];
+    d.rho[a.G + x * plane + yz] = r[1];
+    if (d.U) {
+        float up, un;
+        skyrme_node<float>(d.cA, d.cB, d.cC, d.gamma, r[0], r[1], up, un);
+        d.U[x * plane + yz] = up;
+        d.U[a.G + x * plane + yz] = un;
+    }
+}
+
+const void *discs_kernel(int r) {
+    switch (r) {
+    case 1: return (const void *)k_smooth_discs<1>;
+    case 2: return (const void *)k_smooth_discs<2>;
+    case 3: return (const void *)k_smooth_discs<3>;
+    case 4: return (const void *)k_smooth_discs<4>;
+    case 5: return (const void *)k_smooth_discs<5>;
+    case 6: return (const void *)k_smooth_discs<6>;
+    case 7: return (const void *)k_smooth_discs<7>;
+    case 8: return (const void *)k_smooth_discs<8>;
+    case 9: return (const void *)k_smooth_discs<9>;
+    case 10: return (const void *)k_smooth_discs<10>;
+    case 11: return (const void *)k_smooth_discs<11>;
+    case 12: return (const void *)k_smooth_discs<12>;
+    case 13: return (const void *)k_smooth_discs<13>;
+    case 14: return (const void *)k_smooth_discs<14>;
+    case 15: return (const void *)k_smooth_discs<15>;
+    case 16: return (const void *)k_smooth_discs<16>;
+    default: return nullptr;
     }
 }
 
@@ -789,7 +955,7 @@ int log2_exact(int n) {
 
 // Builds the decomposition from the tap table, or leaves ok = false when the
 // table is not symmetric with contiguous z-runs.
-hv_status smooth_fast_plan(hv_ctx *c) {
+static hv_status plan_tables(hv_ctx *c) {
     SmoothFast &f = c->fused.smooth;
     f.ok = false;
     const TapTable &t = c->taps;
@@ -851,6 +1017,7 @@ hv_status smooth_fast_plan(hv_ctx *c) {
     f.per = R;
     f.smem = sizeof(float) * ((size_t)rows * cols + (size_t)(R + 1) * rows * kMBK + (size_t)(2 * A + 1) * kMThreads);
     HV_TRY(allow_max_dynamic_smem(march_kernel(R), c->device));
+    HV_TRY(allow_max_dynamic_smem(discs_kernel(R), c->device));
     // x segments: more blocks raise the warps per SM (the kernel is bound by
     // shared-memory latency) but each segment re-reads 2A halo planes; take
     // the split with the fewest (waves x planes per block), fewer blocks on
@@ -984,7 +1151,7 @@ hv_status smooth_fast_plan(hv_ctx *c) {
 
 void smooth_fast_release(hv_ctx *c) {
     SmoothFast &f = c->fused.smooth;
-    void *ptrs[] = {f.fwork, f.khat, f.tw, f.edge, f.occ, f.wlist};
+    void *ptrs[] = {f.fwork, f.khat, f.tw, f.edge, f.occ, f.wlist, f.discs};
     for (void *q : ptrs)
         if (q) cudaFree(q);
     f = SmoothFast();
@@ -997,7 +1164,22 @@ bool smooth_fft_runs(const hv_ctx *c) {
     return f.ok && f.fft && (c->fast.smooth_fft == 2 || (c->fast.smooth_fft == 1 && wide));
 }
 
-hv_status smooth_fast_launch(hv_ctx *c, const float *rho_raw, float *rho, const int *wcount) {
+hv_status smooth_fast_plan(hv_ctx *c) {
+    HV_TRY(plan_tables(c));
+    SmoothFast &f = c->fused.smooth;
+    if (!f.ok || smooth_fft_runs(c)) return HV_OK;
+    const Geom &g = c->geom;
+    const size_t sums = (size_t)(f.A + 1) * 2 * g.G;
+    const size_t tiles = (size_t)((g.ny + kMBY - 1) / kMBY) * ((g.nz + kMBK - 1) / kMBK);
+    HV_CUDA(cudaMalloc((void **)&f.discs, sizeof(float) * (sums + 2 * g.nx * tiles)));
+    f.flags = reinterpret_cast<int *>(f.discs + sums);
+    return HV_OK;
+}
+
+// U (null: not wanted): *potential is set when the launch wrote the Skyrme
+// potential there too.
+hv_status smooth_fast_launch(hv_ctx *c, const float *rho_raw, float *rho, const int *wcount, float *U,
+                             bool *potential) {
     const SmoothFast &f = c->fused.smooth;
     const Geom &g = c->geom;
     const hv_run_params &p = c->params;
@@ -1019,7 +1201,12 @@ hv_status smooth_fast_launch(hv_ctx *c, const float *rho_raw, float *rho, const 
         a.gz[i] = f.gz[i];
         a.bm[i] = f.bm[i];
     }
-    for (int i = 0; i < (kMaxR + 1) * (kMaxR + 1); i++) a.wt[i] = f.wt[i];
+    const int zstride = (kMBY + 2 * f.per) * kMBK;  // one width's rows of a block
+    for (int i = 0; i < (kMaxR + 1) * (kMaxR + 1); i++) {
+        a.wt[i] = f.wt[i];
+        a.zoff[i] = std::max(f.wt[i], 0) * zstride;
+        a.gyt[i] = f.wt[i] >= 0 ? f.gy[i % (kMaxR + 1)] : 0.0f;
+    }
     a.src = rho_raw;
     a.dst = rho;
     a.edge = nullptr;
@@ -1065,6 +1252,17 @@ hv_status smooth_fast_launch(hv_ctx *c, const float *rho_raw, float *rho, const 
         HV_CUDA(cudaGetLastError());
     }
     const int tz = (g.nz + kMBK - 1) / kMBK, ty = (g.ny + kMBY - 1) / kMBY;
+    if (!smooth_fft_runs(c) && f.discs) {
+        const hv_skyrme &sk = p.skyrme;
+        DiscArgs d{f.discs, f.flags, rho, U, (float)sk.A, (float)sk.B, (float)sk.C, (float)sk.gamma};
+        const size_t smem = f.smem - sizeof(float) * (size_t)(2 * f.A + 1) * kMThreads;  // without the ring
+        void *dargs[] = {&a, &d};
+        HV_CUDA(cudaLaunchKernel(discs_kernel(f.per), dim3(ty * tz, g.nx, 2), dim3(kMThreads), dargs, smem, c->stream));
+        k_smooth_planes<<<dim3(ty * tz, g.nx), kMThreads, 0, c->stream>>>(a, d);
+        HV_CUDA(cudaGetLastError());
+        if (potential) *potential = U != nullptr;
+        return HV_OK;
+    }
     void *args[] = {&a};
     HV_CUDA(cudaLaunchKernel(march_kernel(f.per), dim3(2 * f.xsplit * ty * tz), dim3(kMThreads), args, f.smem,
                              c->stream));
