@@ -40,15 +40,24 @@ struct hv_batch {
     int cap = -1;                         // SOR block cap of the current plan (0: own plans)
     cudaGraphExec_t graph = nullptr;
     int graph_len = 0;
+    cudaGraphExec_t tail_graph = nullptr; // a run's last, shorter chunk, once its length has come twice
+    int tail_len = 0;
     int chunk = 8;
+    char *staging = nullptr;              // pinned: rows, iteration rings, status and seed words of a run
+    size_t staging_bytes = 0;
 };
 
 namespace {
+
+constexpr int kWindow = 4096;  // steps whose rows wait in pinned memory (a multiple of the chunk)
 
 void drop_graph(hv_batch *b) {
     if (b->graph) cudaGraphExecDestroy(b->graph);
     b->graph = nullptr;
     b->graph_len = 0;
+    if (b->tail_graph) cudaGraphExecDestroy(b->tail_graph);
+    b->tail_graph = nullptr;
+    b->tail_len = 0;
 }
 
 // One step of every instance, on the batch stream with per-instance branches.
@@ -75,6 +84,20 @@ hv_status enqueue_batch_step(hv_batch *b) {
 hv_status enqueue_batch_steps(hv_batch *b, int k) {
     for (int s = 0; s < k; s++) HV_TRY(enqueue_batch_step(b));
     return HV_OK;
+}
+
+// k steps captured as a graph (null when that is not possible here).
+cudaGraphExec_t capture_steps(hv_batch *b, int k) {
+    cudaGraph_t gr = nullptr;
+    cudaGraphExec_t ex = nullptr;
+    if (cudaStreamBeginCapture(b->stream, cudaStreamCaptureModeThreadLocal) == cudaSuccess) {
+        const hv_status es = enqueue_batch_steps(b, k);
+        const cudaError_t ce = cudaStreamEndCapture(b->stream, &gr);
+        if (es != HV_OK || ce != cudaSuccess || !gr || cudaGraphInstantiate(&ex, gr, 0) != cudaSuccess) ex = nullptr;
+        if (gr) cudaGraphDestroy(gr);
+        cudaGetLastError();
+    }
+    return ex;
 }
 
 void release_waves(hv_batch *b) {
@@ -133,6 +156,7 @@ hv_status hv_batch_destroy(hv_batch *b) {
     if (b->stream) cudaStreamSynchronize(b->stream);
     drop_graph(b);
     release_waves(b);
+    if (b->staging) cudaFreeHost(b->staging);
     for (cudaStream_t s : b->streams)
         if (s) cudaStreamDestroy(s);
     for (cudaEvent_t e : b->ev_a)
@@ -236,42 +260,84 @@ hv_status hv_batch_run(hv_batch *b, int n_steps, hv_observables *obs) {
     if (n_steps == 0) return HV_OK;
     HV_CUDA(cudaSetDevice(b->device));
     const int n = (int)b->ctx.size();
-    std::vector<int> exc(n, -1);
-    for (int i = 0; i < n; i++) HV_TRY(fused_batch_begin(b->ctx[i], n_steps, &exc[i]));
-    int done = 0;
-    while (done < n_steps) {
+    // pinned room for what a window of steps reads back, so that the host waits
+    // once a window: per instance the rows, every chunk's iteration ring, two words
+    const int window = std::min(n_steps, kWindow);
+    const int ring = fused_batch_ring(), chunks = (window + b->chunk - 1) / b->chunk;
+    const size_t rows_bytes = sizeof(double) * 8 * (size_t)window, its_bytes = sizeof(int) * (size_t)ring * chunks;
+    const size_t per = rows_bytes + its_bytes + 64;
+    if (b->staging_bytes < per * n) {
+        if (b->staging) cudaFreeHost(b->staging);
+        b->staging = nullptr;
+        b->staging_bytes = 0;
+        HV_CUDA(cudaMallocHost((void **)&b->staging, per * n));
+        b->staging_bytes = per * n;
+    }
+    auto rows = [&](int i, int step) { return reinterpret_cast<double *>(b->staging + per * i) + (size_t)8 * step; };
+    auto its = [&](int i, int q) { return reinterpret_cast<int *>(b->staging + per * i + rows_bytes) + (size_t)ring * q; };
+    auto words = [&](int i) { return reinterpret_cast<int *>(b->staging + per * i + rows_bytes + its_bytes); };
+    std::vector<int> exc(n, -1), start(n);
+    for (int i = 0; i < n; i++) {
+        hv_ctx *c = b->ctx[i];
+        start[i] = c->step_index;
+        HV_TRY(fused_batch_begin(c, n_steps, &exc[i]));
+        HV_CUDA(cudaEventRecord(b->ev_a[i], c->stream));
+        HV_CUDA(cudaStreamWaitEvent(b->stream, b->ev_a[i], 0));
+    }
+    int from = 0;  // first step of the window
+    for (int done = 0, q = 0; done < n_steps;) {
         const int k = std::min(b->chunk, n_steps - done);
-        bool launched = false;
+        cudaGraphExec_t graph = nullptr;
         if (k == b->chunk) {
-            if (!b->graph || b->graph_len != k) {
-                drop_graph(b);
-                cudaGraph_t gr = nullptr;
-                if (cudaStreamBeginCapture(b->stream, cudaStreamCaptureModeThreadLocal) == cudaSuccess) {
-                    hv_status es = enqueue_batch_steps(b, k);
-                    cudaError_t ce = cudaStreamEndCapture(b->stream, &gr);
-                    if (es == HV_OK && ce == cudaSuccess && gr &&
-                        cudaGraphInstantiate(&b->graph, gr, 0) == cudaSuccess)
-                        b->graph_len = k;
-                    else
-                        b->graph = nullptr;
-                    if (gr) cudaGraphDestroy(gr);
-                    cudaGetLastError();
-                }
-            }
-            if (b->graph) {
-                HV_CUDA(cudaGraphLaunch(b->graph, b->stream));
-                launched = true;
-            }
+            if (!b->graph) b->graph = capture_steps(b, k);
+            graph = b->graph;
+        } else if (b->tail_len == k) {
+            if (!b->tail_graph) b->tail_graph = capture_steps(b, k);
+            graph = b->tail_graph;
+        } else {
+            // launched directly the first time: a length that does not come
+            // again is not worth a capture
+            if (b->tail_graph) cudaGraphExecDestroy(b->tail_graph);
+            b->tail_graph = nullptr;
+            b->tail_len = k;
         }
-        if (!launched) HV_TRY(enqueue_batch_steps(b, k));
+        if (graph) HV_CUDA(cudaGraphLaunch(graph, b->stream));
+        else HV_TRY(enqueue_batch_steps(b, k));
+        // the instances' rows side by side; the next chunk starts after them
+        HV_CUDA(cudaEventRecord(b->ev_fork_a, b->stream));
         for (int i = 0; i < n; i++) {
-            hv_ctx *c = b->ctx[i];
-            HV_TRY(fused_batch_rows(c, b->stream, c->step_index + done, k,
-                                    obs ? obs + (size_t)i * n_steps + done : nullptr));
+            HV_CUDA(cudaStreamWaitEvent(b->streams[i], b->ev_fork_a, 0));
+            HV_TRY(fused_batch_rows(b->ctx[i], b->streams[i], start[i] + done, k, rows(i, done - from), its(i, q)));
+            HV_CUDA(cudaEventRecord(b->ev_a[i], b->streams[i]));
+            HV_CUDA(cudaStreamWaitEvent(b->stream, b->ev_a[i], 0));
         }
         done += k;
+        q++;
+        if (done < n_steps && done - from < window) continue;
+        // a solve that gave up leaves every instance's run where it was
+        for (int i = 0; i < n; i++)
+            HV_CUDA(cudaMemcpyAsync(words(i), b->ctx[i]->fused.sor.status, sizeof(int), cudaMemcpyDeviceToHost,
+                                    b->stream));
+        HV_CUDA(cudaStreamSynchronize(b->stream));
+        hv_status failed = HV_OK;
+        for (int i = 0; i < n; i++) {
+            const hv_status st = fused_batch_status(b->ctx[i], words(i)[0]);
+            if (st != HV_OK) failed = st;
+        }
+        HV_TRY(failed);
+        if (obs)
+            for (int i = 0; i < n; i++)
+                for (int s = from, c = 0; s < done; s += b->chunk, c++)
+                    fused_batch_decode(b->ctx[i], start[i] + s, std::min(b->chunk, done - s), rows(i, s - from),
+                                       its(i, c), obs + (size_t)i * n_steps + s);
+        from = done;
+        q = 0;
     }
-    for (int i = 0; i < n; i++) HV_TRY(fused_batch_end(b->ctx[i], n_steps, exc[i]));
+    for (int i = 0; i < n; i++) HV_TRY(fused_batch_end(b->ctx[i], n_steps, exc[i], words(i) + 1));
+    for (int i = 0; i < n; i++) {
+        HV_CUDA(cudaStreamSynchronize(b->ctx[i]->stream));
+        if (words(i)[1] > 0) b->ctx[i]->fused.m_hint = words(i)[1];
+    }
     return HV_OK;
 }
 

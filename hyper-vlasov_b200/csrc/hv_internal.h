@@ -335,8 +335,14 @@ hv_status fused_batch_ready(hv_ctx *c);
 hv_status fused_batch_begin(hv_ctx *c, int n_steps, int *exc);
 hv_status fused_batch_phase_a(hv_ctx *c, cudaStream_t s);
 hv_status fused_batch_phase_c(hv_ctx *c, cudaStream_t s);
-hv_status fused_batch_rows(hv_ctx *c, cudaStream_t s, int s0, int k, hv_observables *obs);
-hv_status fused_batch_end(hv_ctx *c, int n_steps, int exc);
+// the observable rows of k steps from s0 into pinned memory (rows: 8 doubles a
+// step, its: fused_batch_ring ints), stream-ordered; decoded once copied
+int fused_batch_ring();
+hv_status fused_batch_rows(hv_ctx *c, cudaStream_t s, int s0, int k, double *rows, int *its);
+void fused_batch_decode(hv_ctx *c, int s0, int k, const double *rows, const int *its, hv_observables *obs);
+hv_status fused_batch_status(hv_ctx *c, int status0);
+// a run's end, enqueued on the context's stream; *mh (pinned): the solver's seed
+hv_status fused_batch_end(hv_ctx *c, int n_steps, int exc, int *mh);
 void fused_batch_sor_inputs(hv_ctx *c, const float **rho, int **ctl, int **its_ring, int *ring);
 void adjoint_release(hv_ctx *c);
 // fused FP64 steps one at a time for the adjoint (k_fused.cu): the control

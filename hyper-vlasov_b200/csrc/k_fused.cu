@@ -947,7 +947,7 @@ hv_status enqueue_steps(hv_ctx *c, int n) {
 // Before n_steps fused steps: the fused state brought up to date with the plain
 // buffers and the control words set; returns the excitation step (or -1).
 template <typename T>
-hv_status run_begin(hv_ctx *c, int n_steps, int *exc_out) {
+hv_status run_begin(hv_ctx *c, int n_steps, int *exc_out, bool wait = true) {
     State<T> &s = st<T>(c);
     Fused &f = c->fused;
     const Geom &g = c->geom;
@@ -979,8 +979,9 @@ hv_status run_begin(hv_ctx *c, int n_steps, int *exc_out) {
     int h_ctl[5] = {c->step_index, f.m_hint, 0, exc, 0};
     HV_TRY(sor_fast_clear_error(c));
     HV_CUDA(cudaMemcpyAsync(ctl + CTL_STEP, &h_ctl[0], sizeof(int), cudaMemcpyHostToDevice, c->stream));
+    // (pageable words: the copies are staged before the calls return)
     HV_CUDA(cudaMemcpyAsync(ctl + CTL_EXCITE, &h_ctl[3], sizeof(int) * 2, cudaMemcpyHostToDevice, c->stream));
-    HV_CUDA(cudaStreamSynchronize(c->stream));
+    if (wait) HV_CUDA(cudaStreamSynchronize(c->stream));
     *exc_out = exc;
     return HV_OK;
 }
@@ -1165,8 +1166,9 @@ hv_status run_typed(hv_ctx *c, int n_steps, hv_observables *obs) {
 
 // After a run of n_steps: step counter, excitation flag, the closing kick/2
 // and the plain-path view of the fields.
+// *mh receives the solver's first-cycle seed (stream-ordered).
 template <typename T>
-hv_status run_end(hv_ctx *c, int n_steps, int exc) {
+hv_status run_end_enqueue(hv_ctx *c, int n_steps, int exc, int *mh) {
     Fused &f = c->fused;
     const Geom &g = c->geom;
     int *ctl = ctl_of(c);
@@ -1190,10 +1192,16 @@ hv_status run_end(hv_ctx *c, int n_steps, int exc) {
     k_unpack_f4<T><<<nblk(2 * g.G, 256), 256, 0, c->stream>>>(2 * g.G, reinterpret_cast<const T *>(f.F4), S.Fx, S.Fy, S.Fz);
     k_merge_out<T><<<nblk(g.G, 256), 256, 0, c->stream>>>(g.G, f.phi64, S.U, S.phi);
     HV_CUDA(cudaGetLastError());
+    HV_CUDA(cudaMemcpyAsync(mh, ctl + CTL_MHINT, sizeof(int), cudaMemcpyDeviceToHost, c->stream));
+    return HV_OK;
+}
+
+template <typename T>
+hv_status run_end(hv_ctx *c, int n_steps, int exc) {
     int mh = 0;
-    HV_CUDA(cudaMemcpyAsync(&mh, ctl + CTL_MHINT, sizeof(int), cudaMemcpyDeviceToHost, c->stream));
+    HV_TRY(run_end_enqueue<T>(c, n_steps, exc, &mh));
     HV_CUDA(cudaStreamSynchronize(c->stream));
-    f.m_hint = mh > 0 ? mh : f.m_hint;
+    if (mh > 0) c->fused.m_hint = mh;
     return HV_OK;
 }
 
@@ -1371,7 +1379,7 @@ hv_status fused_batch_ready(hv_ctx *c) {
     if (st != HV_OK) fused_release(c);
     return st;
 }
-hv_status fused_batch_begin(hv_ctx *c, int n_steps, int *exc) { return run_begin<float>(c, n_steps, exc); }
+hv_status fused_batch_begin(hv_ctx *c, int n_steps, int *exc) { return run_begin<float>(c, n_steps, exc, false); }
 hv_status fused_batch_phase_a(hv_ctx *c, cudaStream_t s) {
     StreamSwap sw(c, s);
     return enqueue_phase_a<float>(c);
@@ -1380,11 +1388,16 @@ hv_status fused_batch_phase_c(hv_ctx *c, cudaStream_t s) {
     StreamSwap sw(c, s);
     return enqueue_phase_c<float>(c);
 }
-hv_status fused_batch_rows(hv_ctx *c, cudaStream_t s, int s0, int k, hv_observables *obs) {
+int fused_batch_ring() { return kRing; }
+hv_status fused_batch_rows(hv_ctx *c, cudaStream_t s, int s0, int k, double *rows, int *its) {
     StreamSwap sw(c, s);
-    return run_rows<float>(c, s0, k, obs);
+    return rows_enqueue(c, s0, k, rows, its);
 }
-hv_status fused_batch_end(hv_ctx *c, int n_steps, int exc) { return run_end<float>(c, n_steps, exc); }
+void fused_batch_decode(hv_ctx *c, int s0, int k, const double *rows, const int *its, hv_observables *obs) {
+    rows_decode<float>(c, s0, k, rows, its, obs);
+}
+hv_status fused_batch_status(hv_ctx *c, int status0) { return rows_status(c, status0); }
+hv_status fused_batch_end(hv_ctx *c, int n_steps, int exc, int *mh) { return run_end_enqueue<float>(c, n_steps, exc, mh); }
 void fused_batch_sor_inputs(hv_ctx *c, const float **rho, int **ctl, int **its_ring, int *ring) {
     *rho = c->d32.rho;
     *ctl = ctl_of(c);
