@@ -479,7 +479,7 @@ __device__ __forceinline__ bool clamp4(float4 &v) {
 }
 
 template <typename T>
-__global__ void k_skyrme_fast(long long G, T A, T B, T C, T gamma, T *rho, T *U) {
+__global__ void k_skyrme_fast(long long G, double A, double B, double C, double gamma, T *rho, T *U) {
     long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if constexpr (sizeof(T) == 4) {
         // four nodes per thread with 16-byte loads and stores (G a multiple
@@ -732,7 +732,7 @@ hv_status enqueue_density_and_potential(hv_ctx *c, const int *wcount) {
     if (!potential) {
         ProfScope ps(c, HV_K_SKYRME);
         k_skyrme_fast<T><<<nblk(skyrme_threads<T>(c->geom.G), 256), 256, 0, c->stream>>>(
-            c->geom.G, T(sk.A), T(sk.B), T(sk.C), T(sk.gamma), s.rho, s.U);
+            c->geom.G, sk.A, sk.B, sk.C, sk.gamma, s.rho, s.U);
     }
     HV_CUDA(cudaGetLastError());
     return HV_OK;

@@ -339,7 +339,7 @@ struct DiscArgs {
     float *y;     // [species][x][A + 1][ny nz]
     int *flag;    // [species][x][tiles]: the tile plane holds density
     float *rho, *U;
-    float cA, cB, cC, gamma;  // Skyrme coefficients
+    double cA, cB, cC, gamma;  // Skyrme coefficients
 };
 
 template <int R>
@@ -1254,7 +1254,7 @@ hv_status smooth_fast_launch(hv_ctx *c, const float *rho_raw, float *rho, const 
     const int tz = (g.nz + kMBK - 1) / kMBK, ty = (g.ny + kMBY - 1) / kMBY;
     if (!smooth_fft_runs(c) && f.discs) {
         const hv_skyrme &sk = p.skyrme;
-        DiscArgs d{f.discs, f.flags, rho, U, (float)sk.A, (float)sk.B, (float)sk.C, (float)sk.gamma};
+        DiscArgs d{f.discs, f.flags, rho, U, sk.A, sk.B, sk.C, sk.gamma};
         const size_t smem = f.smem - sizeof(float) * (size_t)(2 * f.A + 1) * kMThreads;  // without the ring
         void *dargs[] = {&a, &d};
         HV_CUDA(cudaLaunchKernel(discs_kernel(f.per), dim3(ty * tz, g.nx, 2), dim3(kMThreads), dargs, smem, c->stream));
