@@ -84,19 +84,20 @@ __global__ void k_cell_keys(Geom g, int protons, int total, const T *__restrict_
     vals[i] = i;
 }
 
-// A sorted particle: its fractional offsets in the cell, its index, and
-// whether it is the last of its cell (the sign of the index word).
+// A sorted particle: its fractional offsets in the cell, and the index of the
+// next particle of its cell (kNoParticle: it is the last).
+constexpr int kNoParticle = 0x7fffffff;
 template <typename T>
 struct Entry;
 template <>
 struct __align__(16) Entry<float> {
     float d[3];
-    int id;
+    int next;
 };
 template <>
 struct __align__(16) Entry<double> {
     double d[3];
-    int id, pad;
+    int next, pad;
 };
 
 // Entries in sorted order, and every occupied cell's first one (cell_start is
@@ -117,7 +118,7 @@ __global__ void k_deposit_entries(Geom g, int total, const T *__restrict__ x, co
     e.d[0] = cx - (int)cx;
     e.d[1] = cy - (int)cy;
     e.d[2] = cz - (int)cz;
-    e.id = s + 1 == total || keys[s + 1] != key ? i | (int)0x80000000 : i;
+    e.next = s + 1 == total || keys[s + 1] != key ? kNoParticle : sorted_idx[s + 1];
     ent[s] = e;
     if (s == 0 || keys[s - 1] != key) cell_start[key] = s;
 }
@@ -125,22 +126,24 @@ __global__ void k_deposit_entries(Geom g, int total, const T *__restrict__ x, co
 // One thread per node: merges the particle lists of the (up to) eight cells
 // that touch the node, in increasing particle index, and sums their CIC
 // weights sequentially from 0 -- the order of a single-threaded run of the
-// reference's deposit loop (include/tools.hpp:46-95).  The list with the
-// smallest head is followed while it stays below every other head (slots
-// sorted by cell make that most of a list); the eight heads stay in registers.
+// reference's deposit loop (include/tools.hpp:46-95).  One entry a turn for
+// every lane, whatever list it comes from: a loop that follows one list while
+// it stays the smallest takes fewer turns per node, but its lanes leave it at
+// different turns and wait for each other.  The heads are in registers, the
+// places in shared memory ([list][thread]: no bank conflicts), and an entry
+// brings its successor's index, so that a turn waits for memory once.
 // Block: nodes along z; grid: (z blocks, y, x of both species).  Bound by the
-// latency of a node's chain of ~160 entries (208Pb 2.08 M, 128^3: 232 us with
-// freshly sorted slots; 547 with the heads in local memory and the positions
-// fetched per particle).
+// instructions of a turn (~60) times a node's ~100 entries.
 template <typename T>
-__global__ void k_deposit_merge(Geom g, const Entry<T> *__restrict__ ent, const int *__restrict__ cell_start, T *rho) {
-    const int iz = blockIdx.x * blockDim.x + threadIdx.x, iy = blockIdx.y;
+__global__ void __launch_bounds__(128) k_deposit_merge(Geom g, const Entry<T> *__restrict__ ent,
+                                                       const int *__restrict__ cell_start,
+                                                       const int *__restrict__ sorted_idx, T *rho) {
+    __shared__ int s_pos[8][128];
+    const int iz = blockIdx.x * blockDim.x + threadIdx.x, iy = blockIdx.y, tid = threadIdx.x;
     const int sp = blockIdx.z >= (unsigned)g.nx ? 1 : 0, ix = blockIdx.z - sp * g.nx;
     const long long s_off = sp ? g.G : 0;
-    const int lane = threadIdx.x & 31;
-    constexpr int kNone = 0x7fffffff;
-    int pos[8], head[8];
-    bool any = false;
+    const int lane = tid & 31;
+    int head[8];
 #pragma unroll
     for (int r = 0; r < 4; r++) {
         const int dx = r >> 1, dy = r & 1, cx = ix - dx, cy = iy - dy;
@@ -152,54 +155,35 @@ __global__ void k_deposit_merge(Geom g, const Entry<T> *__restrict__ ent, const 
         }
         const int up = __shfl_up_sync(0xffffffffu, here, 1);
         if (lane) below = up;
-        pos[2 * r] = here;
-        pos[2 * r + 1] = below;
-        any = any || here >= 0 || below >= 0;
+        s_pos[2 * r][tid] = here;
+        s_pos[2 * r + 1][tid] = below;
+        head[2 * r] = here >= 0 ? __ldg(sorted_idx + here) : kNoParticle;
+        head[2 * r + 1] = below >= 0 ? __ldg(sorted_idx + below) : kNoParticle;
     }
     if (iz >= g.nz) return;
-    const long long node = s_off + ((long long)ix * g.ny + iy) * g.nz + iz;
     T acc = T(0.0);
-    if (any) {
+    while (true) {
+        const int m = min(min(min(head[0], head[1]), min(head[2], head[3])),
+                          min(min(head[4], head[5]), min(head[6], head[7])));
+        if (m == kNoParticle) break;
+        // a particle is in one list only
+        int best = 0;
 #pragma unroll
-        for (int l = 0; l < 8; l++) head[l] = pos[l] >= 0 ? ent[pos[l]].id & kNone : kNone;
-        while (true) {
-            int m = kNone, lim = kNone, best = 0, p = 0;
+        for (int l = 1; l < 8; l++)
+            if (head[l] == m) best = l;
+        const int p = s_pos[best][tid];
+        const Entry<T> e = ent[p];
+        s_pos[best][tid] = p + 1;
 #pragma unroll
-            for (int l = 0; l < 8; l++) {
-                if (head[l] < m) {
-                    lim = m;
-                    m = head[l];
-                    best = l;
-                    p = pos[l];
-                } else if (head[l] < lim) {
-                    lim = head[l];
-                }
-            }
-            if (m == kNone) break;
-            Entry<T> e = ent[p];
-            int next;
-            while (true) {
-                // node = cell + corner; corner bit 1 means the "1" side (weight d);
-                // the entry after the array's last is allocated
-                const Entry<T> n = ent[p + 1];
-                const T wx = (best & 4) ? e.d[0] : T(1.0) - e.d[0];
-                const T wy = (best & 2) ? e.d[1] : T(1.0) - e.d[1];
-                const T wz = (best & 1) ? e.d[2] : T(1.0) - e.d[2];
-                acc += wx * wy * wz;
-                p++;
-                next = e.id < 0 ? kNone : n.id & kNone;
-                if (next >= lim) break;
-                e = n;
-            }
-#pragma unroll
-            for (int l = 0; l < 8; l++)
-                if (l == best) {
-                    head[l] = next;
-                    pos[l] = p;
-                }
-        }
+        for (int l = 0; l < 8; l++)
+            if (head[l] == m) head[l] = e.next;
+        // node = cell + corner; corner bit 1 means the "1" side (weight d)
+        const T wx = (best & 4) ? e.d[0] : T(1.0) - e.d[0];
+        const T wy = (best & 2) ? e.d[1] : T(1.0) - e.d[1];
+        const T wz = (best & 1) ? e.d[2] : T(1.0) - e.d[2];
+        acc += wx * wy * wz;
     }
-    rho[node] = acc;
+    rho[s_off + ((long long)ix * g.ny + iy) * g.nz + iz] = acc;
 }
 
 // ---- smoothing (include/physics.hpp:202-234) -----------------------------
@@ -900,14 +884,15 @@ hv_status launch_deposit_sorted(hv_ctx *c, const T *x, const T *y, const T *z, T
     HV_CUDA(cudaGetLastError());
     const Geom &g = c->geom;
     const int zt = std::min(128, (g.nz + 31) / 32 * 32);
-    k_deposit_merge<T><<<dim3((g.nz + zt - 1) / zt, g.ny, 2 * g.nx), zt, 0, c->stream>>>(g, ent, s.cell_start, rho);
+    k_deposit_merge<T><<<dim3((g.nz + zt - 1) / zt, g.ny, 2 * g.nx), zt, 0, c->stream>>>(g, ent, s.cell_start, s.vals_alt,
+                                                                                        rho);
     HV_CUDA(cudaGetLastError());
     return HV_OK;
 }
 
-// Bytes of the sorted deposit's entries (one more is read, not used).
+// Bytes of the sorted deposit's entries.
 size_t sorted_deposit_entry_bytes(int total, hv_precision prec) {
-    return ((size_t)total + 1) * (prec == HV_F64 ? sizeof(Entry<double>) : sizeof(Entry<float>));
+    return (size_t)total * (prec == HV_F64 ? sizeof(Entry<double>) : sizeof(Entry<float>));
 }
 
 // Bytes of CUB temporary storage for a sort of `total` keys.
