@@ -131,10 +131,18 @@ __global__ void k_deposit_entries(Geom g, int total, const T *__restrict__ x, co
 // it stays the smallest takes fewer turns per node, but its lanes leave it at
 // different turns and wait for each other.  The heads are in registers, the
 // places in shared memory ([list][thread]: no bank conflicts), and an entry
-// brings its successor's index, so that a turn waits for memory once.
+// brings its successor's index, so that a turn waits for memory once.  A head
+// is a key, index times eight plus list, and the keys are kept sorted: the
+// popped one's successor moves to its place by minima and maxima alone.
+// K: 32 bits where every index fits (kMaxIndex32), else 64.
 // Block: nodes along z; grid: (z blocks, y, x of both species).  Bound by the
-// instructions of a turn (~60) times a node's ~100 entries.
-template <typename T>
+// instructions of a turn times a node's ~100 entries.  208Pb 2.08 M / 128^3 in
+// float: 102 us; 133 with the smallest of eight unsorted heads searched each
+// turn, 232 following one list while it is the smallest; blocks of 64 or 32
+// threads 8 or 20 % slower.  40Ca, 4,000 in double: 24-34 us, latency.
+constexpr int kMaxIndex32 = (1 << 29) - 2;  // its key is below kNoParticle's, 0xfffffff8
+
+template <typename T, typename K>
 __global__ void __launch_bounds__(128) k_deposit_merge(Geom g, const Entry<T> *__restrict__ ent,
                                                        const int *__restrict__ cell_start,
                                                        const int *__restrict__ sorted_idx, T *rho) {
@@ -143,7 +151,20 @@ __global__ void __launch_bounds__(128) k_deposit_merge(Geom g, const Entry<T> *_
     const int sp = blockIdx.z >= (unsigned)g.nx ? 1 : 0, ix = blockIdx.z - sp * g.nx;
     const long long s_off = sp ? g.G : 0;
     const int lane = tid & 31;
-    int head[8];
+    constexpr K none = (K)kNoParticle << 3;
+    K head[8];  // ascending
+#pragma unroll
+    for (int l = 0; l < 8; l++) head[l] = none | 7;
+    // x takes its place among head[1..7], and head[0] is dropped
+    auto replace_first = [&](K x) {
+#pragma unroll
+        for (int l = 0; l < 7; l++) {
+            head[l] = min(head[l + 1], x);
+            x = max(head[l + 1], x);
+        }
+        head[7] = x;
+    };
+    int first[8];
 #pragma unroll
     for (int r = 0; r < 4; r++) {
         const int dx = r >> 1, dy = r & 1, cx = ix - dx, cy = iy - dy;
@@ -155,28 +176,37 @@ __global__ void __launch_bounds__(128) k_deposit_merge(Geom g, const Entry<T> *_
         }
         const int up = __shfl_up_sync(0xffffffffu, here, 1);
         if (lane) below = up;
-        s_pos[2 * r][tid] = here;
-        s_pos[2 * r + 1][tid] = below;
-        head[2 * r] = here >= 0 ? __ldg(sorted_idx + here) : kNoParticle;
-        head[2 * r + 1] = below >= 0 ? __ldg(sorted_idx + below) : kNoParticle;
+        first[2 * r] = here;
+        first[2 * r + 1] = below;
     }
     if (iz >= g.nz) return;
-    T acc = T(0.0);
-    while (true) {
-        const int m = min(min(min(head[0], head[1]), min(head[2], head[3])),
-                          min(min(head[4], head[5]), min(head[6], head[7])));
-        if (m == kNoParticle) break;
-        // a particle is in one list only
-        int best = 0;
+    int lists = 0;
 #pragma unroll
-        for (int l = 1; l < 8; l++)
-            if (head[l] == m) best = l;
+    for (int l = 0; l < 8; l++) {
+        s_pos[l][tid] = first[l];
+        first[l] = first[l] >= 0 ? __ldg(sorted_idx + first[l]) : kNoParticle;
+        lists += first[l] != kNoParticle;
+    }
+    if (lists) {
+        // what leaves at the end is always `none`
+#pragma unroll
+        for (int l = 0; l < 8; l++) {
+            K x = (K)first[l] << 3 | l;
+#pragma unroll
+            for (int q = 0; q < 8; q++) {
+                const K lo = min(head[q], x);
+                x = max(head[q], x);
+                head[q] = lo;
+            }
+        }
+    }
+    T acc = T(0.0);
+    while (head[0] < none) {
+        const int best = (int)(head[0] & 7);
         const int p = s_pos[best][tid];
         const Entry<T> e = ent[p];
         s_pos[best][tid] = p + 1;
-#pragma unroll
-        for (int l = 0; l < 8; l++)
-            if (head[l] == m) head[l] = e.next;
+        replace_first((K)e.next << 3 | best);
         // node = cell + corner; corner bit 1 means the "1" side (weight d)
         const T wx = (best & 4) ? e.d[0] : T(1.0) - e.d[0];
         const T wy = (best & 2) ? e.d[1] : T(1.0) - e.d[1];
@@ -884,8 +914,11 @@ hv_status launch_deposit_sorted(hv_ctx *c, const T *x, const T *y, const T *z, T
     HV_CUDA(cudaGetLastError());
     const Geom &g = c->geom;
     const int zt = std::min(128, (g.nz + 31) / 32 * 32);
-    k_deposit_merge<T><<<dim3((g.nz + zt - 1) / zt, g.ny, 2 * g.nx), zt, 0, c->stream>>>(g, ent, s.cell_start, s.vals_alt,
-                                                                                        rho);
+    const dim3 grid((g.nz + zt - 1) / zt, g.ny, 2 * g.nx);
+    if (c->total <= kMaxIndex32)
+        k_deposit_merge<T, unsigned><<<grid, zt, 0, c->stream>>>(g, ent, s.cell_start, s.vals_alt, rho);
+    else
+        k_deposit_merge<T, unsigned long long><<<grid, zt, 0, c->stream>>>(g, ent, s.cell_start, s.vals_alt, rho);
     HV_CUDA(cudaGetLastError());
     return HV_OK;
 }
