@@ -852,7 +852,12 @@ hv_status poisson_plan(hv_ctx *c) {
     const size_t nw = (size_t)mx * ncol, np = 4 * (size_t)c->sm_count;
     const size_t at_work = up((int)all.size(), 64), at_delta = at_work + (nw + 63) / 64 * 64;
     const size_t at_part = at_delta + ((size_t)g.G + 63) / 64 * 64, words_all = at_part + np + 64;
-    HV_CUDA(cudaMalloc((void **)&d.tables, words_all * sizeof(float)));
+    // where that does not fit in memory, the sweeps run as they would without it
+    if (cudaMalloc((void **)&d.tables, words_all * sizeof(float)) != cudaSuccess) {
+        cudaGetLastError();
+        d.tables = nullptr;
+        return HV_OK;
+    }
     d.work = d.tables + at_work;
     d.delta = d.tables + at_delta;
     d.partials = reinterpret_cast<double *>(d.tables + at_part);

@@ -1171,7 +1171,12 @@ hv_status smooth_fast_plan(hv_ctx *c) {
     const Geom &g = c->geom;
     const size_t sums = (size_t)(f.A + 1) * 2 * g.G;
     const size_t tiles = (size_t)((g.ny + kMBY - 1) / kMBY) * ((g.nz + kMBK - 1) / kMBK);
-    HV_CUDA(cudaMalloc((void **)&f.discs, sizeof(float) * (sums + 2 * g.nx * tiles)));
+    // where that does not fit in memory, the march runs
+    if (cudaMalloc((void **)&f.discs, sizeof(float) * (sums + 2 * g.nx * tiles)) != cudaSuccess) {
+        cudaGetLastError();
+        f.discs = nullptr;
+        return HV_OK;
+    }
     f.flags = reinterpret_cast<int *>(f.discs + sums);
     return HV_OK;
 }
