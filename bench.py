@@ -208,6 +208,22 @@ def sor_checks(n_sor, sweeps_per_cycle):
     return math.ceil(n_sor / sweeps_per_cycle) + 1 if sweeps_per_cycle > 0 else 2
 
 
+def direct_solve(n, its, corrected):
+    """Whether the run's solves took the direct form: corrected cycles counted
+    as one iteration each (sweeps count at least a cycle of them)."""
+    return bool(corrected) and n <= 170 and sum(its) < 8 * len(its)
+
+
+def direct_bytes(w, n):
+    """Algorithmic bytes of a direct solve of n corrections.  The first, per
+    node: source 4, start 8, residual written 8; spectrum written and read
+    twice 16; correction written and read 8; residual, start, phi and the
+    solution before it read 32, phi, that and the next start written 24.  A
+    later one: correction 4, residual read and written 16; 24 as above;
+    residual 8, phi and the next start read and written 32."""
+    return w.G * (100 + 84 * (max(int(n), 1) - 1))
+
+
 def step_bytes(w, n_sor, wordsize=4, checks=2, touched=None, force_frac=None):
     """Algorithmic bytes of one step, per kernel.  The particle step: 48 B per
     particle (x, k read and written) and, per grid node its particles touch
@@ -884,6 +900,10 @@ def our_arm(args, world, rank, local):
     force_frac = row_group_fraction(raw, w.n, 4) if gated else None
     nbytes = step_bytes(w, its_p.mean(), ws_, float(np.mean([sor_checks(n, per_cycle) for n in its_p])),
                         touched=touched, force_frac=force_frac)
+    direct = direct_solve(w.n, its_p, prec == hv.HV_F32 and fo.sor_coarse)
+    sor_b = sum(direct_bytes(w, n) if direct else step_bytes(w, n, ws_, sor_checks(n, per_cycle))["sor"] for n in its_p)
+    if direct:
+        nbytes["sor"] = sor_b / len(its_p)
     tot_ms = sum(v[0] for v in kt.values())
     kernels = {}
     for k, (kms, n) in kt.items():
@@ -898,20 +918,24 @@ def our_arm(args, world, rank, local):
     if "forces" in kernels and force_frac is not None:
         kernels["forces"]["computed_row_groups"] = force_frac
     peak, peak_kind = peaks()
-    sor_b = sum(step_bytes(w, n, ws_, sor_checks(n, per_cycle))["sor"] for n in its_p)
     sor_ms = kt["sor"][0]
     achieved = sor_b / (sor_ms / 1e3) / 1e9 if sor_ms > 0 else None
     traffic = None
     if os.path.exists(PROFILE_TRAFFIC):
         try:
             with open(PROFILE_TRAFFIC) as f:
-                traffic = json.load(f).get("bytes_per_launch")
+                rec = json.load(f)
+            if direct == rec.get("kernel", "").startswith("k_poisson_direct"):
+                traffic = rec.get("bytes_per_launch")
         except Exception:
             traffic = None
     roofline = {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s",
                 "frac": achieved / peak if achieved else None, "traffic": traffic,
-                "kernel": "k_sor_fast (persistent red-black SOR, coarse-grid corrected)", "peak_source": peak_kind,
-                "bytes": "per solve: 12 B per node per red+black iteration (read phi, rho_p; write phi), 48 B per "
+                "kernel": "k_poisson_direct (exact corrections by sine transforms and elimination)" if direct else
+                          "k_sor_fast (persistent red-black SOR, coarse-grid corrected)", "peak_source": peak_kind,
+                "bytes": "per node: 100 B for a solve's first correction (source, start, residual, history, the "
+                         "spectrum and the correction), 84 B for a later one" if direct else
+                         "per solve: 12 B per node per red+black iteration (read phi, rho_p; write phi), 48 B per "
                          "node for the extrapolated start, 32 B per node per FP64 residual check",
                 "mean_sor_iterations": float(its_p.mean()),
                 "sor_checks_per_solve": float(np.mean([sor_checks(n, per_cycle) for n in its_p]))}
