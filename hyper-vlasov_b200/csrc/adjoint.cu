@@ -55,7 +55,7 @@ __global__ void k_adj_gather_field(Geom g, int protons, int total, const double 
     if (i >= total) return;
     const int nx = g.nx, ny = g.ny, nz = g.nz;
     const double cx = cell(x[i], g.dmx, nx), cy = cell(y[i], g.dmy, ny), cz = cell(z[i], g.dmz, nz);
-    if (cx < 0.0 || cy < 0.0 || cz < 0.0 || cx >= nx || cy >= ny || cz >= nz) return;
+    if (!(cx >= 0.0 && cy >= 0.0 && cz >= 0.0 && cx < nx && cy < ny && cz < nz)) return;  // NaN is outside
     const int x0 = (int)cx, y0 = (int)cy, z0 = (int)cz;
     const double dx = cx - x0, dy = cy - y0, dz = cz - z0;
     const double wx[2] = {1.0 - dx, dx}, wy[2] = {1.0 - dy, dy}, wz[2] = {1.0 - dz, dz};
@@ -90,7 +90,7 @@ __global__ void k_adj_weights(Geom g, int protons, int total, const double *__re
     if (i >= total) return;
     const int nx = g.nx, ny = g.ny, nz = g.nz;
     const double cx = cell(x[i], g.dmx, nx), cy = cell(y[i], g.dmy, ny), cz = cell(z[i], g.dmz, nz);
-    if (cx < 0.0 || cy < 0.0 || cz < 0.0 || cx >= nx || cy >= ny || cz >= nz) return;
+    if (!(cx >= 0.0 && cy >= 0.0 && cz >= 0.0 && cx < nx && cy < ny && cz < nz)) return;  // NaN is outside
     const int x0 = (int)cx, y0 = (int)cy, z0 = (int)cz;
     const double dx = cx - x0, dy = cy - y0, dz = cz - z0;
     const double hx = nx / (2.0 * g.dmx), hy = ny / (2.0 * g.dmy), hz = nz / (2.0 * g.dmz);  // dc/dpos

@@ -92,6 +92,13 @@ __device__ __forceinline__ void cell_coords(const CellMap<T> &m, T px, T py, T p
     }
 }
 
+// Whether grid coordinates lie in a cell; NaN does not (converted to an index
+// it would be any).
+template <typename T>
+__device__ __forceinline__ bool in_grid(T cx, T cy, T cz, int nx, int ny, int nz) {
+    return cx >= T(0) && cy >= T(0) && cz >= T(0) && cx < nx && cy < ny && cz < nz;
+}
+
 // CIC force gather at (px,py,pz) (distribute_forces_to_particles_cic,
 // include/tools.hpp:98-168; corner order and corner drop as there).
 template <typename T>
@@ -101,7 +108,7 @@ __device__ __forceinline__ void gather_at(const Geom &g, const CellMap<T> &m, co
     ax = ay = az = T(0);
     T cx, cy, cz;
     cell_coords<T>(m, px, py, pz, cx, cy, cz);
-    if (cx < T(0) || cy < T(0) || cz < T(0) || cx >= nx || cy >= ny || cz >= nz) return;
+    if (!in_grid<T>(cx, cy, cz, nx, ny, nz)) return;
     int x0 = (int)cx, y0 = (int)cy, z0 = (int)cz;
     T dx = cx - x0, dy = cy - y0, dz = cz - z0;
     T tx = T(1) - dx, ty = T(1) - dy, tz = T(1) - dz;
@@ -136,7 +143,7 @@ __device__ __forceinline__ void deposit_at(const Geom &g, const CellMap<T> &m, T
     const int nx = g.nx, ny = g.ny, nz = g.nz;
     T cx, cy, cz;
     cell_coords<T>(m, px, py, pz, cx, cy, cz);
-    if (cx < T(0) || cy < T(0) || cz < T(0) || cx >= nx || cy >= ny || cz >= nz) return;
+    if (!in_grid<T>(cx, cy, cz, nx, ny, nz)) return;
     int x0 = (int)cx, y0 = (int)cy, z0 = (int)cz;
     T dx = cx - x0, dy = cy - y0, dz = cz - z0;
     T tx = T(1) - dx, ty = T(1) - dy, tz = T(1) - dz;
@@ -230,7 +237,7 @@ __device__ __forceinline__ void deposit_warp(const Geom &g, const CellMap<float>
     const int lane = threadIdx.x & 31;
     float cx, cy, cz;
     cell_coords<float>(m, px, py, pz, cx, cy, cz);
-    const bool in = valid && !(cx < 0.0f || cy < 0.0f || cz < 0.0f || cx >= nx || cy >= ny || cz >= nz);
+    const bool in = valid && in_grid<float>(cx, cy, cz, nx, ny, nz);
     int x0 = 0, y0 = 0, z0 = 0;
     float w[8] = {0, 0, 0, 0, 0, 0, 0, 0};
     long long key = -1;
@@ -301,7 +308,7 @@ __device__ __forceinline__ void list_wrap(const PArgs<float> &a, const CellMap<f
     float cx, cy, cz;
     cell_coords<float>(m, px, py, pz, cx, cy, cz);
     bool want = false;
-    if (valid && !(cx < 0.0f || cy < 0.0f || cz < 0.0f || cx >= nx || cy >= ny || cz >= nz)) {
+    if (valid && in_grid<float>(cx, cy, cz, nx, ny, nz)) {
         const int x0 = (int)cx, y0 = (int)cy, z0 = (int)cz;
         want = x0 < a.wA || x0 >= nx - a.wA - 1 || y0 < a.wB || y0 >= ny - a.wB - 1 || z0 < a.wW ||
                z0 >= nz - a.wW - 1;

@@ -30,7 +30,8 @@ __device__ __forceinline__ T cell_coord(T pos, T dmax, int n) {
 
 template <typename T>
 __device__ __forceinline__ bool in_grid(T cx, T cy, T cz, int nx, int ny, int nz) {
-    return !(cx < T(0.0) || cy < T(0.0) || cz < T(0.0) || cx >= nx || cy >= ny || cz >= nz);
+    // a NaN coordinate is outside: converted to an index it would be any
+    return cx >= T(0.0) && cy >= T(0.0) && cz >= T(0.0) && cx < nx && cy < ny && cz < nz;
 }
 
 // ---- CIC deposit, atomic (include/tools.hpp:35-96) -----------------------
