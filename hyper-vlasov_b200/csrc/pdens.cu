@@ -33,6 +33,7 @@ __global__ void k_bbox_partials(int total, const T *__restrict__ x, const T *__r
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < total; i += gridDim.x * blockDim.x) {
         const double v[3] = {(double)x[i], (double)y[i], (double)z[i]};
         for (int a = 0; a < 3; a++) {
+            if (!isfinite(v[a])) continue;  // no partner of anything: any cell does
             lo[a] = fmin(lo[a], v[a]);
             hi[a] = fmax(hi[a], v[a]);
         }
@@ -194,7 +195,7 @@ __global__ void __launch_bounds__(kBlock) k_pair_densities(int total, Cells cl, 
                 const typename Vec4<T>::type o = sp[j];
                 const T ex = xi - o.x, ey = yi - o.y, ez = zi - o.z;
                 const T d2 = ex * ex + ey * ey + ez * ez;
-                if (d2 > cutoff) continue;
+                if (!(d2 <= cutoff)) continue;  // NaN too
                 const T f = gauss(d2, exp_term, exp2_term, table);
                 a += o.w * f;        // protons
                 b += f - o.w * f;    // neutrons
@@ -246,13 +247,22 @@ hv_status particle_densities_at(hv_ctx *c, int N, int protons, const T *px, cons
     const double sig = c->params.sigma_r;
     double edge = sig;
     Cells cl;
+    // counted in double: the box of a run that has blown up overflows an int
+    for (int a = 0; a < 3; a++) {
+        if (hi[a] < lo[a]) lo[a] = hi[a] = 0.0;  // no finite position
+        lo[a] = std::min(std::max(lo[a], -1e150), 1e150);
+        hi[a] = std::min(std::max(hi[a], -1e150), 1e150);
+    }
     for (;;) {
-        long long cells = 1;
+        double cells = 1.0, n[3];
         for (int a = 0; a < 3; a++) {
-            cl.n[a] = (int)std::floor((hi[a] - lo[a]) / edge) + 1;
-            cells *= cl.n[a];
+            n[a] = std::floor((hi[a] - lo[a]) / edge) + 1.0;
+            cells *= n[a];
         }
-        if (cells <= kMaxCells) break;
+        if (cells <= kMaxCells) {
+            for (int a = 0; a < 3; a++) cl.n[a] = (int)n[a];
+            break;
+        }
         edge *= 2.0;
     }
     for (int a = 0; a < 3; a++) cl.lo[a] = lo[a];
