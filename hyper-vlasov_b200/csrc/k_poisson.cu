@@ -652,7 +652,9 @@ __device__ __forceinline__ void direct_body(const DirectArgs<T> &a, const int b)
         a.ctl[1] = max(its, 1);
         // solutions held before phi; a start from phi leaves none
         a.ctl[2] = a.extrapolate ? min(a.ctl[2] + 1, 2) : 0;
-        if (a.its_ring) a.its_ring[step % a.ring] = converged ? its : -its;
+        // negative where the rule was not met, also by a solve that was not
+        // finite before its first correction
+        if (a.its_ring) a.its_ring[step % a.ring] = converged ? its : -max(its, 1);
     }
 }
 

@@ -1443,7 +1443,9 @@ __device__ __forceinline__ void sor_body(const SorArgs<T, S> &a, const int b) {
         a.metric[0] = a.criterion == HV_SOR_REL_RESIDUAL ? rel : maxd;
         a.ctl[1] = max(its, 1);
         if (a.extrapolate) a.ctl[2] = min(a.ctl[2] + 1, 2);
-        if (a.its_ring) a.its_ring[step % a.ring] = converged ? its : -its;
+        // negative where the rule was not met, also by a solve that was not
+        // finite before its first cycle
+        if (a.its_ring) a.its_ring[step % a.ring] = converged ? its : -max(its, 1);
     }
 }
 
