@@ -372,10 +372,12 @@ __device__ __forceinline__ void solve_columns(const DirectArgs<T> &a, float *sm,
         const float other = __shfl_xor_sync(0xffffffffu, y, 16);
         float x;
         if (mx & 1) {
-            // the middle node, between the two sides' last ones
-            x = (lds(fp) + y + other) / (l + 2.0f * e);
+            // the middle node, between the two sides' last ones: their sum
+            // first, so that both sides form the same bits, and one of them
+            // stores it (y and other change places between the sides)
+            x = (lds(fp) + (y + other)) / (l + 2.0f * e);
             __syncwarp();
-            sts(fp, x);
+            if (!side) sts(fp, x);
         } else {
             // the other side's last node: x_other = (y_other + c y) / (1 - c^2)
             x = (other + rc * y) / (e * (1.0f + rc));
