@@ -175,10 +175,9 @@ __global__ void k_adj_skyrme(long long G, double A, double B, double C, double g
 }
 
 // acc[0..3] += the block partials, summed in block order (loaded all at once:
-// the serial chains then wait for additions only, 21 -> 6 us); *norm = 0 for
-// k_adj_coulomb_src.
+// the serial chains then wait for additions only, 21 -> 6 us).
 constexpr int kAccRows = 1024;
-__global__ void k_adj_accumulate(const double *__restrict__ partials, int nb, double *acc, unsigned long long *norm) {
+__global__ void k_adj_accumulate(const double *__restrict__ partials, int nb, double *acc) {
     __shared__ double sh[4 * kAccRows];
     const int c = threadIdx.x;
     double v = 0.0;
@@ -193,23 +192,13 @@ __global__ void k_adj_accumulate(const double *__restrict__ partials, int nb, do
         __syncthreads();
     }
     if (c < 4) acc[c] += v;
-    if (c == 0) *norm = 0ull;
 }
 
 // Source of the transposed Poisson solve: the SOR kernel solves
 // lap mu = -c src, so src = -lam_phi / c gives lap mu = lam_phi.
-// *norm: the largest |src|, as the bits of a double (they order like the values).
-__global__ void k_adj_coulomb_src(long long G, double inv_c, const double *__restrict__ LU, double *src,
-                                  unsigned long long *norm) {
+__global__ void k_adj_coulomb_src(long long G, double inv_c, const double *__restrict__ LU, double *src) {
     const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    const double v = i < G ? -LU[i] * inv_c : 0.0;
-    if (i < G) src[i] = v;
-    unsigned long long m = (unsigned long long)__double_as_longlong(fabs(v));
-    for (int o = 16; o > 0; o >>= 1) {
-        const unsigned long long q = __shfl_xor_sync(0xffffffffu, m, o);
-        m = q > m ? q : m;
-    }
-    if ((threadIdx.x & 31) == 0 && m > *(volatile unsigned long long *)norm) atomicMax(norm, m);
+    if (i < G) src[i] = -LU[i] * inv_c;
 }
 
 __global__ void k_adj_coulomb_add(long long G, double c, const double *__restrict__ mu, double *Lrho) {
@@ -267,7 +256,7 @@ struct Adjoint {
     double *src = nullptr;   // G
     double *mu = nullptr;    // G, zero on the boundary
     double *mu_hist = nullptr;  // fused path: 2 G, mu's two earlier solutions
-    int *actl = nullptr;     // the transposed solves' control words (8), counts (2) and largest source (words 12, 13)
+    int *actl = nullptr;     // fused path: the transposed solves' control words (8) and counts (2)
     double *partials = nullptr;
     double *acc = nullptr;   // 4: dJ/d(A, B, gamma, C)
     // the slot-to-caller permutation of the checkpointed particle state (the
@@ -342,10 +331,10 @@ hv_status adjoint_alloc(hv_ctx *c, int steps, int every, hv_step_path path) {
     HV_TRY(alloc(&a->partials, 4 * (size_t)a->nb_sky));
     HV_TRY(alloc(&a->acc, 4));
     HV_TRY(alloci(&a->perm, N));
-    HV_TRY(alloci(&a->actl, 16));
     if (fused_layout(path)) {
         HV_TRY(alloc(&a->mu_hist, 2 * G));
         HV_TRY(alloci(&a->ck_ctl, (size_t)fused_ctl_words() * (nseg + 1)));
+        HV_TRY(alloci(&a->actl, 10));
     }
     a->cap_steps = steps;
     a->cap_every = every;
@@ -489,18 +478,16 @@ hv_status force_adjoint(hv_ctx *c, int j) {
     const hv_skyrme &sk = c->params.skyrme;
     k_adj_skyrme<<<a->nb_sky, kBlock, 0, c->stream>>>((long long)G, sk.A, sk.B, sk.C, sk.gamma, rho, a->LU, a->Lrho,
                                                      a->partials);
-    unsigned long long *norm = reinterpret_cast<unsigned long long *>(a->actl + 12);
-    k_adj_accumulate<<<1, 256, 0, c->stream>>>(a->partials, a->nb_sky, a->acc, norm);
+    k_adj_accumulate<<<1, 256, 0, c->stream>>>(a->partials, a->nb_sky, a->acc);
     // Coulomb: the proton potential's phi term, through the transposed solve
     const double cc = 4.0 * kPi * kE2;
-    k_adj_coulomb_src<<<nblocks(G), kBlock, 0, c->stream>>>((long long)G, 1.0 / cc, a->LU, a->src, norm);
+    k_adj_coulomb_src<<<nblocks(G), kBlock, 0, c->stream>>>((long long)G, 1.0 / cc, a->LU, a->src);
     HV_CUDA(cudaGetLastError());
     if (fz) {
         // on the persistent kernel, started from the extrapolation of the
         // previous reversed steps' mu; counted on the device
         if (poisson_direct_runs(c))
-            HV_TRY(poisson_launch_adjoint(c, a->src, reinterpret_cast<const double *>(norm), a->mu, a->mu_hist,
-                                          a->mu_hist + G, a->actl));
+            HV_TRY(poisson_launch_adjoint(c, a->src, a->mu, a->mu_hist, a->mu_hist + G, a->actl));
         else
             HV_TRY(sor_fast_launch_adjoint(c, a->src, a->mu, a->mu_hist, a->mu_hist + G, a->actl));
         k_adj_sor_count<<<1, 32, 0, c->stream>>>(sor_fast_status_words(c), a->actl + 8);

@@ -128,12 +128,13 @@ struct PoissonDirect {
     int rt = 0, nt = 0;        // kernel form: rows of a thread's tile, tiles per warp
     int nt8 = 0;               // tiles per warp with eight rows (launches shared with larger planes)
     int shared_tab = 0, nblocks = 0;
-    int plane = 0, one = 0;    // floats of the stored plane, of one direction's matrices
+    int plane = 0, one = 0, axis = 0;  // words of the stored plane, of one direction's matrices, of its larger axis'
+    size_t word = 0;           // bytes of a word: the context's precision
     size_t limit = 0, smem = 0;
-    float *tables = nullptr;   // sine matrices of z and y, both directions, and the eigenvalues (owns the
+    void *tables = nullptr;    // sine matrices of z and y, both directions, and the eigenvalues (owns the
                                // allocation the pointers below lie in)
-    float *work = nullptr;     // the planes' spectrum
-    float *delta = nullptr;    // correction per node, zero on the faces
+    void *work = nullptr;      // the planes' spectrum
+    void *delta = nullptr;     // correction per node, zero on the faces
     double *partials = nullptr;
     unsigned *bar = nullptr;   // [0] arrivals, [1] their count at the last solve's end
 };
@@ -288,8 +289,8 @@ void poisson_release(hv_ctx *c);
 bool poisson_direct_runs(const hv_ctx *c);
 template <typename T>
 hv_status poisson_launch(hv_ctx *c, const T *rho, int *ctl, int *its_ring, int ring, bool step_solve);
-hv_status poisson_launch_adjoint(hv_ctx *c, const double *src, const double *norm, double *mu, double *mu_prev,
-                                 double *mu_guess, int *ctl);
+hv_status poisson_launch_adjoint(hv_ctx *c, const double *src, double *mu, double *mu_prev, double *mu_guess,
+                                 int *ctl);
 hv_status poisson_clear(hv_ctx *c);
 
 // Several float SOR solves run by one cooperative launch (k_sor_fast.cu).

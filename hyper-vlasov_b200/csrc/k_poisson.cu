@@ -2,11 +2,11 @@
 // residual is solved exactly on the run's own grid.
 //
 // The cycle is the persistent SOR's (k_sor_fast.cu): phi in double, the double
-// residual r = b + lap_h phi, the stopping rule tested on it, and a float
-// correction delta with -lap_h delta = r folded in as phi += delta.  Only the
-// way delta is found differs.  The red-black sweeps need dozens of exchanges
+// residual r = b + lap_h phi, the stopping rule tested on it, and a correction
+// delta in the context's precision with -lap_h delta = r, folded in as phi +=
+// delta.  Only the way delta is found differs.  The red-black sweeps need dozens of exchanges
 // between blocks per solve, each a round trip through L2; here delta comes
-// from sine transforms along y and z (dense float matrices, exact for every
+// from sine transforms along y and z (dense matrices, exact for every
 // extent) and a tridiagonal elimination along x, so that a solve is a fixed
 // four phases with a grid barrier after each:
 //   A  per x plane: r (double, from the extrapolated phi), the two forward
@@ -17,7 +17,8 @@
 // and the rule is tested after A and after D.  A float correction leaves the
 // residual's rounding noise, ~1e-6 of it for the rough residual of an
 // extrapolated start and ~3e-4 for the smooth one of a first guess, so a step
-// takes one correction and a first solve two or three.
+// takes one correction and a first solve two or three.  A double one leaves
+// less than any rule that lets a double context take this form.
 //
 // A symmetric half-length form of the transforms halves their work: row j and
 // its mirror are replaced by their sum and difference, of which the odd and
@@ -36,6 +37,12 @@
 // of its loads), transforms 35 (the shared loads of their operands, not the
 // multiply-adds), B 19 (its loads and the chain of eliminations), C 54, D 50
 // (latency), the four barriers with the wait for the slowest block about 25.
+// In double, a step's solve at a rule of 1e-10: 32^3 35 us, 64^3 59, 96^3 132,
+// 128^3 229 (float corrections, two of them for such a rule: 51, 69, 139, 208).
+//
+// All forms spill at 128 registers a thread: 136 to 180 bytes those of planes
+// up to about 150 x 150 in float, 330 and 950 with two and three tiles a warp,
+// 470 to 550 in double (the two walks' operands, not the transforms').
 #include <algorithm>
 #include <cmath>
 #include <cstring>
@@ -48,9 +55,8 @@ namespace hv {
 namespace {
 
 // Double solves take the direct form when their rule is at least this tight: it
-// then pins phi far below what the way to it could show (the correction is in
-// float, the residual and phi in double).  At looser rules the point where the
-// sweeps stop is part of a double run's result, and stays.
+// then pins phi far below what the way to it could show.  At looser rules the
+// point where the sweeps stop is part of a double run's result, and stays.
 constexpr double kDoubleTol = 1e-9;
 constexpr int kThreads = 512;
 constexpr int kWarps = kThreads / 32;
@@ -62,20 +68,19 @@ struct DirectArgs {
     int off, wz, ps;              // second half's column, columns of a stored plane, its pitch in shared memory
     int py;                       // pitch of the y matrices
     int nblocks, cw, cpitch;      // columns of a phase-B group, their pitch
-    int zlen, ylen;               // floats of one z (y) matrix pair
-    int shared_tab, keep_tab;     // y matrices are the z ones; both directions stay in shared memory
-    int front;                    // floats of shared memory before the matrices
+    int zlen, ylen;               // words of one z (y) matrix pair (a word: one T)
+    int shared_tab, tabs;         // y matrices are the z ones; matrices in shared memory: 2 both directions,
+                                  // 1 one direction at a time, 0 one axis of one direction
+    int front;                    // words of shared memory before the matrices
     double dhx2i, dhy2i, dhz2i, ddiag, src_c, tol;
-    float scale;                  // hx^2: the elimination's equations are scaled by it
-    const double *norm;           // largest |source| (null: taken as 1): the float correction works on
-                                  // values of its order, whatever the caller's units
+    T scale;                      // hx^2: the elimination's equations are scaled by it
     int max_iter, extrapolate;
     long long max_spin;
     const T *rho;
     double *phi, *prev, *guess, *resid;  // guess: the next solve's start (interior nodes)
-    float *work, *delta;          // [mx][my][wz] spectrum, [nx][ny][nz] correction (zero on the faces)
-    const float *wz_f, *wz_i, *wy_f, *wy_i;  // matrix pairs: forward and inverse
-    const float *lamy, *lamz;     // eigenvalues times hx^2 in stored order (zero in the gaps)
+    T *work, *delta;              // [mx][my][wz] spectrum, [nx][ny][nz] correction (zero on the faces)
+    const T *wz_f, *wz_i, *wy_f, *wy_i;  // matrix pairs: forward and inverse
+    const T *lamy, *lamz;         // eigenvalues times hx^2 in stored order (zero in the gaps)
     double *partials;
     unsigned *bar;
     int *status;
@@ -86,25 +91,68 @@ struct DirectArgs {
     const int *binst, *bfirst;
 };
 
-__device__ __forceinline__ float rcp_fast(float v) {
+// Four words of a row: what a thread loads, stores and holds of a plane.
+template <typename T>
+struct Quad;
+template <>
+struct Quad<float> {
+    using type = float4;
+};
+struct __align__(16) Double4 {
+    double x, y, z, w;
+};
+template <>
+struct Quad<double> {
+    using type = Double4;
+};
+template <typename T>
+using quad = typename Quad<T>::type;
+
+template <typename T>
+__device__ __forceinline__ quad<T> ld4(const T *p) { return *reinterpret_cast<const quad<T> *>(p); }
+template <typename T>
+__device__ __forceinline__ void st4(T *p, const quad<T> &v) { *reinterpret_cast<quad<T> *>(p) = v; }
+__device__ __forceinline__ float4 ldcg4(const float *p) { return __ldcg(reinterpret_cast<const float4 *>(p)); }
+__device__ __forceinline__ Double4 ldcg4(const double *p) {
+    const double2 a = __ldcg(reinterpret_cast<const double2 *>(p)), b = __ldcg(reinterpret_cast<const double2 *>(p) + 1);
+    return Double4{a.x, a.y, b.x, b.y};
+}
+__device__ __forceinline__ void stcg4(float *p, const float4 &v) { __stcg(reinterpret_cast<float4 *>(p), v); }
+__device__ __forceinline__ void stcg4(double *p, const Double4 &v) {
+    __stcg(reinterpret_cast<double2 *>(p), make_double2(v.x, v.y));
+    __stcg(reinterpret_cast<double2 *>(p) + 1, make_double2(v.z, v.w));
+}
+
+__device__ __forceinline__ float rcp_of(float v) {
     float r;
     asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(v));
     return r;
 }
+__device__ __forceinline__ double rcp_of(double v) { return 1.0 / v; }
 
-__device__ __forceinline__ float lds(unsigned p) {
-    float v;
-    asm volatile("ld.shared.f32 %0, [%1];" : "=f"(v) : "r"(p) : "memory");
-    return v;
+template <typename T>
+__device__ __forceinline__ T lds(unsigned p) {
+    if constexpr (sizeof(T) == 4) {
+        float v;
+        asm volatile("ld.shared.f32 %0, [%1];" : "=f"(v) : "r"(p) : "memory");
+        return v;
+    } else {
+        double v;
+        asm volatile("ld.shared.f64 %0, [%1];" : "=d"(v) : "r"(p) : "memory");
+        return v;
+    }
 }
 __device__ __forceinline__ void sts(unsigned p, float v) { asm volatile("st.shared.f32 [%0], %1;" ::"r"(p), "f"(v) : "memory"); }
+__device__ __forceinline__ void sts(unsigned p, double v) { asm volatile("st.shared.f64 [%0], %1;" ::"r"(p), "d"(v) : "memory"); }
 
 // The matrices' copy to shared memory runs under the work before their first
 // use (tab_wait and a block barrier).
-__device__ __forceinline__ void load_tab(float *dst, const float *src, int n) {
+template <typename T>
+__device__ __forceinline__ void load_tab(T *dst, const T *src, int n) {
+    constexpr int kPer = 16 / sizeof(T);
     const unsigned d = (unsigned)__cvta_generic_to_shared(dst);
-    for (int e = 4 * threadIdx.x; e < n; e += 4 * kThreads)
-        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(d + 4 * e), "l"(src + e) : "memory");
+    for (int e = kPer * threadIdx.x; e < n; e += kPer * kThreads)
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(d + (unsigned)sizeof(T) * e), "l"(src + e) : "memory");
 }
 __device__ __forceinline__ void tab_wait() { asm volatile("cp.async.wait_all;" ::: "memory"); }
 
@@ -132,35 +180,35 @@ __device__ __forceinline__ Tile tile_of(int wt, int CG, int RG) {
 // whole block to have read its operands).  Thread tile: rows rg + RG i, four
 // columns; 12 shared loads of 16 bytes per 4 x 32 multiply-adds (RT = 8).
 template <typename T, int RT, int NT>
-__device__ __forceinline__ void transform_z(const DirectArgs<T> &a, float *P, const float *W) {
+__device__ __forceinline__ void transform_z(const DirectArgs<T> &a, T *P, const T *W) {
     const int RG = (a.my + RT - 1) / RT, CG = a.off / 4, warp = threadIdx.x >> 5, ps = a.ps;
     const int k1 = a.wz - a.off;
-    float acc[NT][RT][4];
+    T acc[NT][RT][4];
     Tile t[NT];
 #pragma unroll
     for (int n = 0; n < NT; n++) {
         t[n] = tile_of<RT>(warp + n * kWarps, CG, RG);
         if (t[n].par && 4 * t[n].cg >= k1) t[n].on = false, t[n].cg = 0;
 #pragma unroll
-        for (int i = 0; i < RT; i++) acc[n][i][0] = acc[n][i][1] = acc[n][i][2] = acc[n][i][3] = 0.0f;
+        for (int i = 0; i < RT; i++) acc[n][i][0] = acc[n][i][1] = acc[n][i][2] = acc[n][i][3] = T(0);
         if (!__any_sync(0xffffffffu, t[n].on)) continue;
-        const float *w = W + t[n].par * a.off * a.off + 4 * t[n].cg;
-        const float *p = P + t[n].rg * ps + t[n].par * a.off;
+        const T *w = W + t[n].par * a.off * a.off + 4 * t[n].cg;
+        const T *p = P + t[n].rg * ps + t[n].par * a.off;
         const int K = t[n].par ? k1 : a.off;
         for (int k = 0; k < K; k += 4) {
-            float4 v[RT];
+            quad<T> v[RT];
 #pragma unroll
-            for (int i = 0; i < RT; i++) v[i] = *reinterpret_cast<const float4 *>(p + RG * i * ps + k);
+            for (int i = 0; i < RT; i++) v[i] = ld4(p + RG * i * ps + k);
 #pragma unroll
             for (int q = 0; q < 4; q++) {
-                const float4 m = *reinterpret_cast<const float4 *>(w + (k + q) * a.off);
+                const quad<T> m = ld4(w + (k + q) * a.off);
 #pragma unroll
                 for (int i = 0; i < RT; i++) {
-                    const float s = q == 0 ? v[i].x : q == 1 ? v[i].y : q == 2 ? v[i].z : v[i].w;
-                    acc[n][i][0] = fmaf(s, m.x, acc[n][i][0]);
-                    acc[n][i][1] = fmaf(s, m.y, acc[n][i][1]);
-                    acc[n][i][2] = fmaf(s, m.z, acc[n][i][2]);
-                    acc[n][i][3] = fmaf(s, m.w, acc[n][i][3]);
+                    const T s = q == 0 ? v[i].x : q == 1 ? v[i].y : q == 2 ? v[i].z : v[i].w;
+                    acc[n][i][0] = fma(s, m.x, acc[n][i][0]);
+                    acc[n][i][1] = fma(s, m.y, acc[n][i][1]);
+                    acc[n][i][2] = fma(s, m.z, acc[n][i][2]);
+                    acc[n][i][3] = fma(s, m.w, acc[n][i][3]);
                 }
             }
         }
@@ -173,8 +221,8 @@ __device__ __forceinline__ void transform_z(const DirectArgs<T> &a, float *P, co
         for (int i = 0; i < RT; i++) {
             const int r = t[n].rg + RG * i;
             if (r < a.my)
-                *reinterpret_cast<float4 *>(P + r * ps + t[n].par * a.off + 4 * t[n].cg) =
-                    make_float4(acc[n][i][0], acc[n][i][1], acc[n][i][2], acc[n][i][3]);
+                st4(P + r * ps + t[n].par * a.off + 4 * t[n].cg,
+                    quad<T>{acc[n][i][0], acc[n][i][1], acc[n][i][2], acc[n][i][3]});
         }
     }
     __syncthreads();
@@ -183,33 +231,33 @@ __device__ __forceinline__ void transform_z(const DirectArgs<T> &a, float *P, co
 // plane := W^T x plane along y: rows kk0 + i of a half from its nk rows.
 // `out` (pitch op) receives the plane; in place after a barrier when it is P.
 template <typename T, int RT, int NT>
-__device__ __forceinline__ void transform_y(const DirectArgs<T> &a, const float *P, const float *W, float *out,
-                                            int op, bool in_place) {
+__device__ __forceinline__ void transform_y(const DirectArgs<T> &a, const T *P, const T *W, T *out, int op,
+                                            bool in_place) {
     const int RG = (a.hy + RT - 1) / RT, CG = a.wz / 4, warp = threadIdx.x >> 5, ps = a.ps;
-    float acc[NT][RT][4];
+    T acc[NT][RT][4];
     Tile t[NT];
 #pragma unroll
     for (int n = 0; n < NT; n++) {
         t[n] = tile_of<RT>(warp + n * kWarps, CG, RG);
 #pragma unroll
-        for (int i = 0; i < RT; i++) acc[n][i][0] = acc[n][i][1] = acc[n][i][2] = acc[n][i][3] = 0.0f;
+        for (int i = 0; i < RT; i++) acc[n][i][0] = acc[n][i][1] = acc[n][i][2] = acc[n][i][3] = T(0);
         if (!__any_sync(0xffffffffu, t[n].on)) continue;
         const int nk = t[n].par ? a.my - a.hy : a.hy;
-        const float *w = W + t[n].par * a.py * a.py + t[n].rg * RT;
-        const float *p = P + t[n].par * a.hy * ps + 4 * t[n].cg;
+        const T *w = W + t[n].par * a.py * a.py + t[n].rg * RT;
+        const T *p = P + t[n].par * a.hy * ps + 4 * t[n].cg;
 #pragma unroll 4
         for (int k = 0; k < nk; k++) {
-            const float4 v = *reinterpret_cast<const float4 *>(p + k * ps);
-            float m[RT];
+            const quad<T> v = ld4(p + k * ps);
+            T m[RT];
 #pragma unroll
             for (int i = 0; i < RT; i += 4)
-                *reinterpret_cast<float4 *>(m + i) = *reinterpret_cast<const float4 *>(w + k * a.py + i);
+                *reinterpret_cast<quad<T> *>(m + i) = ld4(w + k * a.py + i);
 #pragma unroll
             for (int i = 0; i < RT; i++) {
-                acc[n][i][0] = fmaf(m[i], v.x, acc[n][i][0]);
-                acc[n][i][1] = fmaf(m[i], v.y, acc[n][i][1]);
-                acc[n][i][2] = fmaf(m[i], v.z, acc[n][i][2]);
-                acc[n][i][3] = fmaf(m[i], v.w, acc[n][i][3]);
+                acc[n][i][0] = fma(m[i], v.x, acc[n][i][0]);
+                acc[n][i][1] = fma(m[i], v.y, acc[n][i][1]);
+                acc[n][i][2] = fma(m[i], v.z, acc[n][i][2]);
+                acc[n][i][3] = fma(m[i], v.w, acc[n][i][3]);
             }
         }
     }
@@ -222,8 +270,8 @@ __device__ __forceinline__ void transform_y(const DirectArgs<T> &a, const float 
         for (int i = 0; i < RT; i++) {
             const int kk = t[n].rg * RT + i;
             if (kk < nk)
-                *reinterpret_cast<float4 *>(out + (size_t)(t[n].par * a.hy + kk) * op + 4 * t[n].cg) =
-                    make_float4(acc[n][i][0], acc[n][i][1], acc[n][i][2], acc[n][i][3]);
+                st4(out + (size_t)(t[n].par * a.hy + kk) * op + 4 * t[n].cg,
+                    quad<T>{acc[n][i][0], acc[n][i][1], acc[n][i][2], acc[n][i][3]});
         }
     }
     __syncthreads();
@@ -231,27 +279,26 @@ __device__ __forceinline__ void transform_y(const DirectArgs<T> &a, const float 
 
 // Sums and differences of mirrored columns (rows), in the places of the pair.
 template <typename T>
-__device__ __forceinline__ void butterfly_z(const DirectArgs<T> &a, float *P) {
+__device__ __forceinline__ void butterfly_z(const DirectArgs<T> &a, T *P) {
     const int ha = a.mz - a.hz;
     for (int r = threadIdx.x >> 5; r < a.my; r += kWarps)
         for (int j = threadIdx.x & 31; j < ha; j += 32) {
-            float *u = P + r * a.ps + j, *v = P + r * a.ps + a.off + ha - 1 - j;
-            const float s = *u, d = *v;
+            T *u = P + r * a.ps + j, *v = P + r * a.ps + a.off + ha - 1 - j;
+            const T s = *u, d = *v;
             *u = s + d;
             *v = s - d;
         }
     __syncthreads();
 }
 template <typename T>
-__device__ __forceinline__ void butterfly_y(const DirectArgs<T> &a, float *P) {
+__device__ __forceinline__ void butterfly_y(const DirectArgs<T> &a, T *P) {
     const int ha = a.my - a.hy;
     for (int j = threadIdx.x >> 5; j < ha; j += kWarps)
         for (int c = 4 * (threadIdx.x & 31); c < a.wz; c += 128) {
-            float4 *u = reinterpret_cast<float4 *>(P + j * a.ps + c);
-            float4 *v = reinterpret_cast<float4 *>(P + (a.my - 1 - j) * a.ps + c);
-            const float4 s = *u, d = *v;
-            *u = make_float4(s.x + d.x, s.y + d.y, s.z + d.z, s.w + d.w);
-            *v = make_float4(s.x - d.x, s.y - d.y, s.z - d.z, s.w - d.w);
+            T *u = P + j * a.ps + c, *v = P + (a.my - 1 - j) * a.ps + c;
+            const quad<T> s = ld4(u), d = ld4(v);
+            st4(u, quad<T>{s.x + d.x, s.y + d.y, s.z + d.z, s.w + d.w});
+            st4(v, quad<T>{s.x - d.x, s.y - d.y, s.z - d.z, s.w - d.w});
         }
     __syncthreads();
 }
@@ -321,20 +368,20 @@ __device__ __forceinline__ void walk_plane(const DirectArgs<T> &a, int i, int pa
 // so the smooth columns (l ~ 1e-3) keep full relative accuracy.  Bound by the
 // serial chain, mx / 2 steps of an add, a reciprocal and two products.
 template <typename T>
-__device__ __forceinline__ void solve_columns(const DirectArgs<T> &a, float *sm, int group) {
+__device__ __forceinline__ void solve_columns(const DirectArgs<T> &a, T *sm, int group) {
     const int ncol = a.my * a.wz, c0 = group * a.cw, n = min(a.cw, ncol - c0), mx = a.mx, pitch = a.cpitch;
-    float *f = sm, *cc = sm + (size_t)mx * pitch;
+    T *f = sm, *cc = sm + (size_t)mx * pitch;
     const int quads = n >> 2, xs = kThreads / quads, xq = threadIdx.x / quads, q4 = 4 * (threadIdx.x - xq * quads);
-    float *const g = a.work + c0 + q4;
+    T *const g = a.work + c0 + q4;
     constexpr int kU = 8;  // rows in flight per thread
     for (int x = xq < xs ? xq : mx; x < mx; x += kU * xs) {
-        float4 v[kU];
+        quad<T> v[kU];
 #pragma unroll
         for (int u = 0; u < kU; u++)
-            if (x + u * xs < mx) v[u] = __ldcg(reinterpret_cast<const float4 *>(g + (size_t)(x + u * xs) * ncol));
+            if (x + u * xs < mx) v[u] = ldcg4(g + (size_t)(x + u * xs) * ncol);
 #pragma unroll
         for (int u = 0; u < kU; u++)
-            if (x + u * xs < mx) *reinterpret_cast<float4 *>(f + (x + u * xs) * pitch + q4) = v[u];
+            if (x + u * xs < mx) st4(f + (x + u * xs) * pitch + q4, v[u]);
     }
     __syncthreads();
     const int lane = threadIdx.x & 31, col = (threadIdx.x >> 5) * 16 + (lane & 15), side = lane >> 4;
@@ -343,16 +390,16 @@ __device__ __forceinline__ void solve_columns(const DirectArgs<T> &a, float *sm,
         // columns past the group's end (n is a multiple of four) run on what
         // their place holds; nothing reads their results
         const int gcol = c0 + min(col, n - 1), ky = gcol / a.wz;
-        const float l = __ldg(a.lamy + ky) + __ldg(a.lamz + gcol - ky * a.wz);
+        const T l = __ldg(a.lamy + ky) + __ldg(a.lamz + gcol - ky * a.wz);
         // byte addresses in shared memory: the column's rows from this side's
         // end, and its coefficients
-        const int pb = 4 * pitch, step = side ? -pb : pb;
+        const int pb = (int)sizeof(T) * pitch, step = side ? -pb : pb;
         unsigned fp = (unsigned)__cvta_generic_to_shared(f + col + (side ? (mx - 1) * pitch : 0));
         unsigned cp = (unsigned)__cvta_generic_to_shared(cc + col);
-        float e = 1.0f, y = 0.0f, rc = 0.0f;
-        auto forward = [&](float fv) {
-            const float t = l + e;
-            rc = rcp_fast(1.0f + t);
+        T e = T(1), y = T(0), rc = T(0);
+        auto forward = [&](T fv) {
+            const T t = l + e;
+            rc = rcp_of(T(1) + t);
             e = t * rc;
             y = (fv + y) * rc;
             sts(fp, y);
@@ -362,35 +409,35 @@ __device__ __forceinline__ void solve_columns(const DirectArgs<T> &a, float *sm,
         };
         int i = 0;
         for (; i + 4 <= h; i += 4) {
-            const float f0 = lds(fp), f1 = lds(fp + step), f2 = lds(fp + 2 * step), f3 = lds(fp + 3 * step);
+            const T f0 = lds<T>(fp), f1 = lds<T>(fp + step), f2 = lds<T>(fp + 2 * step), f3 = lds<T>(fp + 3 * step);
             forward(f0);
             forward(f1);
             forward(f2);
             forward(f3);
         }
-        for (; i < h; i++) forward(lds(fp));
-        const float other = __shfl_xor_sync(0xffffffffu, y, 16);
-        float x;
+        for (; i < h; i++) forward(lds<T>(fp));
+        const T other = __shfl_xor_sync(0xffffffffu, y, 16);
+        T x;
         if (mx & 1) {
             // the middle node, between the two sides' last ones: their sum
             // first, so that both sides form the same bits, and one of them
             // stores it (y and other change places between the sides)
-            x = (lds(fp) + (y + other)) / (l + 2.0f * e);
+            x = (lds<T>(fp) + (y + other)) / (l + T(2) * e);
             __syncwarp();
             if (!side) sts(fp, x);
         } else {
             // the other side's last node: x_other = (y_other + c y) / (1 - c^2)
-            x = (other + rc * y) / (e * (1.0f + rc));
+            x = (other + rc * y) / (e * (T(1) + rc));
         }
         __syncwarp();
-        auto back = [&](float cv, float yv) {
-            x = fmaf(cv, x, yv);
+        auto back = [&](T cv, T yv) {
+            x = fma(cv, x, yv);
             fp -= step;
             sts(fp, x);
         };
         for (; i >= 4; i -= 4) {
-            const float c3 = lds(cp - pb), c2 = lds(cp - 2 * pb), c1 = lds(cp - 3 * pb), c0v = lds(cp - 4 * pb);
-            const float y3 = lds(fp - step), y2 = lds(fp - 2 * step), y1 = lds(fp - 3 * step), y0 = lds(fp - 4 * step);
+            const T c3 = lds<T>(cp - pb), c2 = lds<T>(cp - 2 * pb), c1 = lds<T>(cp - 3 * pb), c0v = lds<T>(cp - 4 * pb);
+            const T y3 = lds<T>(fp - step), y2 = lds<T>(fp - 2 * step), y1 = lds<T>(fp - 3 * step), y0 = lds<T>(fp - 4 * step);
             back(c3, y3);
             back(c2, y2);
             back(c1, y1);
@@ -398,13 +445,13 @@ __device__ __forceinline__ void solve_columns(const DirectArgs<T> &a, float *sm,
             cp -= 4 * pb;
         }
         for (; i > 0; i--) {
-            back(lds(cp - pb), lds(fp - step));
+            back(lds<T>(cp - pb), lds<T>(fp - step));
             cp -= pb;
         }
     }
     __syncthreads();
     for (int x = xq < xs ? xq : mx; x < mx; x += xs)
-        __stcg(reinterpret_cast<float4 *>(g + (size_t)x * ncol), *reinterpret_cast<const float4 *>(f + x * pitch + q4));
+        stcg4(g + (size_t)x * ncol, ld4(f + x * pitch + q4));
     __syncthreads();
 }
 
@@ -416,41 +463,43 @@ struct Node {
 
 template <typename T, int RT, int NT>
 __device__ __forceinline__ void direct_body(const DirectArgs<T> &a, const int b) {
-    extern __shared__ __align__(16) float sm[];
+    extern __shared__ __align__(16) unsigned char direct_smem[];
+    T *sm = reinterpret_cast<T *>(direct_smem);
     __shared__ double s_tot[2];
     const int tid = threadIdx.x;
     int *err = a.status;
     // shared memory: plane | z matrices | y matrices (| the inverse ones).
     // Phase B's columns lie where the plane lies; matrices that do not fit
     // beside them are loaded anew by each phase
-    float *P = sm, *tz = sm + a.front;
-    float *ty = a.shared_tab ? tz : tz + a.zlen;
+    T *P = sm, *tz = sm + a.front;
+    // (one axis at a time: the y matrices replace the z ones between the two
+    // transforms of every plane)
+    constexpr bool kOneAxis = sizeof(T) == 8;
+    const bool one_axis = kOneAxis && a.tabs == 0;
+    T *ty = a.shared_tab || one_axis ? tz : tz + a.zlen;
     const int one = a.zlen + (a.shared_tab ? 0 : a.ylen);
-    float *tzi = a.keep_tab ? tz + one : tz, *tyi = a.keep_tab ? ty + one : ty;
+    T *tzi = a.tabs == 2 ? tz + one : tz, *tyi = a.tabs == 2 ? ty + one : ty;
     const int step = a.ctl[0];
     const int hist = a.extrapolate ? a.ctl[2] : 0;
     const long long sx = (long long)a.ny * a.nz;
-    // the power of two of the largest source: the unit of the correction
-    // (double contexts only; a float context's sources are densities)
-    double unit = 1.0;
-    if constexpr (sizeof(T) == 8) {
-        if (a.norm) {
-            const double m = *a.norm;
-            unit = m > 0.0 && m < 1e300 ? exp2(floor(log2(m))) : 1.0;
-        }
-    }
-    auto lap = [&](double xs, double ys, double zs, float c) {
-        const double v = xs * a.dhx2i + ys * a.dhy2i + zs * a.dhz2i - a.ddiag * (double)c;
-        return sizeof(T) == 8 ? unit * v : v;
+    auto lap = [&](double xs, double ys, double zs, T c) {
+        return xs * a.dhx2i + ys * a.dhy2i + zs * a.dhz2i - a.ddiag * (double)c;
     };
-    auto value = [&](float c) { return sizeof(T) == 8 ? unit * (double)c : (double)c; };
 
     auto load_dir = [&](bool inverse) {
-        if (a.keep_tab) return;
+        if (a.tabs != 1) return;
         load_tab(tz, inverse ? a.wz_i : a.wz_f, a.zlen);
         if (!a.shared_tab) load_tab(ty, inverse ? a.wy_i : a.wy_f, a.ylen);
     };
-    if (a.keep_tab) {
+    auto load_y = [&](bool inverse) {
+        if (one_axis) load_tab(tz, inverse ? a.wy_i : a.wy_f, a.ylen);
+    };
+    auto wait_y = [&]() {
+        if (!one_axis) return;
+        tab_wait();
+        __syncthreads();
+    };
+    if (a.tabs == 2) {
         load_tab(tz, a.wz_f, a.zlen);
         load_tab(tzi, a.wz_i, a.zlen);
         if (!a.shared_tab) {
@@ -465,7 +514,7 @@ __device__ __forceinline__ void direct_body(const DirectArgs<T> &a, const int b)
     auto load_delta = [&](long long id, bool) { return __ldcg(a.delta + id); };
     auto to_plane = [&](int y, int z, double r) {
         const int q = z - 1;
-        P[(y - 1) * a.ps + (q < a.hz ? q : a.off + q - a.hz)] = sizeof(T) == 8 ? (float)(r / unit) * a.scale : (float)r * a.scale;
+        P[(y - 1) * a.ps + (q < a.hz ? q : a.off + q - a.hz)] = (T)r * a.scale;
     };
     auto totals = [&](double &u, double &v) {
         if (tid < 32) {
@@ -518,6 +567,7 @@ __device__ __forceinline__ void direct_body(const DirectArgs<T> &a, const int b)
             P[r * a.ps + (q < gap0 ? a.hz + q : a.wz - gaps + q)] = 0.0f;
         }
         for (int i = 1 + b; i <= a.mx; i += a.nblocks) {
+            if (one_axis) load_tab(tz, a.wz_f, a.zlen);
             if (its == 0) {
                 walk_plane<4>(
                     a, i, 0, 1, load_start, [&](long long id) { return __ldg(a.rho + id); },
@@ -532,7 +582,7 @@ __device__ __forceinline__ void direct_body(const DirectArgs<T> &a, const int b)
             } else {
                 walk_plane<4>(
                     a, i, 0, 1, load_delta, [&](long long id) { return a.resid[id]; },
-                    [&](long long id, int y, int z, float c, double xs, double ys, double zs, double r0) {
+                    [&](long long id, int y, int z, T c, double xs, double ys, double zs, double r0) {
                         const double r = r0 + lap(xs, ys, zs, c);
                         a.resid[id] = r;
                         to_plane(y, z, r);
@@ -542,7 +592,9 @@ __device__ __forceinline__ void direct_body(const DirectArgs<T> &a, const int b)
             __syncthreads();
             butterfly_z(a, P);
             transform_z<T, RT, NT>(a, P, tz);
+            load_y(false);
             butterfly_y(a, P);
+            wait_y();
             transform_y<T, RT, NT>(a, P, ty, a.work + (size_t)(i - 1) * a.my * a.wz, a.wz, false);
         }
         if (its == 0) {
@@ -574,31 +626,34 @@ __device__ __forceinline__ void direct_body(const DirectArgs<T> &a, const int b)
         // ---- C: inverse transforms -------------------------------------------
         load_dir(true);
         for (int i = 1 + b; i <= a.mx; i += a.nblocks) {
-            const float *src = a.work + (size_t)(i - 1) * a.my * a.wz;
+            if (one_axis) load_tab(tz, a.wz_i, a.zlen);
+            const T *src = a.work + (size_t)(i - 1) * a.my * a.wz;
             // a row per group of lanes, eight rows in flight per thread
             const int quads = a.wz >> 2, rs = kThreads / quads, rq = tid / quads, q4 = 4 * (tid - rq * quads);
             for (int r = rq < rs ? rq : a.my; r < a.my; r += 8 * rs) {
-                float4 v[8];
+                quad<T> v[8];
 #pragma unroll
                 for (int u = 0; u < 8; u++)
-                    if (r + u * rs < a.my) v[u] = __ldcg(reinterpret_cast<const float4 *>(src + (r + u * rs) * a.wz + q4));
+                    if (r + u * rs < a.my) v[u] = ldcg4(src + (r + u * rs) * a.wz + q4);
 #pragma unroll
                 for (int u = 0; u < 8; u++)
-                    if (r + u * rs < a.my) *reinterpret_cast<float4 *>(P + (r + u * rs) * a.ps + q4) = v[u];
+                    if (r + u * rs < a.my) st4(P + (r + u * rs) * a.ps + q4, v[u]);
             }
             tab_wait();
             __syncthreads();
             transform_z<T, RT, NT>(a, P, tzi);
+            load_y(true);
             butterfly_z(a, P);
+            wait_y();
             transform_y<T, RT, NT>(a, P, tyi, P, a.ps, true);
             const int hay = a.my - a.hy;
             for (int j = tid >> 5; j < a.hy; j += kWarps)
                 for (int q = tid & 31; q < a.mz; q += 32) {
                     const int c = q < a.hz ? q : a.off + q - a.hz;
-                    const float o = P[j * a.ps + c];
-                    float *d = a.delta + i * sx + q + 1;
+                    const T o = P[j * a.ps + c];
+                    T *d = a.delta + i * sx + q + 1;
                     if (j < hay) {
-                        const float e = P[(a.my - 1 - j) * a.ps + c];
+                        const T e = P[(a.my - 1 - j) * a.ps + c];
                         __stcg(d + (long long)(j + 1) * a.nz, o + e);
                         __stcg(d + (long long)(a.my - j) * a.nz, o - e);
                     } else {
@@ -619,20 +674,20 @@ __device__ __forceinline__ void direct_body(const DirectArgs<T> &a, const int b)
                 walk_plane<4>(
                     a, i, part, parts, load_delta,
                     [&](long long id) { return Node{a.resid[id], start[id], a.phi[id], a.prev[id]}; },
-                    [&](long long id, int, int, float c, double xs, double ys, double zs, const Node &n) {
+                    [&](long long id, int, int, T c, double xs, double ys, double zs, const Node &n) {
                         const double r = n.r + lap(xs, ys, zs, c);
                         rr += r * r;
-                        store_first(id, n.start + value(c), n.phi, n.prev);
+                        store_first(id, n.start + (double)c, n.phi, n.prev);
                     });
             else
                 walk_plane<4>(
                     a, i, part, parts, load_delta,
                     [&](long long id) { return Node{a.resid[id], a.extrapolate ? a.guess[id] : 0.0, a.phi[id], 0.0}; },
-                    [&](long long id, int, int, float c, double xs, double ys, double zs, const Node &n) {
+                    [&](long long id, int, int, T c, double xs, double ys, double zs, const Node &n) {
                         const double r = n.r + lap(xs, ys, zs, c);
                         rr += r * r;
-                        a.phi[id] = n.phi + value(c);
-                        if (a.extrapolate) a.guess[id] = n.start + again * value(c);
+                        a.phi[id] = n.phi + (double)c;
+                        if (a.extrapolate) a.guess[id] = n.start + again * (double)c;
                     });
         }
         block_sum2(rr, bb);
@@ -685,11 +740,10 @@ int warp_tiles(const Geom &g, int off, int wz, int RT) {
 }
 
 // One axis' matrix pair (odd and even wavenumbers), forward [position][k] and
-// inverse [k][position], zero-padded to `pitch` squares.
-void sine_tables(int m, int pitch, std::vector<float> &fwd, std::vector<float> &inv) {
+// inverse [k][position], in zeroed `pitch` squares.
+template <typename T>
+void sine_tables(int m, int pitch, T *fwd, T *inv) {
     const int h = (m + 1) / 2, ha = m - h;
-    fwd.assign((size_t)2 * pitch * pitch, 0.0f);
-    inv.assign((size_t)2 * pitch * pitch, 0.0f);
     const double s = std::sqrt(2.0 / (m + 1));
     for (int par = 0; par < 2; par++)
         for (int p = 0; p < (par ? ha : h); p++)
@@ -697,7 +751,7 @@ void sine_tables(int m, int pitch, std::vector<float> &fwd, std::vector<float> &
                 const int j = par ? ha - 1 - p : p, w = 2 * k + 1 + par;
                 // the argument reduced exactly before the sine
                 const long long r = ((long long)(j + 1) * w) % (2ll * (m + 1));
-                const float v = (float)(s * std::sin(kPi * (double)r / (m + 1)));
+                const T v = (T)(s * std::sin(kPi * (double)r / (m + 1)));
                 fwd[((size_t)par * pitch + p) * pitch + k] = v;
                 inv[((size_t)par * pitch + k) * pitch + p] = v;
             }
@@ -711,31 +765,37 @@ void sine_tables(int m, int pitch, std::vector<float> &fwd, std::vector<float> &
 // (128^3: 114 us with 149 KB, 123 with 220).
 struct Layout {
     bool ok;
-    int cw, front, keep_tab;
+    int cw, front, tabs;
     size_t smem;
 };
 Layout layout(const PoissonDirect &d, const Geom &g, int nblocks) {
     const int mx = g.nx - 2, ncol = (g.ny - 2) * d.wz;
-    const size_t col = (size_t)(mx + mx / 2 + 1), plane = d.plane, one = d.one;
+    const size_t col = (size_t)(mx + mx / 2 + 1), plane = d.plane, one = d.one, word = d.word;
     int cw = std::min(up((ncol + nblocks - 1) / nblocks, 16), 256);
-    while (cw > 16 && col * cw * sizeof(float) > d.limit) cw -= 16;
-    auto total = [&](int w) { return (std::max(plane, col * w) + 2 * one) * sizeof(float); };
+    while (cw > 16 && col * cw * word > d.limit) cw -= 16;
+    auto total = [&](int w) { return (std::max(plane, col * w) + 2 * one) * word; };
     while (cw > 64 && total(cw) > d.limit) cw -= 16;
     Layout l;
     l.cw = cw;
-    l.keep_tab = total(cw) <= d.limit ? 1 : 0;
-    l.front = (int)(l.keep_tab ? std::max(plane, col * cw) : plane);
-    l.smem = l.keep_tab ? total(cw) : std::max(plane + one, col * cw) * sizeof(float);
+    // the transforms wait for matrices brought in axis by axis; only a double
+    // plane whose matrices of one direction do not fit takes that form
+    l.tabs = total(cw) <= d.limit ? 2 : word == 4 || (plane + one) * word <= d.limit ? 1 : 0;
+    l.front = (int)(l.tabs == 2 ? std::max(plane, col * cw) : plane);
+    l.smem = l.tabs == 2 ? total(cw) : std::max(plane + (l.tabs ? one : (size_t)d.axis), col * cw) * word;
     l.ok = l.smem <= d.limit;
     return l;
 }
 
 template <typename T, bool kBatch>
 const void *direct_kernel(int rt, int nt) {
-    if (rt == 4) return (const void *)k_poisson_direct<T, 4, 1, kBatch>;
-    return nt == 1   ? (const void *)k_poisson_direct<T, 8, 1, kBatch>
-           : nt == 2 ? (const void *)k_poisson_direct<T, 8, 2, kBatch>
-                     : (const void *)k_poisson_direct<T, 8, 3, kBatch>;
+    if constexpr (sizeof(T) == 8) {
+        return nt == 1 ? (const void *)k_poisson_direct<T, 4, 1, kBatch> : (const void *)k_poisson_direct<T, 4, 2, kBatch>;
+    } else {
+        if (rt == 4) return (const void *)k_poisson_direct<T, 4, 1, kBatch>;
+        return nt == 1   ? (const void *)k_poisson_direct<T, 8, 1, kBatch>
+               : nt == 2 ? (const void *)k_poisson_direct<T, 8, 2, kBatch>
+                         : (const void *)k_poisson_direct<T, 8, 3, kBatch>;
+    }
 }
 
 template <typename T>
@@ -760,7 +820,7 @@ DirectArgs<T> direct_args(hv_ctx *c, const T *rho, int *ctl, int *its_ring, int 
     a.ylen = 2 * d.py * d.py;
     a.shared_tab = d.shared_tab;
     const Layout lay = layout(d, g, nblocks);
-    a.keep_tab = lay.keep_tab;
+    a.tabs = lay.tabs;
     a.front = lay.front;
     a.nblocks = nblocks;
     a.cw = lay.cw;
@@ -771,7 +831,7 @@ DirectArgs<T> direct_args(hv_ctx *c, const T *rho, int *ctl, int *its_ring, int 
     a.dhz2i = 1.0 / (dz * dz);
     a.ddiag = 2.0 * (a.dhx2i + a.dhy2i + a.dhz2i);
     a.src_c = 4.0 * kPi * kE2;
-    a.scale = (float)(dx * dx);
+    a.scale = (T)(dx * dx);
     a.tol = c->params.sor.tol;
     a.max_iter = c->params.sor.max_iter;
     a.extrapolate = c->fast.sor_warm_start == HV_WARM_EXTRAPOLATE ? 1 : c->fast.sor_warm_start == HV_WARM_QUADRATIC ? 2 : 0;
@@ -781,9 +841,9 @@ DirectArgs<T> direct_args(hv_ctx *c, const T *rho, int *ctl, int *its_ring, int 
     a.prev = c->fused.phi64_prev;
     a.guess = c->fused.phi64_prev2;
     a.resid = c->fused.sor.resid;
-    a.work = d.work;
-    a.delta = d.delta;
-    a.wz_f = d.tables;
+    a.work = static_cast<T *>(d.work);
+    a.delta = static_cast<T *>(d.delta);
+    a.wz_f = static_cast<const T *>(d.tables);
     a.wz_i = a.wz_f + a.zlen;
     a.wy_f = a.wz_i + a.zlen;
     a.wy_i = a.wy_f + a.ylen;
@@ -801,82 +861,108 @@ DirectArgs<T> direct_args(hv_ctx *c, const T *rho, int *ctl, int *its_ring, int 
 
 }  // namespace
 
-// Plans the direct solve of a float context: it runs on every grid whose y-z
-// plane, with the transforms' matrices, fits in one block's shared memory and
-// registers (about 174 nodes per axis); larger planes keep the sweeps.
-hv_status poisson_plan(hv_ctx *c) {
+namespace {
+
+// Fills the sine matrices of z and y (both directions) and the eigenvalues
+// times hx^2 in stored order, zero in the gaps.
+template <typename T>
+std::vector<T> direct_tables(const PoissonDirect &d, const Geom &g) {
+    const int my = g.ny - 2, mz = g.nz - 2, hy = (my + 1) / 2, hz = (mz + 1) / 2;
+    const size_t zlen = (size_t)2 * d.off * d.off, ylen = (size_t)2 * d.py * d.py;
+    std::vector<T> all(2 * zlen + 2 * ylen + up(my, 4) + d.wz, T(0));
+    T *y = all.data() + 2 * zlen, *lam = y + 2 * ylen;
+    sine_tables(mz, d.off, all.data(), all.data() + zlen);
+    sine_tables(my, d.py, y, y + ylen);
+    const double dx = 2.0 * g.dmx / g.nx, dy = 2.0 * g.dmy / g.ny, dz = 2.0 * g.dmz / g.nz;
+    auto eigen = [](int m, int w) { const double s = std::sin(kPi * w / (2.0 * (m + 1))); return 4.0 * s * s; };
+    for (int r = 0; r < my; r++)
+        lam[r] = (T)(eigen(my, r < hy ? 2 * r + 1 : 2 * (r - hy) + 2) * (dx * dx) / (dy * dy));
+    for (int q = 0; q < mz; q++)
+        lam[up(my, 4) + (q < hz ? q : d.off + q - hz)] =
+            (T)(eigen(mz, q < hz ? 2 * q + 1 : 2 * (q - hz) + 2) * (dx * dx) / (dz * dz));
+    return all;
+}
+
+template <typename T>
+hv_status plan_direct(hv_ctx *c) {
     PoissonDirect &d = c->fused.direct;
     const Geom &g = c->geom;
-    d.ok = false;
-    if (c->prec == HV_F64 && c->params.sor.tol > kDoubleTol) return HV_OK;
     const int mx = g.nx - 2, my = g.ny - 2, mz = g.nz - 2;
     const int hy = (my + 1) / 2, hz = (mz + 1) / 2;
+    constexpr bool f64 = sizeof(T) == 8;
+    d.word = sizeof(T);
     d.off = up(hz, 8);
     d.wz = d.off + up(mz - hz, 4);
     d.py = up(hy, 8);
     d.ps = d.wz;
     while (d.ps % 32 != 4 && d.ps % 32 != 12 && d.ps % 32 != 20 && d.ps % 32 != 28) d.ps += 4;
+    // tiles of four rows while one a warp covers the plane, else of eight; in
+    // double eight rows would not fit in registers, but planes that take more
+    // than two tiles of four do not fit in shared memory either
+    const int nt4 = (warp_tiles(g, d.off, d.wz, 4) + kWarps - 1) / kWarps;
     d.nt8 = (warp_tiles(g, d.off, d.wz, 8) + kWarps - 1) / kWarps;
-    if (d.nt8 > 3) return HV_OK;
-    d.rt = warp_tiles(g, d.off, d.wz, 4) <= kWarps ? 4 : 8;
-    d.nt = d.rt == 4 ? 1 : d.nt8;
+    if (f64 ? nt4 > 2 : d.nt8 > 3) return HV_OK;
+    d.rt = f64 || nt4 == 1 ? 4 : 8;
+    d.nt = d.rt == 4 ? nt4 : d.nt8;
     int optin = 0;
     HV_CUDA(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, c->device));
-    const size_t limit = optin - 4096;  // the kernels' static shared memory
     const size_t plane = (size_t)up(my, 8) * d.ps, zl = (size_t)2 * d.off * d.off, yl = (size_t)2 * d.py * d.py;
     d.shared_tab = my == mz ? 1 : 0;
-    const size_t one = zl + (d.shared_tab ? 0 : yl);
     const int ncol = my * d.wz;
     // one block per x plane, more where they shorten phase B
     d.nblocks = std::min(c->sm_count, std::max(mx, (ncol + 31) / 32));
     d.plane = (int)plane;
-    d.one = (int)one;
-    d.limit = limit;
+    d.one = (int)(zl + (d.shared_tab ? 0 : yl));
+    d.axis = (int)std::max(zl, yl);
+    d.limit = optin - 4096;  // the kernels' static shared memory
     const Layout lay = layout(d, g, d.nblocks);
     if (!lay.ok) return HV_OK;
     d.smem = lay.smem;
-    const bool f64 = c->prec == HV_F64;
-    for (const void *k : {f64 ? direct_kernel<double, false>(d.rt, d.nt) : direct_kernel<float, false>(d.rt, d.nt),
-                          f64 ? nullptr : direct_kernel<float, true>(d.rt, d.nt)}) {
+    const void *kernels[2] = {direct_kernel<T, false>(d.rt, d.nt), nullptr};
+    if constexpr (!f64) kernels[1] = direct_kernel<T, true>(d.rt, d.nt);
+    for (const void *k : kernels) {
         if (!k) continue;
         HV_TRY(allow_max_dynamic_smem(k, c->device));
         int per_sm = 0;
         HV_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, kThreads, d.smem));
         if (per_sm < 1) return HV_OK;
     }
-    std::vector<float> zf, zi, yf, yi, lam;
-    sine_tables(mz, d.off, zf, zi);
-    sine_tables(my, d.py, yf, yi);
-    const double dx = 2.0 * g.dmx / g.nx, dy = 2.0 * g.dmy / g.ny, dz = 2.0 * g.dmz / g.nz;
-    auto eigen = [](int m, int w) { const double s = std::sin(kPi * w / (2.0 * (m + 1))); return 4.0 * s * s; };
-    lam.assign((size_t)up(my, 4) + d.wz, 0.0f);
-    for (int r = 0; r < my; r++)
-        lam[r] = (float)(eigen(my, r < hy ? 2 * r + 1 : 2 * (r - hy) + 2) * (dx * dx) / (dy * dy));
-    for (int q = 0; q < mz; q++)
-        lam[up(my, 4) + (q < hz ? q : d.off + q - hz)] =
-            (float)(eigen(mz, q < hz ? 2 * q + 1 : 2 * (q - hz) + 2) * (dx * dx) / (dz * dz));
-    std::vector<float> all;
-    for (const auto *v : {&zf, &zi, &yf, &yi, &lam}) all.insert(all.end(), v->begin(), v->end());
+    const std::vector<T> all = direct_tables<T>(d, g);
     // one allocation: the tables, the spectrum, the correction (zero on the
     // faces), the partial sums and the barrier words
-    const size_t nw = (size_t)mx * ncol, np = 4 * (size_t)c->sm_count;
-    const size_t at_work = up((int)all.size(), 64), at_delta = at_work + (nw + 63) / 64 * 64;
-    const size_t at_part = at_delta + ((size_t)g.G + 63) / 64 * 64, words_all = at_part + np + 64;
+    const size_t nw = (size_t)mx * ncol, np = 2 * (size_t)c->sm_count;
+    const size_t at_work = (all.size() + 63) / 64 * 64, at_delta = at_work + (nw + 63) / 64 * 64;
+    const size_t at_part = at_delta + ((size_t)g.G + 63) / 64 * 64;
+    const size_t bytes = at_part * sizeof(T) + np * sizeof(double) + 256;
     // where that does not fit in memory, the sweeps run as they would without it
-    if (cudaMalloc((void **)&d.tables, words_all * sizeof(float)) != cudaSuccess) {
+    if (cudaMalloc(&d.tables, bytes) != cudaSuccess) {
         cudaGetLastError();
         d.tables = nullptr;
         return HV_OK;
     }
-    d.work = d.tables + at_work;
-    d.delta = d.tables + at_delta;
-    d.partials = reinterpret_cast<double *>(d.tables + at_part);
-    d.bar = reinterpret_cast<unsigned *>(d.tables + at_part + np);
-    HV_CUDA(cudaMemsetAsync(d.delta, 0, (words_all - at_delta) * sizeof(float), c->stream));
-    HV_CUDA(cudaMemcpyAsync(d.tables, all.data(), all.size() * sizeof(float), cudaMemcpyHostToDevice, c->stream));
+    T *base = static_cast<T *>(d.tables);
+    d.work = base + at_work;
+    d.delta = base + at_delta;
+    d.partials = reinterpret_cast<double *>(base + at_part);
+    d.bar = reinterpret_cast<unsigned *>(d.partials + np);
+    HV_CUDA(cudaMemsetAsync(d.delta, 0, bytes - at_delta * sizeof(T), c->stream));
+    HV_CUDA(cudaMemcpyAsync(d.tables, all.data(), all.size() * sizeof(T), cudaMemcpyHostToDevice, c->stream));
     HV_CUDA(cudaStreamSynchronize(c->stream));
     d.ok = true;
     return HV_OK;
+}
+
+}  // namespace
+
+// Plans the direct solve: it runs on every grid whose y-z plane, with the
+// transforms' matrices of one direction (in double: of one axis of it), fits in
+// one block's shared memory and in the registers of the forms above -- square
+// planes of up to 194 x 194 nodes in float, 130 x 130 in double -- of float contexts, and of double ones with a
+// rule of kDoubleTol or tighter.  The others keep the sweeps.
+hv_status poisson_plan(hv_ctx *c) {
+    c->fused.direct.ok = false;
+    if (c->prec == HV_F32) return plan_direct<float>(c);
+    return c->params.sor.tol <= kDoubleTol ? plan_direct<double>(c) : HV_OK;
 }
 
 void poisson_release(hv_ctx *c) {
@@ -914,14 +1000,13 @@ template hv_status poisson_launch<float>(hv_ctx *, const float *, int *, int *, 
 template hv_status poisson_launch<double>(hv_ctx *, const double *, int *, int *, int, bool);
 
 // The adjoint's transposed solve, lap mu = -4 pi e^2 src, with its own history
-// and control words; norm: the largest |src|.
-hv_status poisson_launch_adjoint(hv_ctx *c, const double *src, const double *norm, double *mu, double *mu_prev,
-                                 double *mu_guess, int *ctl) {
+// and control words.
+hv_status poisson_launch_adjoint(hv_ctx *c, const double *src, double *mu, double *mu_prev, double *mu_guess,
+                                 int *ctl) {
     DirectArgs<double> a = direct_args<double>(c, src, ctl, nullptr, 0, c->fused.direct.nblocks);
     a.phi = mu;
     a.prev = mu_prev;
     a.guess = mu_guess;
-    a.norm = norm;
     return launch_one(c, a);
 }
 
