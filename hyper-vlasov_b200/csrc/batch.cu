@@ -43,13 +43,12 @@ struct hv_batch {
     cudaGraphExec_t tail_graph = nullptr; // a run's last, shorter chunk, once its length has come twice
     int tail_len = 0;
     int chunk = 8;
-    char *staging = nullptr;              // pinned: rows, iteration rings, status and seed words of a run
-    size_t staging_bytes = 0;
+    cudaEvent_t ev_done[2] = {nullptr, nullptr};  // end of a chunk's copies, by the chunk's parity
+    char *staging = nullptr;              // pinned: two chunks' rows, iteration rings and status words, and
+                                          // the instances' seed words
 };
 
 namespace {
-
-constexpr int kWindow = 4096;  // steps whose rows wait in pinned memory (a multiple of the chunk)
 
 void drop_graph(hv_batch *b) {
     if (b->graph) cudaGraphExecDestroy(b->graph);
@@ -128,9 +127,8 @@ hv_status hv_batch_create(int n, hv_ctx *const *ctxs, hv_batch **out) {
     };
     if (cudaSetDevice(b->device) != cudaSuccess) return fail(HV_ERR_CUDA);
     if (cudaStreamCreateWithFlags(&b->stream, cudaStreamNonBlocking) != cudaSuccess) return fail(HV_ERR_CUDA);
-    if (cudaEventCreateWithFlags(&b->ev_fork_a, cudaEventDisableTiming) != cudaSuccess ||
-        cudaEventCreateWithFlags(&b->ev_fork_c, cudaEventDisableTiming) != cudaSuccess)
-        return fail(HV_ERR_CUDA);
+    for (cudaEvent_t *e : {&b->ev_fork_a, &b->ev_fork_c, &b->ev_done[0], &b->ev_done[1]})
+        if (cudaEventCreateWithFlags(e, cudaEventDisableTiming) != cudaSuccess) return fail(HV_ERR_CUDA);
     b->streams.resize(n);
     b->ev_a.resize(n);
     b->ev_c.resize(n);
@@ -163,8 +161,8 @@ hv_status hv_batch_destroy(hv_batch *b) {
         if (e) cudaEventDestroy(e);
     for (cudaEvent_t e : b->ev_c)
         if (e) cudaEventDestroy(e);
-    if (b->ev_fork_a) cudaEventDestroy(b->ev_fork_a);
-    if (b->ev_fork_c) cudaEventDestroy(b->ev_fork_c);
+    for (cudaEvent_t e : {b->ev_fork_a, b->ev_fork_c, b->ev_done[0], b->ev_done[1]})
+        if (e) cudaEventDestroy(e);
     if (b->stream) cudaStreamDestroy(b->stream);
     delete b;
     return HV_OK;
@@ -260,22 +258,16 @@ hv_status hv_batch_run(hv_batch *b, int n_steps, hv_observables *obs) {
     if (n_steps == 0) return HV_OK;
     HV_CUDA(cudaSetDevice(b->device));
     const int n = (int)b->ctx.size();
-    // pinned room for what a window of steps reads back, so that the host waits
-    // once a window: per instance the rows, every chunk's iteration ring, two words
-    const int window = std::min(n_steps, kWindow);
-    const int ring = fused_batch_ring(), chunks = (window + b->chunk - 1) / b->chunk;
-    const size_t rows_bytes = sizeof(double) * 8 * (size_t)window, its_bytes = sizeof(int) * (size_t)ring * chunks;
+    // pinned room for what two chunks read back, per instance: the rows, the
+    // iteration ring, the status word and (used once) the solver's seed
+    const int ring = fused_batch_ring();
+    const size_t rows_bytes = sizeof(double) * 8 * (size_t)b->chunk, its_bytes = sizeof(int) * (size_t)ring;
     const size_t per = rows_bytes + its_bytes + 64;
-    if (b->staging_bytes < per * n) {
-        if (b->staging) cudaFreeHost(b->staging);
-        b->staging = nullptr;
-        b->staging_bytes = 0;
-        HV_CUDA(cudaMallocHost((void **)&b->staging, per * n));
-        b->staging_bytes = per * n;
-    }
-    auto rows = [&](int i, int step) { return reinterpret_cast<double *>(b->staging + per * i) + (size_t)8 * step; };
-    auto its = [&](int i, int q) { return reinterpret_cast<int *>(b->staging + per * i + rows_bytes) + (size_t)ring * q; };
-    auto words = [&](int i) { return reinterpret_cast<int *>(b->staging + per * i + rows_bytes + its_bytes); };
+    if (!b->staging) HV_CUDA(cudaMallocHost((void **)&b->staging, 2 * per * n));
+    auto slot = [&](int q, int i) { return b->staging + per * ((size_t)(q & 1) * n + i); };
+    auto rows = [&](int q, int i) { return reinterpret_cast<double *>(slot(q, i)); };
+    auto its = [&](int q, int i) { return reinterpret_cast<int *>(slot(q, i) + rows_bytes); };
+    auto words = [&](int q, int i) { return reinterpret_cast<int *>(slot(q, i) + rows_bytes + its_bytes); };
     std::vector<int> exc(n, -1), start(n);
     for (int i = 0; i < n; i++) {
         hv_ctx *c = b->ctx[i];
@@ -284,9 +276,27 @@ hv_status hv_batch_run(hv_batch *b, int n_steps, hv_observables *obs) {
         HV_CUDA(cudaEventRecord(b->ev_a[i], c->stream));
         HV_CUDA(cudaStreamWaitEvent(b->stream, b->ev_a[i], 0));
     }
-    int from = 0;  // first step of the window
-    for (int done = 0, q = 0; done < n_steps;) {
-        const int k = std::min(b->chunk, n_steps - done);
+    const int chunks = (n_steps + b->chunk - 1) / b->chunk;
+    // Waits for chunk q and decodes its rows.  A solve that gave up ends the
+    // run for every instance; the others' rows of that chunk, and all rows of
+    // the chunks before it, are written.
+    auto settle = [&](int q) -> hv_status {
+        HV_CUDA(cudaEventSynchronize(b->ev_done[q & 1]));
+        const int s0 = q * b->chunk, k = std::min(b->chunk, n_steps - s0);
+        hv_status failed = HV_OK;
+        for (int i = 0; i < n; i++) {
+            const hv_status st = fused_batch_status(b->ctx[i], words(q, i)[0]);
+            if (st != HV_OK) failed = st;
+            else if (obs)
+                fused_batch_decode(b->ctx[i], start[i] + s0, k, rows(q, i), its(q, i), obs + (size_t)i * n_steps + s0);
+        }
+        return failed;
+    };
+    // the host stays one chunk ahead of the device: it learns of a solve that
+    // gave up before a second further chunk is enqueued, and the device never
+    // waits for it
+    for (int q = 0; q < chunks; q++) {
+        const int s0 = q * b->chunk, k = std::min(b->chunk, n_steps - s0);
         cudaGraphExec_t graph = nullptr;
         if (k == b->chunk) {
             if (!b->graph) b->graph = capture_steps(b, k);
@@ -306,37 +316,25 @@ hv_status hv_batch_run(hv_batch *b, int n_steps, hv_observables *obs) {
         // the instances' rows side by side; the next chunk starts after them
         HV_CUDA(cudaEventRecord(b->ev_fork_a, b->stream));
         for (int i = 0; i < n; i++) {
-            HV_CUDA(cudaStreamWaitEvent(b->streams[i], b->ev_fork_a, 0));
-            HV_TRY(fused_batch_rows(b->ctx[i], b->streams[i], start[i] + done, k, rows(i, done - from), its(i, q)));
-            HV_CUDA(cudaEventRecord(b->ev_a[i], b->streams[i]));
+            const cudaStream_t st = b->streams[i];
+            HV_CUDA(cudaStreamWaitEvent(st, b->ev_fork_a, 0));
+            HV_TRY(fused_batch_rows(b->ctx[i], st, start[i] + s0, k, rows(q, i), its(q, i)));
+            HV_CUDA(cudaMemcpyAsync(words(q, i), b->ctx[i]->fused.sor.status, sizeof(int), cudaMemcpyDeviceToHost, st));
+            HV_CUDA(cudaEventRecord(b->ev_a[i], st));
             HV_CUDA(cudaStreamWaitEvent(b->stream, b->ev_a[i], 0));
         }
-        done += k;
-        q++;
-        if (done < n_steps && done - from < window) continue;
-        // a solve that gave up leaves every instance's run where it was
-        for (int i = 0; i < n; i++)
-            HV_CUDA(cudaMemcpyAsync(words(i), b->ctx[i]->fused.sor.status, sizeof(int), cudaMemcpyDeviceToHost,
-                                    b->stream));
-        HV_CUDA(cudaStreamSynchronize(b->stream));
-        hv_status failed = HV_OK;
-        for (int i = 0; i < n; i++) {
-            const hv_status st = fused_batch_status(b->ctx[i], words(i)[0]);
-            if (st != HV_OK) failed = st;
+        HV_CUDA(cudaEventRecord(b->ev_done[q & 1], b->stream));
+        hv_status st = q > 0 ? settle(q - 1) : HV_OK;
+        if (st == HV_OK && q + 1 == chunks) st = settle(q);
+        if (st != HV_OK) {
+            HV_CUDA(cudaStreamSynchronize(b->stream));
+            return st;
         }
-        HV_TRY(failed);
-        if (obs)
-            for (int i = 0; i < n; i++)
-                for (int s = from, c = 0; s < done; s += b->chunk, c++)
-                    fused_batch_decode(b->ctx[i], start[i] + s, std::min(b->chunk, done - s), rows(i, s - from),
-                                       its(i, c), obs + (size_t)i * n_steps + s);
-        from = done;
-        q = 0;
     }
-    for (int i = 0; i < n; i++) HV_TRY(fused_batch_end(b->ctx[i], n_steps, exc[i], words(i) + 1));
+    for (int i = 0; i < n; i++) HV_TRY(fused_batch_end(b->ctx[i], n_steps, exc[i], words(0, i) + 1));
     for (int i = 0; i < n; i++) {
         HV_CUDA(cudaStreamSynchronize(b->ctx[i]->stream));
-        if (words(i)[1] > 0) b->ctx[i]->fused.m_hint = words(i)[1];
+        if (words(0, i)[1] > 0) b->ctx[i]->fused.m_hint = words(0, i)[1];
     }
     return HV_OK;
 }
