@@ -617,7 +617,7 @@ hv_status hv_ctx_destroy(hv_ctx *c) {
     free_state(c->d64);
     free_state(c->d32);
     Scratch &s = c->scratch;
-    void *ptrs[] = {c->perm, c->taps_dev, s.partials, s.sor, s.sort_stage, s.entries, s.dens, s.dens_out, c->taps_runs, s.result, s.keys, s.keys_alt, s.vals, s.vals_alt,
+    void *ptrs[] = {c->perm, c->taps_dev, s.partials, s.sort_stage, s.entries, s.dens, s.dens_out, c->taps_runs, s.result, s.keys, s.keys_alt, s.vals, s.vals_alt,
                     s.cell_start, s.cub_tmp, s.sort_tmp};
     for (void *p : ptrs)
         if (p) cudaFree(p);

@@ -76,13 +76,12 @@ struct State {
 struct Scratch {
     double *partials = nullptr;     // deterministic reduction partials
     size_t partials_len = 0;
-    void *sor = nullptr;            // plain SOR: saved values, partial results, barrier, outcome
-    double *result = nullptr;       // small device results (reductions)
+    double *result = nullptr;       // small device results: reductions, from word 56 the plain SOR's barrier and outcome
     double *h_result = nullptr;     // pinned host mirror of result
     // sorted-deposit buffers
     unsigned int *keys = nullptr, *keys_alt = nullptr;
     int *vals = nullptr, *vals_alt = nullptr;
-    int *cell_start = nullptr;      // [2G + 1]
+    int *cell_start = nullptr;      // [2G + 1]; the plain SOR's saved values between deposits
     void *entries = nullptr;        // sorted particles (allocated when the deposit mode is the sorted one)
     void *cub_tmp = nullptr;
     size_t cub_tmp_bytes = 0;

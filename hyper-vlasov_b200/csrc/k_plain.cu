@@ -1041,14 +1041,11 @@ hv_status launch_sor_plain(hv_ctx *c, T *phi, const T *rho, int *iters, double *
     const T dx = T(2.0) * T(g.dmx) / g.nx, dy = T(2.0) * T(g.dmy) / g.ny, dz = T(2.0) * T(g.dmz) / g.nz;
     const T hx2 = dx * dx, hy2 = dy * dy, hz2 = dz * dz;
     const T inv_dx2 = T(1.0) / (T(2.0) / hx2 + T(2.0) / hy2 + T(2.0) / hz2);
-    // the solver's work space, kept by the context: the saved values, the
-    // partial results, the barrier, the outcome
+    // the solver's work space is the context's: the saved values lie where the
+    // sorted deposit keeps its cells' first particles (2 G + 1 ints, written
+    // anew by every deposit), the partial results and the barrier among the
+    // reductions' words
     Scratch &sc = c->scratch;
-    const size_t nsaved = ((size_t)g.G * sizeof(T) + 255) / 256 * 256, npart = 2 * 2 * (size_t)c->sm_count;
-    if (!sc.sor) {
-        HV_CUDA(cudaMalloc(&sc.sor, nsaved + npart * sizeof(double) + 256));
-    }
-    char *base = static_cast<char *>(sc.sor);
     PlainSor<T> a;
     a.nx = g.nx;
     a.ny = g.ny;
@@ -1079,10 +1076,10 @@ hv_status launch_sor_plain(hv_ctx *c, T *phi, const T *rho, int *iters, double *
     a.nblocks = std::min(c->sm_count, std::max(1, div_up(a.count, kSorBlock)));
     a.max_spin = kDefaultSpin;
     a.phi = phi;
-    a.saved = reinterpret_cast<T *>(base);
+    a.saved = reinterpret_cast<T *>(sc.cell_start);
     a.rho = rho;
-    a.partials = reinterpret_cast<double *>(base + nsaved);
-    a.bar = reinterpret_cast<unsigned *>(a.partials + npart);
+    a.partials = sc.partials;  // 32 doubles per SM and more
+    a.bar = reinterpret_cast<unsigned *>(sc.result + 56);
     a.status = reinterpret_cast<int *>(a.bar + 2);
     a.metric = reinterpret_cast<double *>(a.bar + 8);
     HV_CUDA(cudaMemsetAsync(a.bar, 0, 64, c->stream));
