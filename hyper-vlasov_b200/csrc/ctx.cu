@@ -231,42 +231,51 @@ __global__ void k_slot_keys(Geom g, int protons, int total, const T *__restrict_
     vals[i] = i;
 }
 
-// What a slot re-sort moves: x, y, z, kx, ky, kz and the caller permutation.
+// Up to six particle arrays, and the caller permutation (or null): what one
+// pass of a slot re-sort moves.
 template <typename T>
 struct SlotArrays {
     T *v[6];
     int *perm;
 };
 
-template <typename T>
+template <typename T, int K>
 __global__ void k_gather_slots(int n, const int *__restrict__ from, SlotArrays<T> in, SlotArrays<T> out) {
     const int s = blockIdx.x * blockDim.x + threadIdx.x;
     if (s >= n) return;
     const int i = from[s];
-    T v[6];
+    T v[K];
 #pragma unroll
-    for (int q = 0; q < 6; q++) v[q] = in.v[q][i];
-    const int p = in.perm[i];
+    for (int q = 0; q < K; q++) v[q] = in.v[q][i];
+    const int p = in.perm ? in.perm[i] : 0;
 #pragma unroll
-    for (int q = 0; q < 6; q++) out.v[q][s] = v[q];
-    out.perm[s] = p;
+    for (int q = 0; q < K; q++) out.v[q][s] = v[q];
+    if (in.perm) out.perm[s] = p;
 }
 
-template <typename T>
+template <typename T, int K>
 __global__ void k_copy_slots(int n, SlotArrays<T> in, SlotArrays<T> out) {
     const int s0 = blockIdx.x * 1024 + threadIdx.x;
 #pragma unroll
     for (int u = 0; u < 4; u++) {
         const int s = s0 + 256 * u;
         if (s >= n) break;
-        T v[6];
+        T v[K];
 #pragma unroll
-        for (int q = 0; q < 6; q++) v[q] = in.v[q][s];
-        const int p = in.perm[s];
+        for (int q = 0; q < K; q++) v[q] = in.v[q][s];
+        const int p = in.perm ? in.perm[s] : 0;
 #pragma unroll
-        for (int q = 0; q < 6; q++) out.v[q][s] = v[q];
-        out.perm[s] = p;
+        for (int q = 0; q < K; q++) out.v[q][s] = v[q];
+        if (in.perm) out.perm[s] = p;
     }
+}
+
+// Gathers K arrays into the room behind `stage` and copies them back.
+template <typename T, int K>
+void permute_slots(hv_ctx *c, const int *from, const SlotArrays<T> &a, const SlotArrays<T> &stage) {
+    const int n = c->total;
+    k_gather_slots<T, K><<<div_up(n, 256), 256, 0, c->stream>>>(n, from, a, stage);
+    k_copy_slots<T, K><<<div_up(n, 1024), 256, 0, c->stream>>>(n, stage, a);
 }
 
 template <typename T>
@@ -282,17 +291,19 @@ hv_status sort_slots_typed(hv_ctx *c, State<T> &s) {
     size_t bytes = sc.cub_tmp_bytes;
     HV_CUDA(cub::DeviceRadixSort::SortPairs(sc.cub_tmp, bytes, sc.keys, sc.keys_alt, sc.vals, sc.vals_alt, n, 0,
                                             end_bit, c->stream));
-    // positions, wavenumbers and the caller permutation follow the new order:
-    // gathered into a kept buffer, copied back in one go.  (The forces are not
-    // carried: a fused run writes them at its end, from the field.)
-    const size_t stride = ((size_t)n + 63) / 64 * 64;
-    if (!sc.sort_stage) HV_CUDA(cudaMalloc(&sc.sort_stage, stride * (6 * sizeof(T) + sizeof(int))));
-    SlotArrays<T> a{{s.x, s.y, s.z, s.kx, s.ky, s.kz}, c->perm}, b;
-    T *stage = static_cast<T *>(sc.sort_stage);
-    for (int q = 0; q < 6; q++) b.v[q] = stage + q * stride;
-    b.perm = reinterpret_cast<int *>(stage + 6 * stride);
-    k_gather_slots<T><<<div_up(n, 256), 256, 0, c->stream>>>(n, sc.vals_alt, a, b);
-    k_copy_slots<T><<<div_up(n, 1024), 256, 0, c->stream>>>(n, b, a);
+    // positions, wavenumbers and the caller permutation follow the new order.
+    // (The forces are not carried: a fused run writes them at its end, from the
+    // field.)  The gathered arrays wait in buffers that are free between steps:
+    // the forces', the transfers' stage (8 bytes a particle) and the sort's own
+    if constexpr (sizeof(T) == 4) {
+        T *t = reinterpret_cast<T *>(sc.sort_tmp);
+        permute_slots<T, 6>(c, sc.vals_alt, {{s.x, s.y, s.z, s.kx, s.ky, s.kz}, c->perm},
+                            {{s.fx, s.fy, s.fz, t, t + n, reinterpret_cast<T *>(sc.keys)}, sc.vals});
+    } else {
+        T *t = reinterpret_cast<T *>(sc.sort_tmp);
+        permute_slots<T, 3>(c, sc.vals_alt, {{s.x, s.y, s.z}, c->perm}, {{s.fx, s.fy, t}, sc.vals});
+        permute_slots<T, 3>(c, sc.vals_alt, {{s.kx, s.ky, s.kz}, nullptr}, {{s.fx, s.fy, t}, nullptr});
+    }
     HV_CUDA(cudaGetLastError());
     c->permuted = true;
     return HV_OK;
@@ -617,7 +628,7 @@ hv_status hv_ctx_destroy(hv_ctx *c) {
     free_state(c->d64);
     free_state(c->d32);
     Scratch &s = c->scratch;
-    void *ptrs[] = {c->perm, c->taps_dev, s.partials, s.sort_stage, s.entries, s.dens, s.dens_out, c->taps_runs, s.result, s.keys, s.keys_alt, s.vals, s.vals_alt,
+    void *ptrs[] = {c->perm, c->taps_dev, s.partials, s.entries, s.dens, s.dens_out, c->taps_runs, s.result, s.keys, s.keys_alt, s.vals, s.vals_alt,
                     s.cell_start, s.cub_tmp, s.sort_tmp};
     for (void *p : ptrs)
         if (p) cudaFree(p);

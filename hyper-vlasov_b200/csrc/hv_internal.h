@@ -88,9 +88,8 @@ struct Scratch {
     void *dens = nullptr;           // per-particle densities: work space, and both results
     size_t dens_bytes = 0;
     void *dens_out = nullptr;
-    void *sort_stage = nullptr;     // the slot re-sort's gathered arrays
-    void *sort_tmp = nullptr;       // total x 8 bytes: the stage of
-                                    // uploads and downloads in permuted slot order
+    void *sort_tmp = nullptr;       // total x 8 bytes: the stage of uploads and downloads in permuted slot
+                                    // order, and of a slot re-sort's gathered arrays
 };
 
 // Partition and device buffers of the persistent SOR solver (k_sor_fast.cu).
