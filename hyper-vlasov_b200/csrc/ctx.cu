@@ -116,13 +116,14 @@ State<float> &state<float>(hv_ctx *c) { return c->d32; }
 namespace {
 
 // The sorted deposit's entries, once the parameters ask for that mode (steps
-// are captured into graphs, so nothing is allocated when it runs).
-hv_status alloc_entries(hv_ctx *c) {
-    if (c->params.deposit_mode != HV_DEPOSIT_SORTED || c->scratch.entries) return HV_OK;
-    const size_t bytes = sorted_deposit_entry_bytes(c->total, c->prec);
-    HV_CUDA(cudaMalloc(&c->scratch.entries, bytes));
-    HV_CUDA(cudaMemsetAsync(c->scratch.entries, 0, bytes, c->stream));
-    return HV_OK;
+// are captured into graphs, so nothing is allocated when it runs).  Where they
+// do not fit in memory the deposit goes without.
+void alloc_entries(hv_ctx *c) {
+    if (c->params.deposit_mode != HV_DEPOSIT_SORTED || c->scratch.entries) return;
+    if (cudaMalloc(&c->scratch.entries, sorted_deposit_entry_bytes(c->total, c->prec)) != cudaSuccess) {
+        cudaGetLastError();
+        c->scratch.entries = nullptr;
+    }
 }
 
 // The tap runs and slabs on the device.
@@ -593,7 +594,6 @@ hv_status hv_ctx_create(const hv_world *world, int protons, int neutrons, hv_pre
         return fail(cuda_status(cudaGetLastError(), "taps upload"));
     st = prec == HV_F64 ? alloc_state<double>(c) : alloc_state<float>(c);
     if (st == HV_OK) st = upload_runs(c);
-    if (st == HV_OK) st = alloc_entries(c);
     if (st != HV_OK) return fail(st);
     const int n = c->total > 0 ? c->total : 1;
     Scratch &s = c->scratch;
@@ -611,6 +611,7 @@ hv_status hv_ctx_create(const hv_world *world, int protons, int neutrons, hv_pre
         cudaMalloc(&s.cub_tmp, s.cub_tmp_bytes > 0 ? s.cub_tmp_bytes : 16) != cudaSuccess ||
         cudaMalloc(&s.sort_tmp, sizeof(double) * (size_t)n) != cudaSuccess)
         return fail(cuda_status(cudaErrorMemoryAllocation, "scratch"));
+    alloc_entries(c);
     k_iota<<<div_up(n, 256), 256, 0, c->stream>>>(n, c->perm);
     if (cudaStreamSynchronize(c->stream) != cudaSuccess) return fail(cuda_status(cudaGetLastError(), "create"));
     *out = c;
@@ -669,7 +670,7 @@ hv_status hv_ctx_set_params(hv_ctx *c, const hv_run_params *p) {
         HV_CUDA(cudaStreamSynchronize(c->stream));
     }
     HV_CUDA(cudaSetDevice(c->device));
-    HV_TRY(alloc_entries(c));
+    alloc_entries(c);
     HV_CUDA(cudaStreamSynchronize(c->stream));
     fused_release(c);  // plans and graphs depend on the parameters
     return HV_OK;

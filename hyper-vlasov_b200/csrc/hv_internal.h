@@ -82,7 +82,7 @@ struct Scratch {
     unsigned int *keys = nullptr, *keys_alt = nullptr;
     int *vals = nullptr, *vals_alt = nullptr;
     int *cell_start = nullptr;      // [2G + 1]; the plain SOR's saved values between deposits
-    void *entries = nullptr;        // sorted particles (allocated when the deposit mode is the sorted one)
+    void *entries = nullptr;        // sorted particles (when the deposit mode is the sorted one and they fit)
     void *cub_tmp = nullptr;
     size_t cub_tmp_bytes = 0;
     void *dens = nullptr;           // per-particle densities: work space, and both results

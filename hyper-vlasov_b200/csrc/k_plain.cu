@@ -101,27 +101,39 @@ struct __align__(16) Entry<double> {
     int next, pad;
 };
 
-// Entries in sorted order, and every occupied cell's first one (cell_start is
-// -1 for the others; a search per cell cost 63 us at 128^3).
+// The arrays behind the entries.
 template <typename T>
-__global__ void k_deposit_entries(Geom g, int total, const T *__restrict__ x, const T *__restrict__ y,
-                                  const T *__restrict__ z, const unsigned int *__restrict__ keys,
-                                  const int *__restrict__ sorted_idx, int *cell_start, Entry<T> *ent) {
-    const int s = blockIdx.x * blockDim.x + threadIdx.x;
-    if (s >= total) return;
-    const unsigned int key = keys[s];
-    if ((long long)key >= 2 * g.G) return;
-    const int i = sorted_idx[s];
-    const T cx = cell_coord<T>(x[i], T(g.dmx), g.nx);
-    const T cy = cell_coord<T>(y[i], T(g.dmy), g.ny);
-    const T cz = cell_coord<T>(z[i], T(g.dmz), g.nz);
+struct SortedParticles {
+    const T *x, *y, *z;
+    const unsigned int *keys;  // ascending
+    const int *idx;            // particle of each place
+    int total;
+};
+
+template <typename T>
+__device__ __forceinline__ Entry<T> entry_of(const Geom &g, const SortedParticles<T> &p, int s, unsigned int key, int i) {
+    const T cx = cell_coord<T>(p.x[i], T(g.dmx), g.nx);
+    const T cy = cell_coord<T>(p.y[i], T(g.dmy), g.ny);
+    const T cz = cell_coord<T>(p.z[i], T(g.dmz), g.nz);
     Entry<T> e;
     e.d[0] = cx - (int)cx;
     e.d[1] = cy - (int)cy;
     e.d[2] = cz - (int)cz;
-    e.next = s + 1 == total || keys[s + 1] != key ? kNoParticle : sorted_idx[s + 1];
-    ent[s] = e;
-    if (s == 0 || keys[s - 1] != key) cell_start[key] = s;
+    e.next = s + 1 == p.total || p.keys[s + 1] != key ? kNoParticle : p.idx[s + 1];
+    return e;
+}
+
+// Entries in sorted order (ent null: none are kept), and every occupied cell's
+// first place (cell_start is -1 for the others; a search per cell cost 63 us at
+// 128^3).
+template <typename T>
+__global__ void k_deposit_entries(Geom g, SortedParticles<T> p, int *cell_start, Entry<T> *ent) {
+    const int s = blockIdx.x * blockDim.x + threadIdx.x;
+    if (s >= p.total) return;
+    const unsigned int key = p.keys[s];
+    if ((long long)key >= 2 * g.G) return;
+    if (ent) ent[s] = entry_of<T>(g, p, s, key, p.idx[s]);
+    if (s == 0 || p.keys[s - 1] != key) cell_start[key] = s;
 }
 
 // One thread per node: merges the particle lists of the (up to) eight cells
@@ -143,10 +155,13 @@ __global__ void k_deposit_entries(Geom g, int total, const T *__restrict__ x, co
 // threads 8 or 20 % slower.  40Ca, 4,000 in double: 24-34 us, latency.
 constexpr int kMaxIndex32 = (1 << 29) - 2;  // its key is below kNoParticle's, 0xfffffff8
 
-template <typename T, typename K>
+// kKept: the entries are in memory; else each is formed when its turn comes,
+// from arrays in the callers' order (the same bits, more loads).
+template <typename T, typename K, bool kKept>
 __global__ void __launch_bounds__(128) k_deposit_merge(Geom g, const Entry<T> *__restrict__ ent,
                                                        const int *__restrict__ cell_start,
-                                                       const int *__restrict__ sorted_idx, T *rho) {
+                                                       const int *__restrict__ sorted_idx, SortedParticles<T> part,
+                                                       T *rho) {
     __shared__ int s_pos[8][128];
     const int iz = blockIdx.x * blockDim.x + threadIdx.x, iy = blockIdx.y, tid = threadIdx.x;
     const int sp = blockIdx.z >= (unsigned)g.nx ? 1 : 0, ix = blockIdx.z - sp * g.nx;
@@ -205,7 +220,9 @@ __global__ void __launch_bounds__(128) k_deposit_merge(Geom g, const Entry<T> *_
     while (head[0] < none) {
         const int best = (int)(head[0] & 7);
         const int p = s_pos[best][tid];
-        const Entry<T> e = ent[p];
+        Entry<T> e;
+        if constexpr (kKept) e = ent[p];
+        else e = entry_of<T>(g, part, p, part.keys[p], sorted_idx[p]);
         s_pos[best][tid] = p + 1;
         replace_first((K)e.next << 3 | best);
         // node = cell + corner; corner bit 1 means the "1" side (weight d)
@@ -910,16 +927,17 @@ hv_status launch_deposit_sorted(hv_ctx *c, const T *x, const T *y, const T *z, T
                                             c->total, 0, end_bit, c->stream));
     HV_CUDA(cudaMemsetAsync(s.cell_start, 0xff, sizeof(int) * (size_t)ncell, c->stream));
     Entry<T> *ent = static_cast<Entry<T> *>(s.entries);
-    k_deposit_entries<T><<<blocks_for(c->total), kBlock, 0, c->stream>>>(c->geom, c->total, x, y, z, s.keys_alt,
-                                                                        s.vals_alt, s.cell_start, ent);
+    const SortedParticles<T> part{x, y, z, s.keys_alt, s.vals_alt, c->total};
+    k_deposit_entries<T><<<blocks_for(c->total), kBlock, 0, c->stream>>>(c->geom, part, s.cell_start, ent);
     HV_CUDA(cudaGetLastError());
     const Geom &g = c->geom;
     const int zt = std::min(128, (g.nz + 31) / 32 * 32);
     const dim3 grid((g.nz + zt - 1) / zt, g.ny, 2 * g.nx);
-    if (c->total <= kMaxIndex32)
-        k_deposit_merge<T, unsigned><<<grid, zt, 0, c->stream>>>(g, ent, s.cell_start, s.vals_alt, rho);
-    else
-        k_deposit_merge<T, unsigned long long><<<grid, zt, 0, c->stream>>>(g, ent, s.cell_start, s.vals_alt, rho);
+    auto *merge = c->total > kMaxIndex32 ? (ent ? k_deposit_merge<T, unsigned long long, true>
+                                                : k_deposit_merge<T, unsigned long long, false>)
+                  : ent                  ? k_deposit_merge<T, unsigned, true>
+                                         : k_deposit_merge<T, unsigned, false>;
+    merge<<<grid, zt, 0, c->stream>>>(g, ent, s.cell_start, s.vals_alt, part, rho);
     HV_CUDA(cudaGetLastError());
     return HV_OK;
 }

@@ -75,3 +75,43 @@ def test_slot_re_sort_takes_no_memory(hv, prec):
         for a, b in zip(*out):
             assert np.abs(a - b).max() <= (1e-4 if prec == "f32" else 1e-11) * max(1.0, np.abs(a).max())
     assert used < 2 ** 21, used
+
+
+@pytest.mark.parametrize("prec", ["f32", "f64"])
+def test_sorted_deposit_without_room_for_its_entries(hv, prec):
+    """The deterministic mode asked for on a full device: the deposit goes
+    without its entries and gives the same bits, as do a fused step's fields."""
+    import torch
+    from hv_b200 import _lib as L
+    dtype, precision = (np.float64, hv.HV_F64) if prec == "f64" else (np.float32, hv.HV_F32)
+    path = hv.HV_PATH_PLAIN if prec == "f64" else hv.HV_PATH_FUSED
+    w = replace(hv.PB208_104K, ppn=20000, n=64)  # 4.16 M particles: 67 or 133 MB of entries
+    p = hv.workload_particles(w, dtype)
+    atomic = w.run_params()
+    ordered = replace(w, deposit_mode=hv.HV_DEPOSIT_SORTED).run_params()
+    with hv.Session(w.world(), w.protons, w.neutrons, atomic, precision) as s:
+        s.upload_particles(*p)
+        s.deposit()
+        full, size = [], 2 ** 36
+        while size >= 2 ** 22:
+            if _free() > size + 2 ** 25:
+                full.append(torch.empty(size, dtype=torch.uint8, device="cuda"))
+            else:
+                size //= 2
+        assert _free() < 60e6
+        try:
+            L.check(s.lib.hv_ctx_set_params(s.handle, L.C.byref(ordered)), "hv_ctx_set_params")
+            s.deposit()
+            without = s.download_field(hv.HV_FIELD_DENSITY_RAW)
+        finally:
+            del full
+            torch.cuda.empty_cache()
+        s.run(2, path)
+        again = [s.download_field(hv.HV_FIELD_DENSITY_RAW), s.download_field(hv.HV_FIELD_FORCE_Z)]
+    with hv.Session(w.world(), w.protons, w.neutrons, ordered, precision) as s:
+        s.upload_particles(*p)
+        s.deposit()
+        assert np.array_equal(without, s.download_field(hv.HV_FIELD_DENSITY_RAW))
+        s.run(2, path)
+        kept = [s.download_field(hv.HV_FIELD_DENSITY_RAW), s.download_field(hv.HV_FIELD_FORCE_Z)]
+    assert all(np.array_equal(a, b) for a, b in zip(again, kept))
