@@ -126,12 +126,17 @@ void alloc_entries(hv_ctx *c) {
     }
 }
 
-// The tap runs and slabs on the device.
+// The tap runs and slabs on the device.  Where they do not fit in memory the
+// plain smoothing goes tap by tap.
 hv_status upload_runs(hv_ctx *c) {
     if (c->taps_runs) cudaFree(c->taps_runs);
     c->taps_runs = nullptr;
     const std::vector<int> &v = c->taps.slabs;
-    HV_CUDA(cudaMalloc((void **)&c->taps_runs, sizeof(int) * (v.size() + 4)));
+    if (cudaMalloc((void **)&c->taps_runs, sizeof(int) * (v.size() + 4)) != cudaSuccess) {
+        cudaGetLastError();
+        c->taps_runs = nullptr;
+        return HV_OK;
+    }
     HV_CUDA(cudaMemcpyAsync(c->taps_runs, v.data(), sizeof(int) * v.size(), cudaMemcpyHostToDevice, c->stream));
     return HV_OK;
 }
@@ -643,36 +648,52 @@ hv_status hv_ctx_destroy(hv_ctx *c) {
 hv_status hv_ctx_set_params(hv_ctx *c, const hv_run_params *p) {
     if (!c) return HV_ERR_BAD_ARG;
     HV_TRY(check_params(p));
-    bool taps_change = p->sigma_r != c->params.sigma_r;
-    c->params = *p;
-    if (taps_change) {
-        HV_CUDA(cudaSetDevice(c->device));
-        TapTable t = build_taps(c->world, p->sigma_r);
-        if (t.count != c->taps_count) {
-            HV_CUDA(cudaStreamSynchronize(c->stream));
-            cudaFree(c->taps_dev);
-            c->taps_dev = nullptr;
-            HV_CUDA(cudaMalloc((void **)&c->taps_dev, sizeof(int) * (t.count > 0 ? t.count : 1)));
-            if (c->d64.taps_w) { cudaFree(c->d64.taps_w); HV_CUDA(cudaMalloc((void **)&c->d64.taps_w, sizeof(double) * (t.count > 0 ? t.count : 1))); }
-            if (c->d32.taps_w) { cudaFree(c->d32.taps_w); HV_CUDA(cudaMalloc((void **)&c->d32.taps_w, sizeof(float) * (t.count > 0 ? t.count : 1))); }
-        }
-        c->taps = t;
-        c->taps_count = t.count;
-        HV_CUDA(cudaStreamSynchronize(c->stream));
-        HV_TRY(upload_runs(c));
-        if (t.count > 0) {
-            HV_CUDA(cudaMemcpyAsync(c->taps_dev, t.packed.data(), sizeof(int) * t.count, cudaMemcpyHostToDevice, c->stream));
-            if (c->d64.taps_w)
-                HV_CUDA(cudaMemcpyAsync(c->d64.taps_w, t.w64.data(), sizeof(double) * t.count, cudaMemcpyHostToDevice, c->stream));
-            if (c->d32.taps_w)
-                HV_CUDA(cudaMemcpyAsync(c->d32.taps_w, t.w32.data(), sizeof(float) * t.count, cudaMemcpyHostToDevice, c->stream));
-        }
-        HV_CUDA(cudaStreamSynchronize(c->stream));
-    }
     HV_CUDA(cudaSetDevice(c->device));
-    alloc_entries(c);
     HV_CUDA(cudaStreamSynchronize(c->stream));
+    const bool taps_change = p->sigma_r != c->params.sigma_r;
+    TapTable t;
+    int *dev = nullptr;
+    void *weights = nullptr;
+    const size_t es = c->prec == HV_F64 ? 8 : 4;
+    if (taps_change) {
+        // everything that can fail comes before anything changes
+        t = build_taps(c->world, p->sigma_r);
+        for (int a = 0; a < 3; a++)
+            if (t.lim[a] > 500) return HV_ERR_UNSUPPORTED;
+        const size_t n = t.count > 0 ? t.count : 1;
+        HV_CUDA(cudaMalloc((void **)&dev, sizeof(int) * n));
+        const cudaError_t e = cudaMalloc(&weights, es * n);
+        if (e != cudaSuccess) {
+            cudaFree(dev);
+            cudaGetLastError();
+            return cuda_status(e, "taps");
+        }
+    }
     fused_release(c);  // plans and graphs depend on the parameters
+    c->params = *p;
+    alloc_entries(c);
+    if (!taps_change) return HV_OK;
+    void *old = c->prec == HV_F64 ? (void *)c->d64.taps_w : (void *)c->d32.taps_w;
+    cudaFree(c->taps_dev);
+    cudaFree(old);
+    c->taps = std::move(t);
+    c->taps_count = c->taps.count;
+    c->taps_dev = dev;
+    const void *host;
+    if (c->prec == HV_F64) {
+        c->d64.taps_w = static_cast<double *>(weights);
+        host = c->taps.w64.data();
+    } else {
+        c->d32.taps_w = static_cast<float *>(weights);
+        host = c->taps.w32.data();
+    }
+    HV_TRY(upload_runs(c));
+    if (c->taps_count > 0) {
+        HV_CUDA(cudaMemcpyAsync(dev, c->taps.packed.data(), sizeof(int) * c->taps_count, cudaMemcpyHostToDevice,
+                                c->stream));
+        HV_CUDA(cudaMemcpyAsync(weights, host, es * c->taps_count, cudaMemcpyHostToDevice, c->stream));
+    }
+    HV_CUDA(cudaStreamSynchronize(c->stream));
     return HV_OK;
 }
 

@@ -975,7 +975,7 @@ hv_status launch_smooth(hv_ctx *c, const T *rho_raw, T *rho) {
     rt.words = (rt.ty + 2 * lim[1]) * 4 * rt.pitch;
     rt.wmax = (2 * lim[1] + 1) * (2 * lim[2] + 1);
     const size_t smem = sizeof(T) * (size_t)(rt.words + rt.wmax);
-    if (rt.qz <= kRowThreads && smem <= 48 * 1024 && c->taps.runs > 0) {
+    if (rt.qz <= kRowThreads && smem <= 48 * 1024 && c->taps.runs > 0 && c->taps_runs) {
         k_smooth_rows<T><<<dim3((g.ny + rt.ty - 1) / rt.ty, g.nx, 2), kRowThreads, smem, c->stream>>>(
             g, rt, lim[0], lim[1], lim[2], c->taps.runs, c->taps_runs, w, term, rho_raw, rho);
         HV_CUDA(cudaGetLastError());
