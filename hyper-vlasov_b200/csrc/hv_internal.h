@@ -285,6 +285,8 @@ void fused_invalidate(hv_ctx *c);
 hv_status poisson_plan(hv_ctx *c);
 void poisson_release(hv_ctx *c);
 bool poisson_direct_runs(const hv_ctx *c);
+// what a block of a direct solve on `blocks` blocks owns: whole x planes
+void poisson_tile(const hv_ctx *c, int blocks, int *planes, int *rows);
 template <typename T>
 hv_status poisson_launch(hv_ctx *c, const T *rho, int *ctl, int *its_ring, int ring, bool step_solve);
 hv_status poisson_launch_adjoint(hv_ctx *c, const double *src, double *mu, double *mu_prev, double *mu_guess,

@@ -1308,7 +1308,8 @@ void drop_graph(hv_ctx *c) {
 // Chooses the particle step's block size and grid, then the SOR tile, by
 // timing each candidate's kernel over trial steps (coordinate descent: the
 // particle candidates with the planned tile, then the tiles with the chosen
-// particle configuration).  The trial steps advance the run.
+// particle configuration).  A direct solve has no tile to choose: it is timed
+// as it is.  The trial steps advance the run.
 hv_status fused_autotune(hv_ctx *c, int trial, hv_autotune_report *rep) {
     HV_TRY(fused_run(c, 0, nullptr));  // initial solve and plans, if not done
     HV_TRY(fused_prepare(c));
@@ -1333,33 +1334,45 @@ hv_status fused_autotune(hv_ctx *c, int trial, hv_autotune_report *rep) {
     f.pblock = best_b;
     f.obs_blocks = best_g;
     const double particle_ms = best_ms;
-    // SOR tiles: the plan's first few candidates
-    int ntile = 0, best_rank = 0;
+    int best_rank = 0, planes, rows, solve_blocks;
     double sor_best = 0.0;
-    for (int rank = 0; rank < 4; rank++) {
-        if (rank > 0 && rank >= ntile) break;
-        HV_TRY(sor_fast_replan_rank(c, rank, &ntile));
+    if (poisson_direct_runs(c)) {
         drop_graph(c);
-        if (!f.sor.ok) continue;
-        HV_TRY(time_kernel(c, HV_K_SOR, trial, &ms));
+        HV_TRY(time_kernel(c, HV_K_SOR, trial, &sor_best));
         count++;
-        if (rank == 0 || ms < sor_best) {
-            sor_best = ms;
-            best_rank = rank;
+        poisson_tile(c, f.direct.nblocks, &planes, &rows);
+        solve_blocks = f.direct.nblocks;
+    } else {
+        // SOR tiles: the plan's first few candidates
+        int ntile = 0;
+        for (int rank = 0; rank < 4; rank++) {
+            if (rank > 0 && rank >= ntile) break;
+            HV_TRY(sor_fast_replan_rank(c, rank, &ntile));
+            drop_graph(c);
+            if (!f.sor.ok) continue;
+            HV_TRY(time_kernel(c, HV_K_SOR, trial, &ms));
+            count++;
+            if (rank == 0 || ms < sor_best) {
+                sor_best = ms;
+                best_rank = rank;
+            }
         }
-    }
-    HV_TRY(sor_fast_replan_rank(c, best_rank, &ntile));
-    drop_graph(c);
-    if (!f.sor.ok) {
-        set_last_error("autotune: the chosen SOR tile does not fit on chip");
-        return HV_ERR_UNSUPPORTED;
+        HV_TRY(sor_fast_replan_rank(c, best_rank, &ntile));
+        drop_graph(c);
+        if (!f.sor.ok) {
+            set_last_error("autotune: the chosen SOR tile does not fit on chip");
+            return HV_ERR_UNSUPPORTED;
+        }
+        planes = f.sor.P;
+        rows = f.sor.R;
+        solve_blocks = f.sor.nblocks;
     }
     if (rep) {
         rep->particle_block = f.pblock;
         rep->particle_grid = f.obs_blocks;
-        rep->sor_planes = f.sor.P;
-        rep->sor_rows = f.sor.R;
-        rep->sor_blocks = f.sor.nblocks;
+        rep->sor_planes = planes;
+        rep->sor_rows = rows;
+        rep->sor_blocks = solve_blocks;
         rep->sor_tile_rank = best_rank;
         rep->candidates = count;
         rep->particle_ms = particle_ms;

@@ -979,6 +979,11 @@ bool poisson_direct_runs(const hv_ctx *c) {
            c->params.sor.criterion == HV_SOR_REL_RESIDUAL;
 }
 
+void poisson_tile(const hv_ctx *c, int blocks, int *planes, int *rows) {
+    *planes = div_up(c->geom.nx - 2, blocks);
+    *rows = c->geom.ny;
+}
+
 namespace {
 template <typename T>
 hv_status launch_one(hv_ctx *c, DirectArgs<T> &a) {

@@ -134,8 +134,8 @@ class Session:
 
     def autotune(self, trial_steps=4):
         """hv_ctx_autotune: times the particle step's launch configurations and
-        the SOR tiles over trial_steps fused steps each (the steps advance the
-        run) and keeps the fastest; returns what it chose as a dict."""
+        the SOR tiles (sweeps only) over trial_steps fused steps each (the steps
+        advance the run) and keeps the fastest; returns what it chose as a dict."""
         r = L.hv_autotune_report()
         L.check(self.lib.hv_ctx_autotune(self._ctx, int(trial_steps), C.byref(r)), "hv_ctx_autotune")
         return {k: getattr(r, k) for k, _ in r._fields_}

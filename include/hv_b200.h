@@ -384,10 +384,10 @@ typedef struct hv_autotune_report {
     int particle_block;    /* threads per block of the particle step          */
     int particle_grid;     /* its blocks (a multiple of the SM count)         */
     int sor_planes;        /* the SOR tile: planes x rows owned by one block  */
-    int sor_rows;
+    int sor_rows;          /*   (a direct solve: whole planes)                */
     int sor_blocks;        /* blocks of the solve                             */
     int sor_tile_rank;     /* rank of the tile in the plan's own order (0: the
-                              plan's heuristic choice)                        */
+                              plan's heuristic choice, or a direct solve)     */
     int candidates;        /* configurations timed                            */
     double particle_ms;    /* device ms per launch of the chosen particle step */
     double sor_ms;         /* device ms per launch of the solve with the chosen
@@ -397,11 +397,13 @@ typedef struct hv_autotune_report {
 /* Chooses the fused path's launch configuration for this context by timing
  * candidates over trial_steps steps each (CUDA events around each launch):
  * first the particle step's block size (128, 256, 512 threads) and grid (2, 4,
- * 8 blocks per SM) with the planned SOR tile, then the SOR tile among the
+ * 8, 16 blocks per SM) with the planned SOR tile, then the SOR tile among the
  * plan's four best-ranked P x R partitions (the ranking hv_run's plan uses:
  * fewest quads per thread, then least exchanged face, then fewest blocks).
- * The trial steps advance the run like hv_run (solving the initial fields
- * first if needed); the choice holds for later hv_run calls on the context.
+ * Contexts whose solves take the direct form have no tile to choose; their
+ * solve is timed once.  The trial steps advance the run like hv_run (solving
+ * the initial fields first if needed); the choice holds for later hv_run calls
+ * on the context.
  * No counterpart in the reference. */
 HV_API hv_status hv_ctx_autotune(hv_ctx *ctx, int trial_steps, hv_autotune_report *report);
 
