@@ -342,11 +342,19 @@ hv_status hv_batch_run(hv_batch *b, int n_steps, hv_observables *obs) {
 hv_status hv_batch_autotune(hv_batch *b, int trial_steps, int *chosen_cap) {
     if (!b || trial_steps < 1) return HV_ERR_BAD_ARG;
     HV_CUDA(cudaSetDevice(b->device));
-    const int caps[] = {0, 64, 32, 16, 8, 4};
+    // the cap shapes sweeps only: with direct solves alone there is nothing to
+    // choose, and the instances' own plans stay
+    bool sweeps = false;
+    for (hv_ctx *c : b->ctx) sweeps = sweeps || !poisson_direct_runs(c);
+    std::vector<int> caps = {0, 64, 32, 16, 8, 4};
+    if (!sweeps) {
+        caps.clear();
+        if (b->cap != 0) HV_TRY(hv_batch_plan(b, 0));
+    }
     cudaEvent_t e0, e1;
     HV_CUDA(cudaEventCreate(&e0));
     HV_CUDA(cudaEventCreate(&e1));
-    int best = -1;
+    int best = sweeps ? -1 : 0;
     float best_ms = 0.0f;
     for (int cap : caps) {
         if (hv_batch_plan(b, cap) != HV_OK) continue;
@@ -367,7 +375,7 @@ hv_status hv_batch_autotune(hv_batch *b, int trial_steps, int *chosen_cap) {
         cudaEventDestroy(e1);
         return HV_ERR_UNSUPPORTED;
     }
-    HV_TRY(hv_batch_plan(b, best));
+    if (sweeps) HV_TRY(hv_batch_plan(b, best));
     // then the particle step's block size, the same for every instance
     int best_pb = 0;
     best_ms = 0.0f;
@@ -399,8 +407,10 @@ hv_status hv_batch_tiles(const hv_batch *b, int *sor_planes, int *sor_rows, int 
     if (!b || n < 0 || n > (int)b->ctx.size()) return HV_ERR_BAD_ARG;
     for (int i = 0; i < n; i++) {
         const hv_ctx *c = b->ctx[i];
-        if (sor_planes) sor_planes[i] = c->fused.sor.P;
-        if (sor_rows) sor_rows[i] = c->fused.sor.R;
+        int planes = c->fused.sor.P, rows = c->fused.sor.R;
+        if (poisson_direct_runs(c)) poisson_tile(c, b->blocks[i], &planes, &rows);
+        if (sor_planes) sor_planes[i] = planes;
+        if (sor_rows) sor_rows[i] = rows;
         if (sor_blocks) sor_blocks[i] = b->blocks[i];
         if (particle_block) particle_block[i] = c->fused.pblock;
     }

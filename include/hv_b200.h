@@ -629,15 +629,20 @@ HV_API hv_status hv_adjoint_stats(const hv_ctx *ctx, int *path, int *adjoint_sor
  * with each instance's own SOR plan.  hv_batch_plan re-plans every instance's
  * SOR with at most sor_max_blocks blocks (0: the instance's own plan; an
  * instance whose grid needs more blocks' shared memory gets twice the cap, and
- * so on) and packs the solves into waves of at most one block per SM.  hv_batch_autotune
- * times trial_steps batched steps (plus one) for each candidate cap and keeps
- * the fastest, then does the same for the particle step's block size (128,
+ * so on) and packs the solves into waves of at most one block per SM; direct
+ * solves share launches of all SMs by their work, whatever the cap.
+ * hv_batch_autotune times trial_steps batched steps (plus one) for each
+ * candidate cap and keeps the fastest (0 without a trial where every instance
+ * solves directly), then does the same for the particle step's block size (128,
  * 256 or 512 threads, the same for every instance); the trial steps advance
  * every run.  hv_batch_tiles reports, for the first n instances, the SOR tile
- * (planes x rows per block), the blocks of the solve and the particle step's
- * block size (any pointer may be NULL).  hv_batch_run advances all
- * instances n_steps and writes n_steps observable rows per instance,
- * instance-major (obs[i * n_steps + s]; may be NULL). */
+ * (planes x rows per block; whole planes of a direct solve), the blocks of the
+ * solve and the particle step's block size (any pointer may be NULL).
+ * hv_batch_run advances all instances n_steps and writes n_steps observable
+ * rows per instance, instance-major (obs[i * n_steps + s]; may be NULL).  A
+ * solve whose bounded waits ran out ends the run for all (HV_ERR_TIMEOUT) at
+ * most two chunks of eight steps later; the other instances' rows up to its
+ * chunk's end are written. */
 typedef struct hv_batch hv_batch;
 HV_API hv_status hv_batch_create(int n_instances, hv_ctx *const *ctxs, hv_batch **out);
 HV_API hv_status hv_batch_destroy(hv_batch *batch);

@@ -30,3 +30,32 @@ def test_autotune_searches_tiles_for_sweeps_only(hv, coarse):
         assert 13 <= rep["candidates"] <= 16
         # a tile of some rows of some planes covers the interior planes
         assert rep["sor_planes"] * rep["sor_rows"] * rep["sor_blocks"] >= (w.n - 2) * w.n
+
+
+@pytest.mark.parametrize("coarse", [(1, 1), (0, 1), (0, 0)])
+def test_batch_autotune_searches_caps_for_sweeps_only(hv, coarse):
+    """Three block sizes of the particle step, and six caps before them where
+    an instance of the batch sweeps."""
+    from hv_b200.batch import Batch
+    w = hv.CA40_SMALL
+    trial = 1
+    sessions = []
+    for c in coarse:
+        s = hv.Session.from_workload(w, hv.HV_F32)
+        s.set_fast_options(sor_coarse=c)
+        s.upload_particles(*hv.workload_particles(w, np.float32))
+        sessions.append(s)
+    try:
+        with Batch(sessions) as b:
+            cap = b.autotune(trial)
+            tiles = b.tiles()
+            obs = b.run(1)
+    finally:
+        for s in sessions:
+            s.close()
+    trials = 3 if all(coarse) else 9
+    assert np.allclose(obs["t"][:, 0], trials * (1 + trial) * w.dt)
+    assert cap == 0 if all(coarse) else cap in (0, 64, 32, 16, 8, 4)
+    for c, (planes, rows, blocks, _) in zip(coarse, tiles):
+        if c:
+            assert rows == w.n and planes == -(-(w.n - 2) // blocks)
