@@ -208,10 +208,10 @@ def sor_checks(n_sor, sweeps_per_cycle):
     return math.ceil(n_sor / sweeps_per_cycle) + 1 if sweeps_per_cycle > 0 else 2
 
 
-def direct_solve(n, its, corrected):
+def direct_solve(its, corrected):
     """Whether the run's solves took the direct form: corrected cycles counted
     as one iteration each (sweeps count at least a cycle of them)."""
-    return bool(corrected) and n <= 170 and sum(its) < 8 * len(its)
+    return bool(corrected) and sum(its) < 8 * len(its)
 
 
 def direct_bytes(w, n):
@@ -900,7 +900,7 @@ def our_arm(args, world, rank, local):
     force_frac = row_group_fraction(raw, w.n, 4) if gated else None
     nbytes = step_bytes(w, its_p.mean(), ws_, float(np.mean([sor_checks(n, per_cycle) for n in its_p])),
                         touched=touched, force_frac=force_frac)
-    direct = direct_solve(w.n, its_p, prec == hv.HV_F32 and fo.sor_coarse)
+    direct = direct_solve(its_p, prec == hv.HV_F32 and fo.sor_coarse)
     sor_b = sum(direct_bytes(w, n) if direct else step_bytes(w, n, ws_, sor_checks(n, per_cycle))["sor"] for n in its_p)
     if direct:
         nbytes["sor"] = sor_b / len(its_p)

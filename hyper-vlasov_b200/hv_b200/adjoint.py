@@ -15,8 +15,8 @@ respect to theta = (t0, t3, sigma, a_sym):
 
 Everything runs in FP64: on the plain path (one kernel per reference routine,
 the default) or, with path=HV_PATH_FUSED, on the fused kernels (the fused
-particle step, the persistent SOR for the forward and the transposed Poisson
-solves).
+particle step; for the forward and the transposed Poisson solves the direct
+solve where the workload's rule is 1e-9 or tighter, else the persistent SOR).
 """
 from __future__ import annotations
 

@@ -343,18 +343,28 @@ typedef struct hv_fast_options {
     int sor_coarse;       /* 1 (the default): each cycle of the fused float
                              solve finds its correction exactly: on the run's
                              own grid (sine transforms along y and z, an
-                             elimination along x) where the y-z plane fits in
-                             one block's shared memory -- up to about 170 nodes
-                             on y and z -- and each cycle then counts as one
-                             iteration; on larger planes on a coarse grid
-                             (every F-th node, F the smallest power of two
-                             leaving at most 15 interior coarse nodes per axis)
-                             followed by sor_coarse_sweeps red+black
-                             iterations.  Double solves, the max-update rule
-                             and the phase-counter exchange run plain SOR
-                             cycles, as everything does with 0.  The stopping
-                             rule is unchanged, so only the iterations per
-                             solve change                                      */
+                             elimination along x; the direct form) where the
+                             y-z plane and the transforms' matrices fit in one
+                             block's shared memory -- square planes of up to
+                             194 x 194 nodes, 64 x 256 but not 128 x 256 -- and
+                             each cycle then counts as one iteration, of
+                             hv_sor_params.max_iter too; on larger planes on a
+                             coarse grid (every F-th node, F the smallest power
+                             of two leaving at most 15 interior coarse nodes
+                             per axis) followed by sor_coarse_sweeps red+black
+                             iterations, where F divides every axis and a
+                             block's tile fits the staged sweeps, else plain
+                             SOR cycles.  Double solves with the relative rule
+                             at 1e-9 or tighter, the adjoint's transposed
+                             solves among them, take the direct form too, in
+                             double (square planes of up to 130 x 130): sor
+                             iterations and max_iter count its corrections
+                             there.  The direct form uses neither omega nor
+                             sor_inner_min and sor_inner_max.  Looser double
+                             solves, the max-update rule and the phase-counter
+                             exchange run plain SOR cycles, as everything does
+                             with 0.  The stopping rule is unchanged, so only
+                             the iterations per solve change                   */
     int sor_coarse_sweeps;/* red+black iterations after each coarse-grid
                              correction (default 12)                           */
     int deposit_aggregate;/* 1 (the default): the float atomic deposit of the
@@ -412,7 +422,7 @@ typedef enum hv_kernel_id {
     HV_K_PARTICLE = 0,  /* gather + kicks + drift + deposit + observables      */
     HV_K_SMOOTH = 1,    /* Gaussian smoothing                                  */
     HV_K_SKYRME = 2,    /* Skyrme + symmetry potential                         */
-    HV_K_SOR = 3,       /* persistent Coulomb SOR                              */
+    HV_K_SOR = 3,       /* Coulomb solve (direct, or persistent SOR)           */
     HV_K_FORCES = 4,    /* -grad(U + phi) into the interleaved force field     */
     HV_K_COUNT = 5
 } hv_kernel_id;
@@ -595,8 +605,9 @@ HV_API hv_status hv_adjoint_backward(hv_ctx *ctx, const double *dJ_dD, const dou
  * fused FP64 steps (hv_run(HV_PATH_FUSED) per segment; missing fields are
  * solved with the fused kernels), and the following hv_adjoint_backward
  * recomputes its segments with the same steps and runs each transposed
- * Poisson solve on the persistent SOR kernel, started from the extrapolation
- * of the previous reversed steps' solutions as the fused forward starts phi.
+ * Poisson solve with the fused path's solver (direct at rules of 1e-9 and
+ * tighter, else the persistent SOR), started from the extrapolation of the
+ * previous reversed steps' solutions as the fused forward starts phi.
  * Slot re-sorting (hv_fast_options.sort_every) is paused during both passes,
  * since the adjoint state is indexed by slot.  Device memory: (n / K + 1)
  * (9 N + 13 G) doubles for the checkpoints (phi and its two earlier
