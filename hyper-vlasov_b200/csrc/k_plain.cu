@@ -411,12 +411,15 @@ __device__ __forceinline__ T nan_max(T a, T b) {
 // v / h as the reference rounds it.  kDiv 0: a division; 1: h is a power of two;
 // 2: from y, the rounded reciprocal, by Markstein's theorem (Markstein 1990): a
 // quotient within an ulp plus the exact remainder's correction is the rounded
-// quotient (two corrections: the first product may be two ulps off).
+// quotient (two corrections: the first product may be two ulps off).  The
+// remainders are exact while nothing underflows or overflows: outside that
+// range, and for what is not finite, the division itself.
 template <int kDiv, typename T>
 __device__ __forceinline__ T quotient(T v, T h, T y) {
     if constexpr (kDiv == 0) return v / h;
     if constexpr (kDiv == 1) return v * y;
     T q = v * y;
+    if (!(fabs(q) >= T(1e-280) && fabs(q) <= T(1e280))) return v == T(0) ? v : v / h;
     q = fma(fma(-h, q, v), y, q);
     return fma(fma(-h, q, v), y, q);
 }
@@ -1003,15 +1006,15 @@ hv_status launch_boundary(hv_ctx *c, T *phi) {
 }
 
 // How the solver's quotients by h^2 are formed (quotient's kDiv): a power of
-// two divides exactly by its reciprocal; Markstein's remainders are exact while
-// nothing underflows, and phi falls by about 0.3 a node from its sources, so
-// axes of up to 256 nodes keep it far above 1e-290.
+// two divides exactly by its reciprocal; Markstein's form in double, where h^2
+// and its reciprocal are far inside the range too.
 template <typename T>
 static int division_form(const PlainSor<T> &a) {
     int ex;
     auto pow2 = [&](T v) { return std::frexp(v, &ex) == T(0.5); };
+    auto mid = [](T v) { return v >= T(1e-20) && v <= T(1e20); };
     if (pow2(a.hx2) && pow2(a.hy2) && pow2(a.hz2)) return 1;
-    return sizeof(T) == 8 && std::max(a.nx, std::max(a.ny, a.nz)) <= 256 ? 2 : 0;
+    return sizeof(T) == 8 && mid(a.hx2) && mid(a.hy2) && mid(a.hz2) && std::max(a.nx, std::max(a.ny, a.nz)) <= 256 ? 2 : 0;
 }
 
 // Launches the cluster form where it is the faster one: up to three points of a
