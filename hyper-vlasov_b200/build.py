@@ -57,10 +57,11 @@ def _deps():
 
 
 def compile_one(src, force):
+    """(object, error or None, ptxas notes on spilled registers)."""
     name = os.path.basename(src)
     obj = os.path.join(OBJDIR, name + ".o")
     if not force and os.path.exists(obj) and os.path.getmtime(obj) >= max(os.path.getmtime(src), _deps()):
-        return obj, None
+        return obj, None, []
     cmd = [nvcc(), "-ccbin", host_compiler(), *ARCH, *COMMON, *PER_FILE.get(name, []), "-c", src, "-o", obj]
     if src.endswith(".cpp"):
         cmd[cmd.index("-c")] = "-x"
@@ -68,8 +69,8 @@ def compile_one(src, force):
         cmd.insert(cmd.index("-x") + 2, "-c")
     r = subprocess.run(cmd, capture_output=True, text=True)
     if r.returncode != 0:
-        return obj, f"{' '.join(cmd)}\n{r.stdout}\n{r.stderr}"
-    return obj, (r.stderr if "spill" in r.stderr and "0 bytes spill" not in r.stderr else None) and None
+        return obj, f"{' '.join(cmd)}\n{r.stdout}\n{r.stderr}", []
+    return obj, None, [f"{name}: {line}" for line in r.stderr.splitlines() if "spill" in line.lower()]
 
 
 def build(force=False, jobs=None, verbose=False):
@@ -79,8 +80,10 @@ def build(force=False, jobs=None, verbose=False):
     objs = []
     errors = []
     with cf.ThreadPoolExecutor(max_workers=jobs or min(8, os.cpu_count() or 4)) as ex:
-        for obj, err in ex.map(lambda s: compile_one(s, force), srcs):
+        for obj, err, notes in ex.map(lambda s: compile_one(s, force), srcs):
             objs.append(obj)
+            if verbose:
+                print("\n".join(notes), end="\n" if notes else "")
             if err:
                 errors.append(err)
     if errors:
