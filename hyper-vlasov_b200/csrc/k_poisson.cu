@@ -666,7 +666,7 @@ __device__ __forceinline__ void direct_body(const DirectArgs<T> &a, const int b)
         // ---- D: phi += delta, the FP64 residual of the new phi ---------------
         rr = bb = 0.0;
         // a grid with half as many planes as blocks shares each plane out (64^3:
-        // 62 planes, 132 blocks; 16 steps 1181 -> 1162 us)
+        // 62 planes, 124 blocks; 16 steps 1181 -> 1162 us)
         const int parts = max(1, a.nblocks / a.mx);
         for (int q = b; q < parts * a.mx; q += a.nblocks) {
             const int i = 1 + q / parts, part = q % parts;

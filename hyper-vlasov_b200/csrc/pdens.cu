@@ -156,15 +156,18 @@ __device__ __forceinline__ double gauss(double d2, double e, double, const ExpTa
 // rounding of d^2 in T, whose test decides.
 //
 // Bound by issue slots (23 instructions a scanned partner) and, in double, by
-// the double operations of the exponential.  208Pb, whole calls: 416,000
-// particles in float 8.4 -> 7.8 ms, 104,000 in double 2.9 -> 2.3 ms (exp2f and
-// exp before).  One list for a whole warp, or two particles a thread, measured
-// slower: a warp or thread that crosses from one row of cells into the next
-// then scans the whole nucleus and is waited for.
+// the double operations of the exponential.  208Pb, this kernel alone under the
+// profiler: 416,000 particles in float 8.1 -> 7.4 ms, 104,000 in double 2.5 ->
+// 1.95 (exp2f and exp before).  Whole repeated calls went 9.4 -> 7.9 and 3.5 ->
+// 2.2 ms: the rest is the work space that the context keeps.  One list for a
+// whole warp, or two particles a thread, measured slower: a warp or thread that
+// crosses from one row of cells into the next then scans the whole nucleus and
+// is waited for.
 template <typename T>
 __global__ void __launch_bounds__(kBlock) k_pair_densities(int total, Cells cl, double edge, double reach, T exp_term,
-                                                           T exp2_term, T cutoff, T term, const int *__restrict__ idx, const int *__restrict__ start,
-                                 const typename Vec4<T>::type *__restrict__ sp, T *dp, T *dn) {
+                                                           T exp2_term, T cutoff, T term, const int *__restrict__ idx,
+                                                           const int *__restrict__ start,
+                                                           const typename Vec4<T>::type *__restrict__ sp, T *dp, T *dn) {
     __shared__ double powers[64];
     if (sizeof(T) == 8) {
         if (threadIdx.x < 64) powers[threadIdx.x] = exp2(-(double)threadIdx.x / 64.0);
