@@ -10,7 +10,8 @@ pytestmark = pytest.mark.gpu
 
 # extents of the cluster form and of the cooperative one; no spacing squares to
 # a power of two
-@pytest.mark.parametrize("n,half", [((33, 34, 35), (9.3, 8.7, 10.1)), ((80, 78, 82), (12.1, 11.9, 12.3))])
+@pytest.mark.parametrize("n,half", [((33, 34, 35), (9.3, 8.7, 10.1)), ((80, 78, 82), (12.1, 11.9, 12.3)),
+                                    ((300, 9, 10), (40.0, 1.3, 1.4))])
 @pytest.mark.parametrize("scale", [1.0, 1e-281, 1e-295, 1e-307, 1e-316, 1e281, 1e300])
 def test_plain_solver_divides_exactly_at_any_scale(hv, n, half, scale):
     from hv_b200 import _lib as L
