@@ -302,6 +302,7 @@ hv_status adjoint_alloc(hv_ctx *c, int steps, int every, hv_step_path path) {
         (a->cap_steps + a->cap_every - 1) / a->cap_every >= nseg)
         return HV_OK;
     adjoint_release(c);
+    dens_release(c);
     a = c->adjoint = new Adjoint();
     const size_t N = c->total, G = c->geom.G;
     auto alloc = [&](double **p, size_t n) -> hv_status {

@@ -281,6 +281,9 @@ hv_status fused_run(hv_ctx *c, int n_steps, hv_observables *obs);
 hv_status fused_autotune(hv_ctx *c, int trial, hv_autotune_report *rep);
 void fused_invalidate(hv_ctx *c);
 
+// Frees the pair sums' work space (pdens.cu)
+void dens_release(hv_ctx *c);
+
 // Direct Coulomb solve (k_poisson.cu)
 hv_status poisson_plan(hv_ctx *c);
 void poisson_release(hv_ctx *c);

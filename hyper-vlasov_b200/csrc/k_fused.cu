@@ -1217,6 +1217,7 @@ hv_status run_end(hv_ctx *c, int n_steps, int exc) {
 hv_status fused_prepare(hv_ctx *c) {
     Fused &f = c->fused;
     if (f.ready) return HV_OK;
+    dens_release(c);
     const Geom &g = c->geom;
     const size_t es = c->prec == HV_F64 ? 8 : 4;
     HV_CUDA(cudaMalloc((void **)&f.phi64, sizeof(double) * g.G));

@@ -212,6 +212,18 @@ __global__ void __launch_bounds__(kBlock) k_pair_densities(int total, Cells cl, 
 
 }  // namespace
 
+// Gives the pair sums' work space back, before a context makes room for plans
+// or checkpoints: a run after them has the memory that it would have without.
+void dens_release(hv_ctx *c) {
+    Scratch &sc = c->scratch;
+    if (!sc.dens && !sc.dens_out) return;
+    cudaStreamSynchronize(c->stream);
+    if (sc.dens) cudaFree(sc.dens);
+    if (sc.dens_out) cudaFree(sc.dens_out);
+    sc.dens = sc.dens_out = nullptr;
+    sc.dens_bytes = 0;
+}
+
 // The work space of these calls, kept by the context and grown when a call
 // needs more (stream-ordered allocations were mapped anew by every call: up to
 // 6 ms beside a 2.4 ms kernel).
