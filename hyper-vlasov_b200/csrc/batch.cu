@@ -37,6 +37,7 @@ struct hv_batch {
     cudaEvent_t ev_fork_a = nullptr, ev_fork_c = nullptr;
     std::vector<SorWave> waves;
     std::vector<int> blocks;              // blocks of each instance's solve
+    std::vector<unsigned> gen;            // each context's plan_gen that the waves were built from
     int cap = -1;                         // SOR block cap of the current plan (0: own plans)
     cudaGraphExec_t graph = nullptr;
     int graph_len = 0;
@@ -174,6 +175,7 @@ hv_status hv_batch_plan(hv_batch *b, int sor_max_blocks) {
     HV_CUDA(cudaStreamSynchronize(b->stream));
     drop_graph(b);
     release_waves(b);
+    b->gen.clear();
     const int n = (int)b->ctx.size();
     for (hv_ctx *c : b->ctx) {
         HV_CUDA(cudaStreamSynchronize(c->stream));
@@ -248,6 +250,8 @@ hv_status hv_batch_plan(hv_batch *b, int sor_max_blocks) {
             b->blocks[grp[k]] = direct[q] ? blocks[k] : b->ctx[grp[k]]->fused.sor.nblocks;
     }
     b->cap = sor_max_blocks;
+    b->gen.clear();
+    for (hv_ctx *c : b->ctx) b->gen.push_back(c->plan_gen);
     return HV_OK;
 }
 
@@ -258,6 +262,15 @@ hv_status hv_batch_run(hv_batch *b, int n_steps, hv_observables *obs) {
     if (n_steps == 0) return HV_OK;
     HV_CUDA(cudaSetDevice(b->device));
     const int n = (int)b->ctx.size();
+    // an instance's particles, parameters or options may have changed since the
+    // plan: its fields are solved, and the waves, which hold its buffers and
+    // options, built anew
+    bool stale = (int)b->gen.size() != n;
+    for (int i = 0; i < n; i++) {
+        HV_TRY(fused_batch_ready(b->ctx[i]));
+        stale = stale || b->gen[i] != b->ctx[i]->plan_gen;
+    }
+    if (stale) HV_TRY(hv_batch_plan(b, std::max(b->cap, 0)));
     // pinned room for what two chunks read back, per instance: the rows, the
     // iteration ring, the status word and (used once) the solver's seed
     const int ring = fused_batch_ring();

@@ -936,6 +936,7 @@ hv_status hv_ctx_set_fast_options(hv_ctx *c, const hv_fast_options *o) {
         c->fused.graph_len = 0;
     }
     c->fast = *o;
+    c->plan_gen++;
     return HV_OK;
 }
 

@@ -228,6 +228,7 @@ struct hv_ctx {
     int *taps_runs = nullptr;  // taps.slabs
     hv::Scratch scratch;
     hv::Fused fused;
+    unsigned plan_gen = 0;     // changes whenever buffers or options that a batch's waves hold do
     hv::Profile prof;
     hv_fast_options fast{};
     bool boundary_set = false;

@@ -1257,6 +1257,7 @@ hv_status fused_release(hv_ctx *c) {
     poisson_release(c);
     smooth_fast_release(c);
     f = Fused();
+    c->plan_gen++;
     return HV_OK;
 }
 

@@ -1639,6 +1639,7 @@ void sor_fast_release(hv_ctx *c) {
     for (void *p : ptrs)
         if (p) cudaFree(p);
     f = SorFast();
+    c->plan_gen++;
 }
 
 hv_status sor_fast_replan(hv_ctx *c, int max_blocks) {
