@@ -340,7 +340,9 @@ hv_status hv_batch_run(hv_batch *b, int n_steps, hv_observables *obs) {
         hv_status st = q > 0 ? settle(q - 1) : HV_OK;
         if (st == HV_OK && q + 1 == chunks) st = settle(q);
         if (st != HV_OK) {
+            // the chunk behind the failed one may have failed in others too
             HV_CUDA(cudaStreamSynchronize(b->stream));
+            for (int i = 0; i < n; i++) fused_batch_status(b->ctx[i], words(q, i)[0]);
             return st;
         }
     }
