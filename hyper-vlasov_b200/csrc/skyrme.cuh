@@ -42,6 +42,22 @@ __device__ __forceinline__ double pow_mid(double t, double gamma) {
     return __hiloint2double(__double2hiint(q) + (__double2loint(kd) << 20), __double2loint(q));
 }
 
+// t^gamma in float for t in [2^-20, 2^-8] and |gamma| <= 3 (gh + gl: gamma in two
+// floats), to 2^-20.9 of it at gamma 7/6 and 2^-20.5 at 2: the logarithm's error
+// (2^-22 of 1) times gamma ln 2, the exponential's 2^-22, two roundings.  The
+// fast power rounds the product gamma log2 t at its own size, for another 2^-20.5
+// where that passes 16.  Here the exponent's share gamma e goes into the result's
+// exponent as an integer and an exact remainder, and only gamma log2 m, m in
+// [sqrt(1/2), sqrt(2)), is rounded.
+__device__ __forceinline__ float pow_low(float t, float gh, float gl) {
+    const int hi = __float_as_int(t), e = (hi - 0x3f3504f3) >> 23;
+    const float l = __log2f(__int_as_float(hi - (e << 23))), fe = (float)e, k = rintf(gh * fe);
+    const float f = fmaf(gh, l, fmaf(gl, fe, fmaf(gh, fe, -k)));
+    float r;
+    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(f));
+    return r * __int_as_float(((int)k + 127) << 23);
+}
+
 // Skyrme potential (include/physics.hpp:272-281, physics_formulas.hpp:70-77).
 // A t and B t^gamma are some 300 MeV each and nearly cancel, so that a float
 // power (CUDA's fast one: 3e-7 of its value) left more noise in the forces than
@@ -49,8 +65,12 @@ __device__ __forceinline__ double pow_mid(double t, double gamma) {
 // component 3.2e-6 MeV/fm with __powf, 1.2e-6 with this form, and a third of
 // the error in D(t) after 100 steps.  In float the sums are therefore formed in
 // double and rounded once, where t >= 2^-8; below, B t^gamma is under 2 MeV and
-// the fast power's error under 5e-7 MeV.  The halo around a nucleus, most of
-// the box, takes that branch.  The double form (the fused FP64 path) keeps pow.
+// formed in float, in a nucleus's halo (down to 2^-20) with its exponent apart.
+// The rest of the box, empty or holding the 2^-22 to 2^-32 that the FFT smoothing
+// leaves, takes the fast power, whose share of U is small there.  208Pb 128^3,
+// Skyrme kernel: 11.1 us with the fast power from 2^-8 down, 12.7 so, 14.8 with
+// pow_low over the whole box, 12.1 with the doubles from 2^-20 on, which cost a
+// step as much.  The double form (the fused FP64 path) keeps pow.
 template <typename T>
 __device__ __forceinline__ void skyrme_node(double A, double B, double C, double gamma, T rp, T rn, T &up, T &un) {
     if constexpr (sizeof(T) == 4) {
@@ -63,7 +83,11 @@ __device__ __forceinline__ void skyrme_node(double A, double B, double C, double
             up = (float)(base - iso);
             un = (float)(base + iso);
         } else {
-            const float base = (float)A * tf + (float)B * __powf(tf, (float)gamma);
+            const float gh = (float)gamma;
+            const float power = tf >= 9.5367432e-7f && tf < 0.00390625f && fabs(gamma) <= 3.0
+                                    ? pow_low(tf, gh, (float)(gamma - (double)gh))
+                                    : __powf(tf, gh);
+            const float base = (float)A * tf + (float)B * power;
             const float iso = 2.0f * (float)C * ((rn - rp) * inv_rho0);
             up = base - iso;
             un = base + iso;
