@@ -40,7 +40,6 @@ struct hv_batch {
     std::vector<unsigned> gen;            // each context's plan_gen that the waves were built from
     int cap = -1;                         // SOR block cap of the current plan (0: own plans)
     cudaGraphExec_t graph = nullptr;
-    int graph_len = 0;
     cudaGraphExec_t tail_graph = nullptr; // a run's last, shorter chunk, once its length has come twice
     int tail_len = 0;
     int chunk = 8;
@@ -54,7 +53,6 @@ namespace {
 void drop_graph(hv_batch *b) {
     if (b->graph) cudaGraphExecDestroy(b->graph);
     b->graph = nullptr;
-    b->graph_len = 0;
     if (b->tail_graph) cudaGraphExecDestroy(b->tail_graph);
     b->tail_graph = nullptr;
     b->tail_len = 0;
